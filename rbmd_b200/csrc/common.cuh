@@ -16,7 +16,9 @@ constexpr int kWarp = 32;
 constexpr int kPairWarps = 8;          // atoms (warps) per block of the pair kernel
 constexpr int kAtomBlock = 256;        // atoms per block of the streaming kernels
 constexpr int kRhoChunk = 256;         // atoms per block of the structure-factor kernel
-constexpr int kCellBlock = 256;        // cells per block of the cell kernels
+constexpr int kCellBlock = 256;        // cells per work item of the cell kernels
+constexpr int kBuildCells = 32;        // cells per block of the cell-list build
+constexpr int kCellBigGrid = 16384;    // cells of a system above which counts are added up in two levels
 constexpr int kRbeSlack = 64;          // extra Metropolis proposal slots beyond P
 constexpr int kQueue = 64;             // per-warp pair queue of the pair kernel
 constexpr int kMaxF32Types = 16;       // atom types of the FP32 (mixed) pair table
@@ -82,6 +84,11 @@ struct SysState {
   // margins widen by it too.
   unsigned out_bits;
   int mig_n;
+  // Cell-list building (k_cells.cu): the buffer of counts the next list takes (bit 0), and for each
+  // buffer the distance above as it is gathered and the atoms beyond the buckets' capacity.
+  int cell_epoch;
+  unsigned out_acc[2];
+  int ovf_n[2];
   int mig_cell[kMaxMigrated];
 };
 
@@ -101,6 +108,7 @@ struct SysDev {
   // box changes on the device every step.  Cell arrays and the cell work table hold ncell_cap cells
   // (the box at kBoxGrow x L0); kmax indexes the Ewald k lists.
   int npt, ncell_cap, kmax[3], npt_pad;
+  int cell_cap, cell_stride;  // ids a cell's bucket holds; ints between the two count buffers
   double L0[3];
   double p_start, p_stop, p_damp, bulk;
   // geometry and physics
@@ -137,9 +145,11 @@ struct SysDev {
   int* image;          // [3n]
   // cells
   int* cell_of_atom;   // reference flat cell id
-  int* cell_count;     // [ncell]
+  int* cell_count;     // [2][cell_stride] two buffers, taken in turn
   int* cell_start;     // [ncell + 1]
-  int* cell_fill;      // [ncell] scatter cursors
+  int* cell_bucket;    // [ncell][cell_cap] atom ids in order of arrival
+  int* cell_ovf;       // [n] atoms that found their cell's bucket full
+  int* cell_gsum;      // [ncell / 32 + 1] atoms per 32 cells (systems of many cells)
   int* sorted;         // atom ids in cell order
   int* rank;           // [n] position of each atom in cell order (inverse of sorted)
   double4* sx;         // sorted positions + charge (FP64)

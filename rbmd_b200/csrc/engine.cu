@@ -238,13 +238,18 @@ int Context::refresh(System* s) {
   return RBMD_OK;
 }
 
+// Ids a cell's bucket holds: twice the mean occupancy and at least 4 more (a liquid's cells rarely pass
+// 1.5 times it; the atoms beyond go through the overflow list, at a cost per atom of the list's length).
+static int cell_bucket(int n, int ncell) { return (int)(2 * (int64_t)n / ncell + 4 + 3) & ~3; }
+
 int64_t Context::estimate_bytes(const rbmd_system_desc& d, const rbmd_params& p) {
   rbmd_derived dv;
   derive(d, p, dv);
   const int64_t n = d.n_atoms;
   int64_t b = n * (32 * 3 + 16 + 12 + 4 * 2 + 32 + 16 + 16 + 8);  // x v f meta image cells sorted sx sxf smeta fp
   if (p.fix_shake == RBMD_SHAKE_TRUE && d.n_angles > 0) b += n * 32 * 3;
-  b += (int64_t)dv.n_cells * 16 * (p.ensemble == RBMD_ENS_NPT ? 2 : 1);  // NPT: room for kBoxGrow^3
+  b += n * 4 + (int64_t)dv.n_cells * (13 + 4 * cell_bucket(d.n_atoms, dv.n_cells)) *
+                   (p.ensemble == RBMD_ENS_NPT ? 2 : 1);  // NPT: room for kBoxGrow^3
   const int P = p.coulomb == RBMD_COUL_RBE ? p.coulomb_sample_num : 0;
   int64_t nk = P;
   if (p.coulomb == RBMD_COUL_EWALD)
@@ -493,6 +498,8 @@ int Context::add_system(const rbmd_system_desc& d, const rbmd_params& p, int32_t
   } else {
     D.ncell_cap = D.ncell;
   }
+  D.cell_cap = cell_bucket(n, D.ncell);
+  D.cell_stride = (D.ncell_cap + 3) & ~3;
   D.blocks_pair = D.dense ? tile_blocks(D) : (n + kPairWarps - 1) / kPairWarps;
   D.blocks_atom = (n + kAtomBlock - 1) / kAtomBlock;
   D.blocks_rho = (n + kRhoChunk - 1) / kRhoChunk;
@@ -639,9 +646,11 @@ int Context::add_system(const rbmd_system_desc& d, const rbmd_params& p, int32_t
   D.meta = (int4*)dal(sizeof(int4) * n);
   D.image = (int*)dal(sizeof(int) * 3 * n);
   D.cell_of_atom = (int*)dal(sizeof(int) * n);
-  D.cell_count = (int*)dal(sizeof(int) * D.ncell_cap);
+  D.cell_count = (int*)dal(sizeof(int) * 2 * D.cell_stride);
   D.cell_start = (int*)dal(sizeof(int) * (D.ncell_cap + 1));
-  D.cell_fill = (int*)dal(sizeof(int) * D.ncell_cap);
+  D.cell_bucket = (int*)dal(sizeof(int) * (size_t)D.ncell_cap * D.cell_cap);
+  D.cell_ovf = (int*)dal(sizeof(int) * n);
+  D.cell_gsum = (int*)dal(sizeof(int) * (D.ncell_cap / 32 + 1));
   D.sorted = (int*)dal(sizeof(int) * n);
   D.rank = (int*)dal(sizeof(int) * n);
   D.sx = (double4*)dal(sizeof(double4) * n);
@@ -767,6 +776,7 @@ int Context::add_system(const rbmd_system_desc& d, const rbmd_params& p, int32_t
   up(D.x, hx.data(), sizeof(double4) * n);
   up(D.v, hv.data(), sizeof(double4) * n);
   cudaMemsetAsync(D.f, 0, sizeof(double4) * n, stream);
+  cudaMemsetAsync(D.cell_count, 0, sizeof(int) * 2 * D.cell_stride, stream);
   up(D.meta, hmeta.data(), sizeof(int4) * n);
   up(D.image, himg.data(), sizeof(int) * 3 * n);
   up(D.eps, d.epsilon, sizeof(double) * d.n_types);
@@ -909,6 +919,7 @@ Context::BatchRec* Context::build_batch(const std::vector<System*>& group, int& 
     b.band[3] = std::max(b.band[3], D.band[3]);
     slots.push_back(s->slot);
     br->ids.push_back(s->id);
+    if (D.ncell_cap > kCellBigGrid) b.big_cells = 1;
     b.max_P = std::max(b.max_P, std::max(D.P, D.nk_ewald));
     b.natoms += D.n;
     for (int k = 0; k < D.n; k += kAtomBlock) wa.push_back(make_int2(s->slot, k));
@@ -1045,7 +1056,7 @@ void Context::enqueue_step(const Batch& b) {
   if (b.npt == 2) timed("mtk", 0, [&] { launch_mtk_begin(b, stream); });
   else timed("nhc", 0, [&] { launch_nhc_a(b, stream); });
   timed("kick_drift", 0, [&] { launch_kick_drift(b, stream); });
-  timed("cells", 0, [&] { launch_cells(b, stream); });
+  timed("cells", 0, [&] { launch_cells_build(b, stream); });
   if (b.has_shake) timed("shake", 0, [&] { launch_shake(b, stream); });
   if (b.coul == RBMD_COUL_RBE) timed("rbe_sample", 0, [&] { launch_rbe_sample(b, stream); });
   if (b.coul != RBMD_COUL_NONE) timed("rho", 0, [&] { launch_rho(b, stream, b.coul == RBMD_COUL_EWALD); });

@@ -1,26 +1,15 @@
 // k_cells.cu -- cell-list binning by counting sort (replaces ContPointLocator::Build,
 // framework/locator/ContPointLocator.cxx:70-92: BinPointsWorklet + SortByKey + Upper/LowerBounds).
 //
-// count (atomics) -> exclusive scan (one block per system) -> scatter (atomics) -> per-cell sort
-// by atom id (the stable order of the reference's sort of fresh 0..N-1 point ids) fused with the
-// gather of cell-ordered positions, charges and metadata that the pair kernel streams.
-#include <climits>
-
-#include "kernels.h"
+// Two passes.  The first (bin_atom, in the kick-drift kernel of a step, in k_cells_count otherwise)
+// counts each cell's atoms and drops their ids into a bucket per cell.  The second (k_cells_build)
+// adds up the counts before its cells, orders each cell's ids (the stable order of the reference's
+// sort of fresh 0..N-1 point ids) and writes the cell-ordered positions, charges and metadata that the
+// pair kernels stream.  The counts live in two buffers taken in turn: building from one clears the
+// other for the next list, so no launch is spent on clearing.
+#include "cells.cuh"
 
 namespace rbmd {
-
-__global__ void k_cells_zero(const SysDev* __restrict__ S, const int2* __restrict__ work) {
-  const int2 w = work[blockIdx.x];
-  const SysDev& s = S[w.x];
-  const int c = w.y + threadIdx.x;
-  if (c < s.ncell) s.cell_count[c] = 0;
-  if (c == 0) {  // a new cell list: nothing has moved since
-    s.st->shake_disp_bits = 0u;
-    s.st->out_bits = 0u;
-    s.st->mig_n = 0;
-  }
-}
 
 __global__ void k_cells_count(const SysDev* __restrict__ S, const int2* __restrict__ work) {
   const int2 w = work[blockIdx.x];
@@ -29,118 +18,138 @@ __global__ void k_cells_count(const SysDev* __restrict__ S, const int2* __restri
   if (i >= s.n) return;
   const double4 p = s.x[i];
   const double pc[3] = {p.x, p.y, p.z};
-  int ijk[3];
-  double out = 0.0;  // how far the atom lies outside the cell it is binned into
-#pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    long long c = (long long)((pc[k] - s.lo[k]) / s.d[k]);  // truncation, as vtkm::Id3(Vec3f)
-    c = c < 0 ? 0 : c;
-    c = c > s.dims[k] - 1 ? s.dims[k] - 1 : c;
-    ijk[k] = (int)c;
-    out = fmax(out, fmax(s.lo[k] + (double)c * s.d[k] - pc[k], pc[k] - (s.lo[k] + (double)(c + 1) * s.d[k])));
-  }
-  if (out > 0.0) atomicMax(&s.st->out_bits, __float_as_uint(__double2float_ru(out)));  // non-negative: bits order as values
-  // internal numbering is z fastest so that the 2 nc + 1 cells of a traversal row (fixed x and y
-  // offsets) are contiguous in cell order; get_cells reports the reference's x-fastest ids
-  const int cell = ijk[2] + s.dims[2] * (ijk[1] + s.dims[1] * ijk[0]);
-  s.cell_of_atom[i] = cell;
-  atomicAdd(&s.cell_count[cell], 1);
+  bin_atom(s, i, pc);
 }
 
-// One block (1024 threads) per system: exclusive scan of the cell counts.
-__global__ void __launch_bounds__(1024) k_cells_scan(const SysDev* __restrict__ S,
-                                                     const int* __restrict__ slots) {
-  const SysDev& s = S[slots[blockIdx.x]];
-  const int nt = blockDim.x, t = threadIdx.x;
-  const int chunk = (s.ncell + nt - 1) / nt;
-  const int c0 = t * chunk, c1 = min(c0 + chunk, s.ncell);
-  int local = 0;
-  for (int c = c0; c < c1; ++c) local += s.cell_count[c];
-  __shared__ int wsum[32];
-  const int lane = t & 31, wid = t >> 5;
-  int incl = warp_incl_scan(local, lane);
-  if (lane == 31) wsum[wid] = incl;
-  __syncthreads();
-  if (wid == 0) {
-    int vsum = (lane < (nt >> 5)) ? wsum[lane] : 0;
-    int winc = warp_incl_scan(vsum, lane);
-    wsum[lane] = winc - vsum;
-  }
-  __syncthreads();
-  int run = wsum[wid] + incl - local;
-  for (int c = c0; c < c1; ++c) {
-    s.cell_start[c] = run;
-    s.cell_fill[c] = run;
-    run += s.cell_count[c];
-  }
-  if (t == nt - 1) s.cell_start[s.ncell] = s.n;
-}
+// kBuildCells cells per block: one warp scans their counts.  A block per work item (kCellBlock cells)
+// meant 8-16 cells per warp one after the other, and 1 or 2 blocks for a box of a few hundred cells.
+constexpr int kBuildThreads = 256;
+constexpr int kBuildSplit = kCellBlock / kBuildCells;
+static_assert(kCellBlock % kBuildCells == 0, "a work item is a whole number of build blocks");
 
-__global__ void k_cells_scatter(const SysDev* __restrict__ S, const int2* __restrict__ work) {
+// Atoms per group of kBuildCells cells, for systems of more than kCellBigGrid cells.
+__global__ void k_cells_group_sums(const SysDev* __restrict__ S, const int2* __restrict__ work) {
   const int2 w = work[blockIdx.x];
   const SysDev& s = S[w.x];
-  const int i = w.y + threadIdx.x;
-  if (i >= s.n) return;
-  const int slot = atomicAdd(&s.cell_fill[s.cell_of_atom[i]], 1);
-  s.sorted[slot] = i;
+  const int c = w.y + threadIdx.x;
+  const int par = s.st->cell_epoch & 1;
+  const int cnt = c < s.ncell ? s.cell_count[(size_t)par * s.cell_stride + c] : 0;
+  const int sum = __reduce_add_sync(0xffffffffu, cnt);
+  if ((threadIdx.x & 31) == 0 && c < s.ncell) s.cell_gsum[c / kBuildCells] = sum;
 }
 
-// One warp per cell (kSortWarps warps per block, each taking kCellBlock / kSortWarps cells of the
-// block's range): the cell's atom ids ranked by value with shuffles (cells of more than 32 atoms,
-// rare, are sorted by lane 0), then the cell-ordered copies of positions and metadata written by
-// consecutive lanes.  The order is the ids' ascending order, as before.
-constexpr int kSortWarps = 32;
-
-__global__ void __launch_bounds__(kSortWarps * 32) k_cells_sort_gather(const SysDev* __restrict__ S,
-                                                                     const int2* __restrict__ work) {
+// One block per kBuildCells cells.  Bound by latency: the loads of the preceding counts (at most
+// kCellBigGrid / (4 x 256) 16-byte loads per thread; above that the group sums of the kernel before),
+// then one dependent gather per atom.  A cell's ids are taken by 8 lanes where buckets are small (cells
+// of a few atoms) and by a warp otherwise; each lane ranks its ids against the whole bucket, so cells
+// of hundreds of atoms need no serial sort.  `blocks` is the number of blocks per system where the work
+// table covers a single system's present cells only, 0 where it covers the ncell_cap of each.
+__global__ void __launch_bounds__(kBuildThreads) k_cells_build(const SysDev* __restrict__ S,
+                                                             const int2* __restrict__ work, int big, int blocks) {
   const int2 w = work[blockIdx.x];
   const SysDev& s = S[w.x];
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const unsigned FULL = 0xffffffffu;
-  int* ids = s.sorted;
-  for (int cc = wid; cc < kCellBlock; cc += kSortWarps) {
-    const int c = w.y + cc;
-    if (c >= s.ncell) break;  // warp-uniform
-    const int b = s.cell_start[c], e = s.cell_start[c + 1], cnt = e - b;
-    if (cnt <= 32) {
-      const int id = lane < cnt ? ids[b + lane] : INT_MAX;
-      int rank = 0;
-      for (int j = 0; j < cnt; ++j) rank += __shfl_sync(FULL, id, j) < id ? 1 : 0;
-      __syncwarp();
-      if (lane < cnt) ids[b + rank] = id;
-      __syncwarp();
+  SysState* st = s.st;
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  const int c0 = w.y + blockIdx.y * kBuildCells;
+  const int par = st->cell_epoch & 1;
+  const int* count = s.cell_count + (size_t)par * s.cell_stride;
+  int* other = s.cell_count + (size_t)(par ^ 1) * s.cell_stride;
+  __shared__ int s_sum[kBuildThreads / 32], s_start[kBuildCells], s_cnt[kBuildCells];
+  if (c0 < s.ncell) {  // block-uniform
+    int sum = 0;
+    if (big) {
+      for (int g = tid; g < c0 / kBuildCells; g += kBuildThreads) sum += s.cell_gsum[g];
     } else {
-      if (lane == 0)
-        for (int k = b + 1; k < e; ++k) {
-          const int key = ids[k];
-          int j = k - 1;
-          while (j >= b && ids[j] > key) {
-            ids[j + 1] = ids[j];
-            --j;
-          }
-          ids[j + 1] = key;
-        }
-      __syncwarp();
+      const int4* c4 = reinterpret_cast<const int4*>(count);  // c0 is a multiple of 4
+      for (int g = tid; g < c0 / 4; g += kBuildThreads) {
+        const int4 v = c4[g];
+        sum += (v.x + v.y) + (v.z + v.w);
+      }
     }
-    for (int k = b + lane; k < e; k += 32) {
-      const int i = ids[k];
+    sum = __reduce_add_sync(0xffffffffu, sum);
+    if (lane == 0) s_sum[wid] = sum;
+    __syncthreads();
+    if (wid == 0) {
+      int base = lane < kBuildThreads / 32 ? s_sum[lane] : 0;
+      base = __reduce_add_sync(0xffffffffu, base);
+      const int c = c0 + lane;
+      const int cnt = c < s.ncell ? count[c] : 0;
+      const int incl = warp_incl_scan(cnt, lane);
+      s_start[lane] = base + incl - cnt;
+      s_cnt[lane] = cnt;
+      if (c < s.ncell) s.cell_start[c] = base + incl - cnt;
+      if (c == s.ncell - 1) s.cell_start[s.ncell] = base + incl;
+    }
+    __syncthreads();
+    const int cap = s.cell_cap;
+    const int lanes = cap <= 16 ? 8 : 32;  // lanes per cell
+    const int gl = tid & (lanes - 1);
+    auto place = [&](int i, int k) {
+      s.sorted[k] = i;
       s.rank[i] = k;
       const double4 p = s.x[i];
       s.sx[k] = p;
       s.sxf[k] = make_float4((float)p.x, (float)p.y, (float)p.z, (float)p.w);
       const int4 m = s.meta[i];
       s.smeta[k] = make_int4(i, m.x, m.y, m.z);
+    };
+    for (int cc = tid / lanes; cc < kBuildCells; cc += kBuildThreads / lanes) {
+      const int c = c0 + cc, cnt = s_cnt[cc], in = min(cnt, cap);
+      const int* ids = s.cell_bucket + (size_t)c * cap;
+      auto rank_of = [&](int id) {
+        int r = 0;
+        for (int j = 0; j < in; ++j) r += ids[j] < id ? 1 : 0;
+        return r;
+      };
+      if (cnt <= cap) {
+        for (int k = gl; k < cnt; k += lanes) {
+          const int id = ids[k];
+          place(id, s_start[cc] + rank_of(id));
+        }
+      } else {  // more atoms than the bucket holds: the rest are in the overflow list
+        const int novf = st->ovf_n[par];
+        auto rank_ovf = [&](int id) {
+          int r = 0;
+          for (int e = 0; e < novf; ++e) r += (s.cell_ovf[e] < id && s.cell_of_atom[s.cell_ovf[e]] == c) ? 1 : 0;
+          return r;
+        };
+        for (int k = gl; k < in; k += lanes) place(ids[k], s_start[cc] + rank_of(ids[k]) + rank_ovf(ids[k]));
+        for (int e = gl; e < novf; e += lanes) {
+          const int id = s.cell_ovf[e];
+          if (s.cell_of_atom[id] == c) place(id, s_start[cc] + rank_of(id) + rank_ovf(id));
+        }
+      }
+    }
+    if (c0 == 0 && tid == 0) {  // a new cell list: nothing has moved since
+      st->shake_disp_bits = 0u;
+      st->mig_n = 0;
+      st->out_bits = st->out_acc[par];
+      st->out_acc[par ^ 1] = 0u;
+      st->ovf_n[par ^ 1] = 0;
     }
   }
+  if (blocks == 0) blocks = (s.ncell_cap + kCellBlock - 1) / kCellBlock * kBuildSplit;
+  if (tid < kBuildCells && c0 + tid < s.ncell_cap) other[c0 + tid] = 0;
+  if (c0 == 0)
+    for (int c = blocks * kBuildCells + tid; c < s.ncell_cap; c += kBuildThreads) other[c] = 0;
+  // every block has read this list's buffer index: the next list takes the other buffer
+  if (arrive_last(&st->counter[7], (unsigned)blocks) && tid == 0) st->cell_epoch ^= 1;
+}
+
+void launch_cells_build(const Batch& b, cudaStream_t st) {
+  if (b.big_cells) {
+    k_cells_group_sums<<<b.cell.n, kCellBlock, 0, st>>>(b.sys, b.cell.d);
+    note_launch();
+  }
+  k_cells_build<<<dim3(b.cell.n, kBuildSplit), kBuildThreads, 0, st>>>(b.sys, b.cell.d, b.big_cells,
+                                                                           b.cell_blocks);
+  note_launch();
 }
 
 void launch_cells(const Batch& b, cudaStream_t st) {
-  k_cells_zero<<<b.cell.n, kCellBlock, 0, st>>>(b.sys, b.cell.d);
   k_cells_count<<<b.atom.n, kAtomBlock, 0, st>>>(b.sys, b.atom.d);
-  k_cells_scan<<<b.nsys, 1024, 0, st>>>(b.sys, b.d_slots);
-  k_cells_scatter<<<b.atom.n, kAtomBlock, 0, st>>>(b.sys, b.atom.d);
-  k_cells_sort_gather<<<b.cell.n, kSortWarps * 32, 0, st>>>(b.sys, b.cell.d);
-  note_launch(5);
+  note_launch();
+  launch_cells_build(b, st);
 }
 
 }  // namespace rbmd

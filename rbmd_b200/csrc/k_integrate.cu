@@ -14,6 +14,7 @@
 // The scalar thermostat work runs on the device in the last block of each system (last-block
 // reduction of the kinetic-energy partials), so a whole step is a fixed kernel sequence with no
 // host round trip and can be captured in a CUDA graph.
+#include "cells.cuh"
 #include "chain.cuh"
 
 namespace rbmd {
@@ -37,7 +38,8 @@ __global__ void k_nhc_a(const SysDev* __restrict__ S, const int* __restrict__ sl
   }
 }
 
-// v = v * pending * a; v += F/m dt/2; x += v dt; periodic wrap with image flags.  MTK systems
+// v = v * pending * a; v += F/m dt/2; x += v dt; periodic wrap with image flags; the new position's
+// cell (bin_atom: the cell list of the step is built before the constraint).  MTK systems
 // (npt 2) also take the NH_V_Press factors twice before the kick and are remapped to the first
 // half-step box before the drift and to the second after it (InitialIntegrate,
 // ExecutionNPT.cpp:1671-1711); the wrap uses the first box and the second remap does not wrap.
@@ -96,6 +98,7 @@ __global__ void k_kick_drift(const SysDev* __restrict__ S, const int2* __restric
       p[k] = __dadd_rn(__dmul_rn(s.L[k], __dmul_rn(st->mtk_hinv1[k], __dsub_rn(p[k], st->mtk_lo1[k]))), s.lo[k]);
   }
   s.x[i] = make_double4(p[0], p[1], p[2], x.w);
+  bin_atom(s, i, p);
 }
 
 // Applies the pending end-of-step velocity factor (between rbmd_step calls the stored velocities

@@ -33,6 +33,8 @@ struct Batch {
   int lean = 0;              // warp per atom with segment tables (dims >= 2 nc + 1 everywhere)
   int npt = 0;               // NPT barostat: 0 none, 1 Berendsen (end of step), 2 MTK (around the integrator)
   int near = 0;              // RBL Coulomb with the reference's near-Coulomb table (RBMD_NEAR_TABLE)
+  int big_cells = 0;         // a system has more than kCellBigGrid cells
+  int cell_blocks = 0;       // one system whose cell table covers its present cells only: its build blocks
   int max_P = 0;             // largest P (or Ewald nk) in the batch
   float band[4] = {0, 0, 0, 0};  // FP32 classification bands: union over the batch (same rc, rs)
   long long natoms = 0;      // atoms over all systems of the batch
@@ -41,8 +43,11 @@ struct Batch {
 enum FinalMode { kFinalForceOnly = 0, kFinalKick = 1, kFinalInit = 2 };
 
 void launch_nhc_a(const Batch& b, cudaStream_t s);
+// Also bins the drifted atoms: launch_cells_build completes the cell list.
 void launch_kick_drift(const Batch& b, cudaStream_t s);
+// Cell list of the current positions; launch_cells_build alone after atoms were binned by kick_drift.
 void launch_cells(const Batch& b, cudaStream_t s);
+void launch_cells_build(const Batch& b, cudaStream_t s);
 void launch_shake(const Batch& b, cudaStream_t s);
 void launch_rattle(const Batch& b, cudaStream_t s);
 void launch_rbe_sample(const Batch& b, cudaStream_t s);
