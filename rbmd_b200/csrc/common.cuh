@@ -19,7 +19,7 @@ constexpr int kRhoChunk = 256;         // atoms per block of the structure-facto
 constexpr int kCellBlock = 256;        // cells per work item of the cell kernels
 constexpr int kBuildCells = 32;        // cells per block of the cell-list build
 constexpr int kCellBigGrid = 16384;    // cells of a system above which counts are added up in two levels
-constexpr int kRbeSlack = 64;          // extra Metropolis proposal slots beyond P
+constexpr int kRbeSlack = 64;          // Metropolis proposal slots tried beyond the samples still to draw
 constexpr int kQueue = 64;             // per-warp pair queue of the pair kernel
 constexpr int kMaxF32Types = 16;       // atom types of the FP32 (mixed) pair table
 
@@ -103,7 +103,7 @@ struct SysDev {
   int lean;   // segment-table traversal usable (every dimension holds more than nc cells)
   int dense;  // pair kernel layout: 0 warp per atom, 1 tile (warp per home cell), 2 column (warp per
               // column of home cells, lane per atom; FP32 RBL forces only, the tile kernel otherwise)
-  int blocks_pair, blocks_atom, blocks_rho, blocks_tri, rbe_mmax, rbe_slots, has_triples, n_triples;
+  int blocks_pair, blocks_atom, blocks_rho, blocks_tri, rbe_mmax, has_triples, n_triples;
   // NPT barostats (npt 1: Berendsen at the end of the step, 2: MTK around the integrator): the
   // box changes on the device every step.  Cell arrays and the cell work table hold ncell_cap cells
   // (the box at kBoxGrow x L0); kmax indexes the Ewald k lists.

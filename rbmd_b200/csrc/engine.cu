@@ -535,7 +535,6 @@ int Context::add_system(const rbmd_system_desc& d, const rbmd_params& p, int32_t
       smax = std::max(smax, D.rbe_sigma[k] * (D.npt ? kBoxGrow : 1.0));  // NPT: table for the largest box
     }
     D.rbe_mmax = std::min(4096, (int)std::ceil(12.0 * smax) + 4);
-    D.rbe_slots = std::min(1024, D.P + kRbeSlack);
     const int tw = 2 * D.rbe_mmax + 1;
     rbe_tab.assign((size_t)3 * tw * 2, 0.0);
     for (int k = 0; k < 3; ++k) {

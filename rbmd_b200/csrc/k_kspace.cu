@@ -6,17 +6,14 @@
 //                                                framework/run/ExecutionMD.cpp:469-501
 //   ComputeEwaldEnergy                           framework/run/ExecutionMD.cpp:405-443
 //
-// Sampling runs on the device so a step never returns to the host: one block per system draws
-// every Metropolis proposal and acceptance uniform in parallel from Philox (they do not depend on
-// the chain state), then three lanes run the x, y, z chains in lock step, rejecting all-zero
-// vectors together as the reference does.  Proposal probabilities come from per-system tables of
+// Sampling runs on the device so a step never returns to the host.  Proposal probabilities come from per-system tables of
 // P(m) and q(m) built on the host with the reference's formulas, so the chain makes the same
 // accept/reject decisions as the CPU oracle on the same stream.
 #include "kernels.h"
 
 namespace rbmd {
 
-constexpr int kMaxRbeSlots = 1024;  // proposal slots held in shared memory per system
+constexpr int kMaxRbeSlots = 1024;  // proposal slots of a system decided at a time
 
 // Box-Muller proposal of slot t, dimension d (FetchSample_1D, RBEPSample.h:115-145).
 __device__ inline double rbe_gauss(const SysDev& s, uint32_t step, uint32_t t, int d) {
@@ -40,85 +37,155 @@ __device__ inline double rbe_accept(const SysDev& s, uint32_t step, uint32_t t, 
   return u01(o[0], o[1]);
 }
 
-__global__ void __launch_bounds__(256) k_rbe_sample(const SysDev* __restrict__ S,
-                                                    const int* __restrict__ slots) {
+// Probability of moving a chain from m = im to m = iw (MH_Algorithm, RBEPSample.h:64-83), indices into
+// the tables of one dimension.
+__device__ __forceinline__ double rbe_move(const double* tabP, const double* tabQ, int tw, int im, int iw) {
+  double p = 0.0;
+  if (iw >= 0 && iw < tw && im >= 0 && im < tw) p = (tabP[iw] / tabP[im]) * (tabQ[im] / tabQ[iw]);
+  return fmin(p, 1.0);
+}
+
+// One block per system, the proposal slots taken kMaxRbeSlots at a time.  A slot's proposal and uniform
+// do not depend on the chain, and the chain's state is almost always the slot before's proposal (the
+// proposals follow the target closely, so about one in a hundred is refused), so every slot decides
+// in parallel whether it would be accepted from the proposal one slot back and from the one two slots
+// back.  Only the refused slots are left to walk in order: a warp per dimension goes from one clear
+// bit of the first decision to the next, and evaluates a move itself when three or more slots in a row
+// are refused.  The dimensions' chains do not see each other: an all-zero vector is left out of the
+// samples but stays the chain's state.  Counting the slots with a non-zero vector gives each
+// sample's place.  Walking the chain slot by slot was a serial string of table reads and divisions:
+// 91 us for P = 200 and 52 us for P = 100, whatever the system's size.
+constexpr int kRbeThreads = 512;
+constexpr int kRbeWords = kMaxRbeSlots / 32;
+static_assert(kRbeThreads >= 96 && kMaxRbeSlots % 32 == 0, "a warp per dimension, whole words");
+
+__global__ void __launch_bounds__(kRbeThreads) k_rbe_sample(const SysDev* __restrict__ S,
+                                                           const int* __restrict__ slots) {
   const SysDev& s = S[slots[blockIdx.x]];
   if (s.coul != RBMD_COUL_RBE) return;
-  __shared__ double s_m[kMaxRbeSlots * 3];
-  __shared__ double s_u[kMaxRbeSlots * 3];
+  __shared__ int s_m[3][kMaxRbeSlots];         // proposals
+  __shared__ double s_u[3][kMaxRbeSlots];      // acceptance uniforms
+  __shared__ short s_src[3][kMaxRbeSlots];     // slot whose proposal the chain holds after each slot, -1: the
+                                               // state before the first
+  __shared__ unsigned s_acc[2][3][kRbeWords];  // accepted from the proposal one / two slots back
+  __shared__ unsigned s_nz[kRbeWords];         // slots after which the vector is not zero
+  __shared__ int s_prev[3], s_first, s_used;
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  const unsigned FULL = 0xffffffffu;
   const uint32_t step = (uint32_t)s.st->step;
-  const int nslots = min(s.rbe_slots, kMaxRbeSlots);
-  for (int k = threadIdx.x; k < nslots * 3; k += blockDim.x) {
-    const int t = k / 3, d = k % 3;
-    s_m[k] = round(rbe_gauss(s, step, (uint32_t)t, d));
-    s_u[k] = rbe_accept(s, step, (uint32_t)t, d);
-  }
-  __syncthreads();
-  if (threadIdx.x >= 32) return;
-  const int lane = threadIdx.x;
-  const int d = lane < 3 ? lane : 0;
-  const int mmax = s.rbe_mmax, tw = 2 * mmax + 1;
-  const double* tabP = s.rbe_tab + (size_t)d * tw * 2;
-  const double* tabQ = tabP + tw;
-  const double eps = 1e-6;
-  auto prop = [&](int t) -> double {
-    return t < nslots ? s_m[t * 3 + d] : round(rbe_gauss(s, step, (uint32_t)t, d));
-  };
-  auto acc = [&](int t) -> double { return t < nslots ? s_u[t * 3 + d] : rbe_accept(s, step, (uint32_t)t, d); };
+  const int P = s.P, mmax = s.rbe_mmax, tw = 2 * mmax + 1;
   // The reference loops until it finds non-zero vectors; bound the slots so that a degenerate
   // distribution (all proposals rounding to 0) ends with an error word instead of spinning.
-  const int tmax = 4096 + 64 * s.P;
-  int t = 0;
-  bool exhausted = false;
-  double X0;
-  for (;;) {
-    X0 = prop(t);
-    ++t;
-    const bool z = fabs(X0) < eps;
-    const bool zx = __shfl_sync(0xffffffffu, z, 0), zy = __shfl_sync(0xffffffffu, z, 1),
-               zz = __shfl_sync(0xffffffffu, z, 2);
-    if (!(zx && zy && zz)) break;
-    if (t >= tmax) {
-      exhausted = true;
-      X0 = (d == 0) ? 1.0 : 0.0;
-      break;
+  const int tmax = 4096 + 64 * P;
+  int t0 = 0, done = 0;     // slots and samples before this round
+  bool started = false;
+  if (tid < 3) s_prev[tid] = tid == 0 ? 1 : 0;
+  while (done < P && t0 < tmax) {
+    const int ns = min(min(kMaxRbeSlots, P - done + kRbeSlack), tmax - t0);
+    const int nw = (ns + 31) >> 5;
+    if (tid == 0) s_first = started ? -1 : ns;
+    for (int k = tid; k < 3 * ns; k += kRbeThreads) {
+      const int d = k / ns, t = k - d * ns;
+      s_m[d][t] = (int)round(rbe_gauss(s, step, (uint32_t)(t0 + t), d));
+      s_u[d][t] = rbe_accept(s, step, (uint32_t)(t0 + t), d);
     }
-  }
-  if (lane < 3) s.km[d] = (int)X0;
-  for (int i = 1; i < s.P; ++i) {
-    if (t >= tmax) {  // fill the rest with the last vector and flag the system
-      exhausted = true;
-      if (lane < 3) s.km[3 * i + d] = (int)X0;
-      continue;
+    __syncthreads();
+    if (!started) {  // the chains start at the first slot with a non-zero vector, taken as it is
+      for (int t = tid; t < ns; t += kRbeThreads)
+        if ((s_m[0][t] | s_m[1][t] | s_m[2][t]) != 0) atomicMin(&s_first, t);
+      __syncthreads();
     }
-    // MH_Algorithm, RBEPSample.h:64-83
-    const double mw = prop(t);
-    const double u = acc(t);
-    ++t;
-    double X1 = X0;
-    const int im = (int)X0 + mmax, iw = (int)mw + mmax;
-    double Prob = 0.0;
-    if (iw >= 0 && iw < tw && im >= 0 && im < tw)
-      Prob = (tabP[iw] / tabP[im]) * (tabQ[im] / tabQ[iw]);
-    Prob = fmin(Prob, 1.0);
-    if (u <= Prob) X1 = mw;
-    if (lane < 3) s.km[3 * i + d] = (int)X1;
-    X0 = X1;
-    const bool z = fabs(X1) < eps;
-    const bool zx = __shfl_sync(0xffffffffu, z, 0), zy = __shfl_sync(0xffffffffu, z, 1),
-               zz = __shfl_sync(0xffffffffu, z, 2);
-    if (zx && zy && zz) i = i - 1;
+    const int first = s_first;
+    if (first < ns) {
+      for (int w = wid; w < 3 * nw; w += kRbeThreads / 32) {
+        const int d = w / nw, t = 32 * (w - d * nw) + lane;
+        const double *tabP = s.rbe_tab + (size_t)d * tw * 2, *tabQ = tabP + tw;
+        bool one = false, two = false;
+        if (t < ns) {
+          const int iw = s_m[d][t] + mmax;
+          const double u = s_u[d][t];
+          one = u <= rbe_move(tabP, tabQ, tw, (t > 0 ? s_m[d][t - 1] : s_prev[d]) + mmax, iw);
+          if (t > 0) two = u <= rbe_move(tabP, tabQ, tw, (t > 1 ? s_m[d][t - 2] : s_prev[d]) + mmax, iw);
+          one |= t <= first;
+        }
+        const unsigned o = __ballot_sync(FULL, one), q = __ballot_sync(FULL, two);
+        if (lane == 0) {
+          s_acc[0][d][w - d * nw] = o;
+          s_acc[1][d][w - d * nw] = q;
+        }
+        if (t < ns) s_src[d][t] = (short)t;  // overwritten where the chain stays
+      }
+      __syncthreads();
+      if (wid < 3 && lane == 0) {
+        const int d = wid;
+        const double *tabP = s.rbe_tab + (size_t)d * tw * 2, *tabQ = tabP + tw;
+        for (int t = 0; t < ns;) {
+          const unsigned w = s_acc[0][d][t >> 5] | ((1u << (t & 31)) - 1u);
+          if (w == FULL) {  // no refusal up to the end of the word
+            t = (t | 31) + 1;
+            continue;
+          }
+          t = (t & ~31) + __ffs(~w) - 1;
+          if (t >= ns) break;
+          const int src = t - 1;  // slot t refused: the chain stays at the proposal of the slot before
+          const int im = (src >= 0 ? s_m[d][src] : s_prev[d]) + mmax;
+          s_src[d][t] = (short)src;
+          for (++t; t < ns; ++t) {
+            const bool a = t == src + 2 ? (s_acc[1][d][t >> 5] >> (t & 31)) & 1u
+                                        : s_u[d][t] <= rbe_move(tabP, tabQ, tw, im, s_m[d][t] + mmax);
+            if (a) break;
+            s_src[d][t] = (short)src;
+          }
+          ++t;  // accepted
+        }
+      }
+      __syncthreads();
+      auto state = [&](int d, int t) { return s_src[d][t] >= 0 ? s_m[d][s_src[d][t]] : s_prev[d]; };
+      for (int w = wid; w < nw; w += kRbeThreads / 32) {
+        const int t = 32 * w + lane;
+        const bool nz = t < ns && t >= first && (state(0, t) | state(1, t) | state(2, t)) != 0;
+        const unsigned b = __ballot_sync(FULL, nz);
+        if (lane == 0) s_nz[w] = b;
+      }
+      __syncthreads();
+      for (int w = wid; w < nw; w += kRbeThreads / 32) {
+        int before = 0;  // samples of the words before
+        for (int v = lane; v < w; v += 32) before += __popc(s_nz[v]);
+        before = done + __reduce_add_sync(FULL, before);
+        const int t = 32 * w + lane, l = before + __popc(s_nz[w] & lanemask_lt(lane));
+        if ((s_nz[w] >> lane) & 1u && l < P) {
+          for (int d = 0; d < 3; ++d) s.km[3 * l + d] = state(d, t);
+        }
+      }
+      if (wid == 0) {
+        int all = 0;
+        for (int v = lane; v < nw; v += 32) all += __popc(s_nz[v]);
+        all = __reduce_add_sync(FULL, all);
+        if (lane == 0) s_used = all;
+      }
+      int last = 0;
+      if (tid < 3) last = state(tid, ns - 1);
+      __syncthreads();
+      if (tid < 3) s_prev[tid] = last;
+      done += s_used;
+      started = true;
+    }
+    t0 += ns;
+    __syncthreads();
   }
-  __syncwarp();
+  if (done < P) {  // out of slots: the rest repeats the last vector, and the system is flagged
+    for (int k = 3 * done + tid; k < 3 * P; k += kRbeThreads) s.km[k] = s_prev[k % 3];
+    if (tid == 0) atomicOr(&s.st->status, kErrRbeSlots);
+  }
+  __syncthreads();
   // k vectors and force coefficients: k_l = 2 pi m_l / L, coef = -4 pi / (V |k_l|^2)
-  for (int l = lane; l < s.P; l += 32) {
+  for (int l = tid; l < P; l += kRbeThreads) {
     const double kx = 2 * kPi * s.km[3 * l] / s.L[0];
     const double ky = 2 * kPi * s.km[3 * l + 1] / s.L[1];
     const double kz = 2 * kPi * s.km[3 * l + 2] / s.L[2];
     const double k2 = kx * kx + ky * ky + kz * kz;
     s.kv[l] = make_double4(kx, ky, kz, -4 * kPi / (s.volume * k2));
   }
-  if (lane == 0 && exhausted) atomicOr(&s.st->status, kErrRbeSlots);
 }
 
 // Structure factor over a chunk of kRhoChunk atoms per block, every thread owning k indices; the
@@ -208,7 +275,7 @@ __global__ void __launch_bounds__(256) k_rho(const SysDev* __restrict__ S, const
 }
 
 void launch_rbe_sample(const Batch& b, cudaStream_t st) {
-  k_rbe_sample<<<b.nsys, 256, 0, st>>>(b.sys, b.d_slots);
+  k_rbe_sample<<<b.nsys, kRbeThreads, 0, st>>>(b.sys, b.d_slots);
   note_launch();
 }
 
