@@ -198,8 +198,8 @@ def kernel_profile(ctx, ids, systems):
     ctx.step(ids, 2)
     ctx.sync()
     out = {}
-    for name in ("nhc", "kick_drift", "cells", "shake", "rbe_sample", "rho", "bonded", "pair_col", "pair_tile", "pair_lean",
-                 "pair_atom", "final", "rattle"):
+    for name in ("nhc", "kick_drift", "cells", "shake", "rbe_sample", "rho", "far", "bonded", "pair_col", "pair_tile",
+                 "pair_lean", "pair_atom", "final", "rattle"):
         ms, n, units = ctx.profile_get(name)
         if n:
             out[name] = dict(avg_ms=ms, launches=n, units_per_launch=units)

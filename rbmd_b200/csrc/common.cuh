@@ -15,7 +15,8 @@ constexpr double kPif = 3.1415927410125732421875;  // float pi promoted, as the 
 constexpr int kWarp = 32;
 constexpr int kPairWarps = 8;          // atoms (warps) per block of the pair kernel
 constexpr int kAtomBlock = 256;        // atoms per block of the streaming kernels
-constexpr int kRhoChunk = 256;         // atoms per block of the structure-factor kernel
+constexpr int kRhoChunk = 256;         // most atoms per block of the structure-factor kernel
+constexpr int kFarAtoms = 64;          // atoms per block of the far-force kernel (four threads each)
 constexpr int kCellBlock = 256;        // cells per work item of the cell kernels
 constexpr int kBuildCells = 32;        // cells per block of the cell-list build
 constexpr int kCellBigGrid = 16384;    // cells of a system above which counts are added up in two levels
@@ -108,6 +109,7 @@ struct SysDev {
   // box changes on the device every step.  Cell arrays and the cell work table hold ncell_cap cells
   // (the box at kBoxGrow x L0); kmax indexes the Ewald k lists.
   int npt, ncell_cap, kmax[3], npt_pad;
+  int rho_chunk;  // atoms per structure-factor block
   int cell_cap, cell_stride;  // ids a cell's bucket holds; ints between the two count buffers
   double L0[3];
   double p_start, p_stop, p_damp, bulk;
@@ -138,6 +140,8 @@ struct SysDev {
   double4* x;          // x, y, z, charge
   double4* v;          // vx, vy, vz, mass
   double4* f;          // force
+  double4* ffar;       // far force (RBE, Ewald)
+  double* far_vir;     // [6 per kFarAtoms atoms] its virial partials
   double4* xold;       // pre-drift positions (SHAKE)
   double4* vold;       // pre-kick velocities (SHAKE first half)
   double4* vold2;      // pre-kick velocities (RATTLE)

@@ -238,6 +238,11 @@ int Context::refresh(System* s) {
   return RBMD_OK;
 }
 
+// Atoms per block of the structure factor: small while the blocks do not fill the 148 SMs (the sums over
+// a chunk's warps cost more the shorter it is: with 64 and 128 atoms for every system the saline stream's
+// kernel took 127 us for 97 us).  By the system's size alone: its sums are the same in any batch.
+static int rho_chunk(int n) { return n <= 148 * 64 ? 64 : (n <= 148 * 128 ? 128 : kRhoChunk); }
+
 // Ids a cell's bucket holds: twice the mean occupancy and at least 4 more (a liquid's cells rarely pass
 // 1.5 times it; the atoms beyond go through the overflow list, at a cost per atom of the list's length).
 static int cell_bucket(int n, int ncell) { return (int)(2 * (int64_t)n / ncell + 4 + 3) & ~3; }
@@ -257,7 +262,8 @@ int64_t Context::estimate_bytes(const rbmd_system_desc& d, const rbmd_params& p)
   const int64_t nke = p.coulomb != RBMD_COUL_NONE
                           ? (int64_t)(2 * p.kmax[0] + 1) * (2 * p.kmax[1] + 1) * (2 * p.kmax[2] + 1)
                           : 0;
-  const int64_t brho = (n + kRhoChunk - 1) / kRhoChunk;
+  const int64_t brho = (n + rho_chunk((int)n) - 1) / rho_chunk((int)n);
+  if (p.coulomb != RBMD_COUL_NONE) b += n * 32 + (n + kFarAtoms - 1) / kFarAtoms * 48;  // far forces and virial
   b += nk * 48 + nke * 48 + brho * 16 * std::max(nk, nke);
   b += (int64_t)(d.n_bonds * 2 + d.n_angles * 3 + d.n_dihedrals * 4) * 48 +
        (int64_t)(d.n_bonds + d.n_angles + d.n_dihedrals) * 76;
@@ -502,7 +508,8 @@ int Context::add_system(const rbmd_system_desc& d, const rbmd_params& p, int32_t
   D.cell_stride = (D.ncell_cap + 3) & ~3;
   D.blocks_pair = D.dense ? tile_blocks(D) : (n + kPairWarps - 1) / kPairWarps;
   D.blocks_atom = (n + kAtomBlock - 1) / kAtomBlock;
-  D.blocks_rho = (n + kRhoChunk - 1) / kRhoChunk;
+  D.rho_chunk = rho_chunk(n);
+  D.blocks_rho = (n + D.rho_chunk - 1) / D.rho_chunk;
   D.blocks_tri = (D.n_triples + 127) / 128;
 
   // Ewald k lists
@@ -731,6 +738,8 @@ int Context::add_system(const rbmd_system_desc& d, const rbmd_params& p, int32_t
     }
   }
   if (D.coul != RBMD_COUL_NONE) {
+    D.ffar = (double4*)dal(sizeof(double4) * n);
+    D.far_vir = (double*)dal(sizeof(double) * 6 * ((n + kFarAtoms - 1) / kFarAtoms));
     D.km = (int*)dal(sizeof(int) * 3 * std::max(1, D.P));
     D.kv = (double4*)dal(sizeof(double4) * std::max(1, nk_force));
     D.rhok = (double*)dal(sizeof(double) * 2 * std::max(1, nk_force));
@@ -931,7 +940,7 @@ Context::BatchRec* Context::build_batch(const std::vector<System*>& group, int& 
     else
       for (int k = 0; k < D.n; k += kPairWarps) wp.push_back(make_int2(s->slot, k));
     for (int k = 0; k < D.ncell_cap; k += kCellBlock) wc.push_back(make_int2(s->slot, k));
-    for (int k = 0; k < D.n; k += kRhoChunk) wr.push_back(make_int2(s->slot, k));
+    for (int k = 0; k < D.n; k += D.rho_chunk) wr.push_back(make_int2(s->slot, k));
     for (int k = 0; k < D.n_triples; k += 128) wt.push_back(make_int2(s->slot, k));
     for (int k = 0; k < D.n_bonds + D.n_angles + D.n_dihedrals; k += 128) wm.push_back(make_int2(s->slot, k));
   }
@@ -1048,6 +1057,7 @@ void Context::enqueue_forces(const Batch& b, FinalMode mode, int virial) {
   if (b.coul != RBMD_COUL_NONE) timed("rho", 0, [&] { launch_rho(b, stream, b.coul == RBMD_COUL_EWALD); });
   if (b.has_bonded) timed("bonded", 0, [&] { launch_bonded(b, stream, virial); });
   timed(pair_name(b), (double)b.natoms, [&] { launch_pair(b, stream, virial); });
+  timed("far", (double)b.natoms, [&] { launch_far(b, stream, virial); });
   timed("final", (double)b.natoms, [&] { launch_final(b, stream, mode, virial); });
 }
 
@@ -1063,6 +1073,7 @@ void Context::enqueue_step(const Batch& b) {
   const int vir = b.npt;
   if (b.has_bonded) timed("bonded", 0, [&] { launch_bonded(b, stream, vir); });
   timed(pair_name(b), (double)b.natoms, [&] { launch_pair(b, stream, vir); });
+  timed("far", (double)b.natoms, [&] { launch_far(b, stream, vir); });
   timed("final", (double)b.natoms, [&] { launch_final(b, stream, kFinalKick, vir); });
   if (b.has_shake) {
     timed("rattle", 0, [&] { launch_rattle(b, stream); });
@@ -1317,6 +1328,7 @@ int Context::get_thermo_many(const int32_t* ids, int nsys, rbmd_thermo* outs) {
     if (b.coul == RBMD_COUL_RBE) launch_rbe_sample(b, stream);
     if (b.coul != RBMD_COUL_NONE) launch_rho(b, stream, b.coul == RBMD_COUL_EWALD);
     if (b.has_bonded) launch_bonded(b, stream, 1);
+    launch_far(b, stream, 1);
     launch_pair(b, stream, 1);
     launch_final(b, stream, kFinalForceOnly, 1);
     launch_energy(b, stream);

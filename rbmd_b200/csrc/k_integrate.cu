@@ -264,7 +264,131 @@ __global__ void k_bonded(const SysDev* __restrict__ S, const int2* __restrict__ 
 }
 
 // ------------------------------------------------------------------ final force + kick
+// Sum of v over the block, in a fixed order (lanes by butterfly, warps in turn); every thread gets it.
+__device__ inline double block_sum(double v, double* s_w) {
+  v = warp_sum(v);
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0) s_w[threadIdx.x >> 5] = v;
+  __syncthreads();
+  double t = 0.0;
+  for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += s_w[w];
+  return t;
+}
+
+// Far force of every atom (RBE or Ewald) into ffar.  A block takes kFarAtoms atoms and four threads
+// share an atom's k vectors, a quarter each: the sine / cosine loop is the kernel's time, and one thread
+// per atom made it a chain of P evaluations on an SM per 256 atoms (inside the force assembly, which
+// took 49 us for 8000 atoms and P = 200 in FP64, 25 us for 9000 and P = 100 in mixed precision).  A
+// kernel of its own, so that the split costs the assembly's memory-bound part no occupancy.  The
+// quarters are added in order: the sum does not depend on the launch.
 template <bool MIXED, bool VIRIAL>
+__global__ void __launch_bounds__(kAtomBlock, 4) k_far(const SysDev* __restrict__ S, const int2* __restrict__ work) {
+  constexpr int kParts = kAtomBlock / kFarAtoms;
+  constexpr int kK = 256;  // k vectors staged at a time
+  static_assert(kFarAtoms % 32 == 0, "a part is whole warps");
+  const int2 wk = work[blockIdx.x];
+  const SysDev& s = S[wk.x];
+  const int first = wk.y + blockIdx.y * kFarAtoms;
+  if (first >= s.n) return;  // block-uniform
+  const int part = threadIdx.x / kFarAtoms, a = threadIdx.x % kFarAtoms;
+  const int i = first + a;
+  const bool in = i < s.n;
+  __shared__ double4 s_k[kK];
+  __shared__ double2 s_r[kK];
+  __shared__ float4 s_kf[kK];
+  __shared__ float2 s_rf[kK];
+  float4* s_kk = reinterpret_cast<float4*>(s_k);  // mixed precision: FP32 k vectors (s_k unused)
+  __shared__ double s_far[3][kAtomBlock];
+  const double4 xi = in ? s.x[i] : make_double4(0, 0, 0, 0);
+  const int nk = s.coul == RBMD_COUL_RBE ? s.P : s.nk_ewald;
+  double fx = 0, fy = 0, fz = 0;
+  double vir[6] = {0, 0, 0, 0, 0, 0};
+  float gx = 0.f, gy = 0.f, gz = 0.f;
+  const float ux = (float)(xi.x / s.L[0]), uy = (float)(xi.y / s.L[1]), uz = (float)(xi.z / s.L[2]);
+  for (int k0 = 0; k0 < nk; k0 += kK) {
+    const int nch = min(kK, nk - k0);
+    __syncthreads();
+    for (int k = threadIdx.x; k < nch; k += blockDim.x) {
+      const double4 kv = s.kv[k0 + k];
+      const double re = s.rhok[2 * (k0 + k)], im = s.rhok[2 * (k0 + k) + 1];
+      if (MIXED) {
+        const int l = k0 + k;
+        s_kf[k] = make_float4((float)s.km[3 * l], (float)s.km[3 * l + 1], (float)s.km[3 * l + 2], (float)kv.w);
+        s_rf[k] = make_float2((float)re, (float)im);
+        s_kk[k] = make_float4((float)kv.x, (float)kv.y, (float)kv.z, 0.0f);
+      } else {
+        s_k[k] = kv;
+        s_r[k] = make_double2(re, im);
+      }
+    }
+    __syncthreads();
+    const int ka = nch * part / kParts, kb = nch * (part + 1) / kParts;  // this part's k vectors
+    if (in) {
+      if (MIXED) {
+        const float q = (float)xi.w;
+        for (int k = ka; k < kb; ++k) {
+          const float4 m = s_kf[k];
+          float ph = m.x * ux + m.y * uy + m.z * uz;
+          ph -= __fsub_rn(__fadd_rn(ph, 12582912.0f), 12582912.0f);  // rint on the FMA pipe, |ph| < 2^22
+          float sn, cs;
+          __sincosf(6.28318531f * ph, &sn, &cs);  // hardware sin / cos: |2 pi ph| <= pi
+          const float2 r = s_rf[k];
+          const float Fs = m.w * q * (cs * r.y - sn * r.x);
+          const float4 kf = s_kk[k];
+          gx += Fs * kf.x;
+          gy += Fs * kf.y;
+          gz += Fs * kf.z;
+        }
+      } else {
+        for (int k = ka; k < kb; ++k) {
+          const double4 kv = s_k[k];
+          const double2 r = s_r[k];
+          const double dot = kv.x * xi.x + kv.y * xi.y + kv.z * xi.z;
+          double sn, cs;
+          sincos(dot, &sn, &cs);
+          const double Fs = kv.w * xi.w * (cs * r.y - sn * r.x);
+          fx += Fs * kv.x;
+          fy += Fs * kv.y;
+          fz += Fs * kv.z;
+          if (VIRIAL) {  // ComputeKspaceVirial, ExecForceFunction.h:397-410
+            vir[0] += (xi.x * kv.x + xi.x * kv.x) * Fs;
+            vir[1] += (xi.y * kv.y + xi.y * kv.y) * Fs;
+            vir[2] += (xi.z * kv.z + xi.z * kv.z) * Fs;
+            vir[3] += (xi.x * kv.y + xi.y * kv.x) * Fs;
+            vir[4] += (xi.x * kv.z + xi.z * kv.x) * Fs;
+            vir[5] += (xi.y * kv.z + xi.z * kv.y) * Fs;
+          }
+        }
+      }
+    }
+  }
+  s_far[0][threadIdx.x] = MIXED ? (double)gx : fx;
+  s_far[1][threadIdx.x] = MIXED ? (double)gy : fy;
+  s_far[2][threadIdx.x] = MIXED ? (double)gz : fz;
+  __syncthreads();
+  const double sc = (s.coul == RBMD_COUL_RBE ? s.S / s.P : 1.0) * s.qqr2e;
+  if (in && part == 0) {
+    double F[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      double t = 0.0;
+      for (int p = 0; p < kParts; ++p) t += s_far[k][p * kFarAtoms + a];
+      F[k] = t * sc;
+    }
+    s.ffar[i] = make_double4(F[0], F[1], F[2], 0.0);
+  }
+  if (VIRIAL) {  // the block's k-space virial, added up by the force assembly's last block
+    __shared__ double s_w[kAtomBlock / 32];
+    for (int k = 0; k < 6; ++k) {
+      const double t = block_sum(vir[k], s_w);
+      if (threadIdx.x == 0) s.far_vir[(size_t)(first / kFarAtoms) * 6 + k] = t * sc;
+    }
+  }
+}
+
+// Force assembly, half kick, kinetic energy and, in the system's last block, the thermostat.  Bound by
+// memory (240 B per atom and the gathers of the bonded terms).
+template <bool VIRIAL>
 __global__ void __launch_bounds__(kAtomBlock, 4)
 k_final(const SysDev* __restrict__ S, const int2* __restrict__ work, int mode) {
   const int2 wk = work[blockIdx.x];
@@ -272,11 +396,6 @@ k_final(const SysDev* __restrict__ S, const int2* __restrict__ work, int mode) {
   const int i = wk.y + threadIdx.x;
   const bool act = i < s.n;
   SysState* st = s.st;
-  __shared__ double4 s_k[256];
-  __shared__ double2 s_r[256];
-  __shared__ float4 s_kf[256];
-  __shared__ float2 s_rf[256];
-  float4* s_kk = reinterpret_cast<float4*>(s_k);  // mixed precision: FP32 k vectors (s_k unused)
   __shared__ double s_part[kAtomBlock / 32][8];
 
   double4 xi = act ? s.x[i] : make_double4(0, 0, 0, 0);
@@ -294,80 +413,11 @@ k_final(const SysDev* __restrict__ S, const int2* __restrict__ work, int mode) {
     F[2] -= st->fmean[2];
   }
   double vir[6] = {0, 0, 0, 0, 0, 0};
-  // ---- far field
-  const bool far = (s.ff == RBMD_FF_LJ_CUT_COUL_LONG || s.ff == RBMD_FF_CVFF) && s.coul != RBMD_COUL_NONE;
-  if (far) {
-    const int nk = s.coul == RBMD_COUL_RBE ? s.P : s.nk_ewald;
-    double fx = 0, fy = 0, fz = 0;
-    float gx = 0.f, gy = 0.f, gz = 0.f;
-    const float ux = (float)(xi.x / s.L[0]), uy = (float)(xi.y / s.L[1]), uz = (float)(xi.z / s.L[2]);
-    for (int k0 = 0; k0 < nk; k0 += 256) {
-      const int nch = min(256, nk - k0);
-      __syncthreads();
-      for (int k = threadIdx.x; k < nch; k += blockDim.x) {
-        const double4 kv = s.kv[k0 + k];
-        const double re = s.rhok[2 * (k0 + k)], im = s.rhok[2 * (k0 + k) + 1];
-        if (MIXED) {
-          const int l = k0 + k;
-          s_kf[k] = make_float4((float)s.km[3 * l], (float)s.km[3 * l + 1], (float)s.km[3 * l + 2], (float)kv.w);
-          s_rf[k] = make_float2((float)re, (float)im);
-          s_kk[k] = make_float4((float)kv.x, (float)kv.y, (float)kv.z, 0.0f);
-        } else {
-          s_k[k] = kv;
-          s_r[k] = make_double2(re, im);
-        }
-      }
-      __syncthreads();
-      if (act) {
-        if (MIXED) {
-          const float q = (float)xi.w;
-          for (int k = 0; k < nch; ++k) {
-            const float4 m = s_kf[k];
-            float ph = m.x * ux + m.y * uy + m.z * uz;
-            ph -= __fsub_rn(__fadd_rn(ph, 12582912.0f), 12582912.0f);  // rint on the FMA pipe, |ph| < 2^22
-            float sn, cs;
-            __sincosf(6.28318531f * ph, &sn, &cs);  // hardware sin / cos: |2 pi ph| <= pi
-            const float2 r = s_rf[k];
-            const float Fs = m.w * q * (cs * r.y - sn * r.x);
-            const float4 kf = s_kk[k];
-            gx += Fs * kf.x;
-            gy += Fs * kf.y;
-            gz += Fs * kf.z;
-          }
-        } else {
-          for (int k = 0; k < nch; ++k) {
-            const double4 kv = s_k[k];
-            const double2 r = s_r[k];
-            const double dot = kv.x * xi.x + kv.y * xi.y + kv.z * xi.z;
-            double sn, cs;
-            sincos(dot, &sn, &cs);
-            const double Fs = kv.w * xi.w * (cs * r.y - sn * r.x);
-            fx += Fs * kv.x;
-            fy += Fs * kv.y;
-            fz += Fs * kv.z;
-            if (VIRIAL) {  // ComputeKspaceVirial, ExecForceFunction.h:397-410
-              vir[0] += (xi.x * kv.x + xi.x * kv.x) * Fs;
-              vir[1] += (xi.y * kv.y + xi.y * kv.y) * Fs;
-              vir[2] += (xi.z * kv.z + xi.z * kv.z) * Fs;
-              vir[3] += (xi.x * kv.y + xi.y * kv.x) * Fs;
-              vir[4] += (xi.x * kv.z + xi.z * kv.x) * Fs;
-              vir[5] += (xi.y * kv.z + xi.z * kv.y) * Fs;
-            }
-          }
-        }
-      }
-    }
-    if (MIXED) {
-      fx = gx;
-      fy = gy;
-      fz = gz;
-    }
-    const double sc = (s.coul == RBMD_COUL_RBE ? s.S / s.P : 1.0) * s.qqr2e;
-    F[0] = fx * sc + F[0];
-    F[1] = fy * sc + F[1];
-    F[2] = fz * sc + F[2];
-    if (VIRIAL)
-      for (int k = 0; k < 6; ++k) vir[k] *= sc;
+  if (act && s.coul != RBMD_COUL_NONE) {  // far force (k_far)
+    const double4 ff = s.ffar[i];
+    F[0] = ff.x + F[0];
+    F[1] = ff.y + F[1];
+    F[2] = ff.z + F[2];
   }
   if (act) {
     // ---- intramolecular Coulomb exclusion (CVFF + RBL + special bonds)
@@ -447,19 +497,25 @@ k_final(const SysDev* __restrict__ S, const int2* __restrict__ work, int mode) {
     s.atom_part[(size_t)blk * 8 + threadIdx.x] = t;
   }
   if (arrive_last(&st->counter[2], (unsigned)s.blocks_atom)) {
-    __shared__ double s_tot[8];
-    if (threadIdx.x < 8) {
+    double* s_w = &s_part[0][0];  // block_sum's scratch
+    double s_tot[7] = {0, 0, 0, 0, 0, 0, 0}, tv[6] = {0, 0, 0, 0, 0, 0};
+    const int nsum = VIRIAL ? 7 : 1;
+    for (int k = 0; k < nsum; ++k) {
       double t = 0.0;
-      for (int b = 0; b < s.blocks_atom; ++b) t += __ldcg(&s.atom_part[(size_t)b * 8 + threadIdx.x]);
-      s_tot[threadIdx.x] = t;
+      for (int b = threadIdx.x; b < s.blocks_atom; b += kAtomBlock) t += __ldcg(&s.atom_part[(size_t)b * 8 + k]);
+      s_tot[k] = block_sum(t, s_w);
     }
-    __syncthreads();
+    if (VIRIAL) {  // the bonded terms' virial and the far force's
+      const int nt = s.term_vir ? s.n_bonds + s.n_angles + s.n_dihedrals : 0;
+      const int nf = s.coul != RBMD_COUL_NONE ? (s.n + kFarAtoms - 1) / kFarAtoms : 0;
+      for (int t = threadIdx.x; t < nt; t += kAtomBlock)
+        for (int k = 0; k < 6; ++k) tv[k] += s.term_vir[6 * (size_t)t + k];
+      for (int t = threadIdx.x; t < nf; t += kAtomBlock)
+        for (int k = 0; k < 6; ++k) tv[k] += s.far_vir[6 * (size_t)t + k];
+      for (int k = 0; k < 6; ++k) tv[k] = block_sum(tv[k], s_w);
+    }
     if (threadIdx.x == 0) {
       if (VIRIAL) {
-        double tv[6] = {0, 0, 0, 0, 0, 0};
-        if (s.term_vir)
-          for (int t = 0; t < s.n_bonds + s.n_angles + s.n_dihedrals; ++t)
-            for (int k = 0; k < 6; ++k) tv[k] += s.term_vir[6 * (size_t)t + k];
         for (int k = 0; k < 6; ++k) st->virial[k] = st->virial[k] + s_tot[1 + k] + tv[k];
       }
       if (mode == kFinalInit) {
@@ -861,14 +917,18 @@ void launch_bonded(const Batch& b, cudaStream_t st, int virial) {
   note_launch();
 }
 
+void launch_far(const Batch& b, cudaStream_t st, int virial) {
+  if (b.coul == RBMD_COUL_NONE) return;
+  const dim3 grid(b.atom.n, kAtomBlock / kFarAtoms);
+  if (virial) k_far<false, true><<<grid, kAtomBlock, 0, st>>>(b.sys, b.atom.d);
+  else if (b.prec == RBMD_PREC_MIXED && b.coul == RBMD_COUL_RBE) k_far<true, false><<<grid, kAtomBlock, 0, st>>>(b.sys, b.atom.d);
+  else k_far<false, false><<<grid, kAtomBlock, 0, st>>>(b.sys, b.atom.d);
+  note_launch();
+}
+
 void launch_final(const Batch& b, cudaStream_t st, FinalMode mode, int virial) {
-  if (virial) {
-    k_final<false, true><<<b.atom.n, kAtomBlock, 0, st>>>(b.sys, b.atom.d, (int)mode);
-  } else if (b.prec == RBMD_PREC_MIXED && b.coul == RBMD_COUL_RBE) {
-    k_final<true, false><<<b.atom.n, kAtomBlock, 0, st>>>(b.sys, b.atom.d, (int)mode);
-  } else {
-    k_final<false, false><<<b.atom.n, kAtomBlock, 0, st>>>(b.sys, b.atom.d, (int)mode);
-  }
+  if (virial) k_final<true><<<b.atom.n, kAtomBlock, 0, st>>>(b.sys, b.atom.d, (int)mode);
+  else k_final<false><<<b.atom.n, kAtomBlock, 0, st>>>(b.sys, b.atom.d, (int)mode);
   note_launch();
 }
 

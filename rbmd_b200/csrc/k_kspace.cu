@@ -188,39 +188,67 @@ __global__ void __launch_bounds__(kRbeThreads) k_rbe_sample(const SysDev* __rest
   }
 }
 
-// Structure factor over a chunk of kRhoChunk atoms per block, every thread owning k indices; the
-// last block of the system sums the chunk partials in chunk order (deterministic, FP64).
+// Structure factor over a chunk of a system's atoms per block; the last block of the system sums the
+// chunk partials in chunk order (deterministic, FP64).  Bound by the sine / cosine arithmetic (SFU in
+// mixed precision, FP64 otherwise) once every SM has blocks, and by how many have before that: the
+// block takes the k indices 32 at a time, one per lane, and its eight warps an eighth of the chunk's
+// atoms each, so that a small system's few thousand atom-k terms spread over 64-atom blocks and all
+// their warps (one k per thread over 256 atoms left 100 of 256 threads, and an SM per 256 atoms, with
+// work).  The chunk length depends on the system alone, so its sums do not depend on the batch.
+constexpr int kRhoWarps = 8;
+
 template <bool MIXED, bool ENERGY>
-__global__ void __launch_bounds__(256) k_rho(const SysDev* __restrict__ S, const int2* __restrict__ work) {
+__global__ void __launch_bounds__(kRhoWarps * 32) k_rho(const SysDev* __restrict__ S, const int2* __restrict__ work) {
   const int2 wk = work[blockIdx.x];
   const SysDev& s = S[wk.x];
   const int nk = ENERGY ? s.nk_e : (s.coul == RBMD_COUL_RBE ? s.P : s.nk_ewald);
   const double4* kv = ENERGY ? s.kv_e : s.kv;
-  __shared__ double4 s_x[kRhoChunk];
-  __shared__ float4 s_u[kRhoChunk];
-  const int a0 = wk.y;
-  const int na = min(kRhoChunk, s.n - a0);
+  constexpr bool kF32 = MIXED && !ENERGY;
+  __shared__ double4 s_x[kF32 ? 1 : kRhoChunk];
+  __shared__ float4 s_u[kF32 ? kRhoChunk : 1];
+  __shared__ double2 s_red[2][kRhoWarps][32];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int chunk = s.rho_chunk, a0 = wk.y;
+  const int na = min(chunk, s.n - a0);
   for (int k = threadIdx.x; k < na; k += blockDim.x) {
     const double4 p = s.x[a0 + k];
-    s_x[k] = p;
-    if (MIXED)
+    if (kF32)
       s_u[k] = make_float4((float)(p.x / s.L[0]), (float)(p.y / s.L[1]), (float)(p.z / s.L[2]), (float)p.w);
+    else
+      s_x[k] = p;
   }
   __syncthreads();
-  const int blk = a0 / kRhoChunk;
+  const int per = chunk / kRhoWarps;  // at most 32 atoms per warp
+  const int j0 = min(na, wid * per), j1 = min(na, j0 + per);
+  const int blk = a0 / chunk;
+  // the warps' sums of 32 k indices at l0: warp `who` adds them in warp order and hands them to `put`;
+  // two buffers in turn, so one barrier per 32 indices
+  auto gather = [&](int buf, int who, double re, double im, auto&& put) {
+    s_red[buf][wid][lane] = make_double2(re, im);
+    __syncthreads();
+    if (wid == who) {
+      double tr = 0.0, ti = 0.0;
+#pragma unroll
+      for (int w = 0; w < kRhoWarps; ++w) {
+        const double2 v = s_red[buf][w][lane];
+        tr += v.x;
+        ti += v.y;
+      }
+      put(tr, ti);
+    }
+  };
   double* part = s.rho_part + (size_t)blk * 2 * nk;
-  for (int l = threadIdx.x; l < nk; l += blockDim.x) {
-    const double4 k = kv[l];
+  for (int l0 = 0, turn = 0; l0 < nk; l0 += 32, ++turn) {
+    const int l = l0 + lane;
     double re = 0.0, im = 0.0;
-    if (MIXED && !ENERGY) {
-      // phase in turns m . (r / L), reduced to [-1/2, 1/2] before the FP32 sine and cosine (the
-      // SFU approximations, absolute error about 4e-7 on [-pi, pi])
-      const float mxr = (float)s.km[3 * l], myr = (float)s.km[3 * l + 1], mzr = (float)s.km[3 * l + 2];
-      // FP32 partial sums over 32 atoms, added in FP64 (the SFU, which also converts FP32 to
-      // FP64, is this loop's bottleneck); the nearest integer of the phase by the 1.5 * 2^23
-      // addition (round to nearest even, |ph| < 2^22), on the FMA pipe
-      for (int j0 = 0; j0 < na; j0 += 32) {
-        const int j1 = min(na, j0 + 32);
+    if (l < nk) {
+      if (kF32) {
+        // phase in turns m . (r / L), reduced to [-1/2, 1/2] before the FP32 sine and cosine (the
+        // SFU approximations, absolute error about 4e-7 on [-pi, pi]); FP32 partial sums over the
+        // warp's atoms (at most 32), added in FP64 (the SFU also converts FP32 to FP64); the nearest
+        // integer of the phase by the 1.5 * 2^23 addition (round to nearest even, |ph| < 2^22), on
+        // the FMA pipe
+        const float mxr = (float)s.km[3 * l], myr = (float)s.km[3 * l + 1], mzr = (float)s.km[3 * l + 2];
         float pr = 0.0f, pm = 0.0f;
         for (int j = j0; j < j1; ++j) {
           const float4 u = s_u[j];
@@ -231,45 +259,56 @@ __global__ void __launch_bounds__(256) k_rho(const SysDev* __restrict__ S, const
           pr += u.w * cs;
           pm += u.w * sn;
         }
-        re += (double)pr;
-        im += (double)pm;
-      }
-    } else {
-      for (int j = 0; j < na; ++j) {
-        const double4 p = s_x[j];
-        const double dot = k.x * p.x + k.y * p.y + k.z * p.z;
-        double sn, cs;
-        sincos(dot, &sn, &cs);
-        re += p.w * cs;
-        im += p.w * sn;
+        re = (double)pr;
+        im = (double)pm;
+      } else {
+        const double4 k = kv[l];
+        for (int j = j0; j < j1; ++j) {
+          const double4 p = s_x[j];
+          const double dot = k.x * p.x + k.y * p.y + k.z * p.z;
+          double sn, cs;
+          sincos(dot, &sn, &cs);
+          re += p.w * cs;
+          im += p.w * sn;
+        }
       }
     }
-    part[2 * l] = re;
-    part[2 * l + 1] = im;
+    gather(turn & 1, turn % kRhoWarps, re, im, [&](double tr, double ti) {
+      if (l < nk) {
+        part[2 * l] = tr;
+        part[2 * l + 1] = ti;
+      }
+    });
   }
   if (arrive_last(&s.st->counter[ENERGY ? 4 : 1], (unsigned)s.blocks_rho)) {
+    // every warp takes a run of the chunks, lanes 32 k indices
     double* out = ENERGY ? s.rhok_e : s.rhok;
     double esum = 0.0;
-    for (int l = threadIdx.x; l < nk; l += blockDim.x) {
+    const int seg = (s.blocks_rho + kRhoWarps - 1) / kRhoWarps;
+    const int b0 = wid * seg, b1 = min(s.blocks_rho, b0 + seg);
+    for (int l0 = 0, turn = 0; l0 < nk; l0 += 32, ++turn) {
+      const int l = l0 + lane;
       double re = 0.0, im = 0.0;
-      for (int b = 0; b < s.blocks_rho; ++b) {
-        re += __ldcg(&s.rho_part[(size_t)b * 2 * nk + 2 * l]);
-        im += __ldcg(&s.rho_part[(size_t)b * 2 * nk + 2 * l + 1]);
+      if (l < nk) {
+        const double2* p = reinterpret_cast<const double2*>(s.rho_part) + l;
+#pragma unroll 4
+        for (int b = b0; b < b1; ++b) {
+          const double2 v = __ldcg(&p[(size_t)b * nk]);
+          re += v.x;
+          im += v.y;
+        }
       }
-      out[2 * l] = re;
-      out[2 * l + 1] = im;
-      if (ENERGY) esum += kv[l].w * (re * re + im * im);
+      gather(turn & 1, 0, re, im, [&](double tr, double ti) {
+        if (l < nk) {
+          out[2 * l] = tr;
+          out[2 * l + 1] = ti;
+          if (ENERGY) esum += kv[l].w * (tr * tr + ti * ti);
+        }
+      });
     }
-    if (ENERGY) {
-      // fixed-order block reduction of the energy terms
-      __shared__ double s_e[256];
-      s_e[threadIdx.x] = esum;
-      __syncthreads();
-      if (threadIdx.x == 0) {
-        double t = 0.0;
-        for (int k = 0; k < (int)blockDim.x; ++k) t += s_e[k];
-        s.st->energy[6] = t;
-      }
+    if (ENERGY && wid == 0) {
+      esum = warp_sum(esum);
+      if (lane == 0) s.st->energy[6] = esum;
     }
   }
 }
@@ -282,14 +321,14 @@ void launch_rbe_sample(const Batch& b, cudaStream_t st) {
 void launch_rho(const Batch& b, cudaStream_t st, int ewald) {
   (void)ewald;
   if (b.prec == RBMD_PREC_MIXED && b.coul == RBMD_COUL_RBE)
-    k_rho<true, false><<<b.rho.n, 256, 0, st>>>(b.sys, b.rho.d);
+    k_rho<true, false><<<b.rho.n, kRhoWarps * 32, 0, st>>>(b.sys, b.rho.d);
   else
-    k_rho<false, false><<<b.rho.n, 256, 0, st>>>(b.sys, b.rho.d);
+    k_rho<false, false><<<b.rho.n, kRhoWarps * 32, 0, st>>>(b.sys, b.rho.d);
   note_launch();
 }
 
 void launch_ewald_energy(const Batch& b, cudaStream_t st) {
-  k_rho<false, true><<<b.rho.n, 256, 0, st>>>(b.sys, b.rho.d);
+  k_rho<false, true><<<b.rho.n, kRhoWarps * 32, 0, st>>>(b.sys, b.rho.d);
   note_launch();
 }
 

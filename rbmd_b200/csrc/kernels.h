@@ -57,6 +57,8 @@ void launch_pair(const Batch& b, cudaStream_t s, int virial);
 // Blocks of the persistent column kernel for `ncols` columns: resident blocks per SM x SMs of the
 // current device, fewer when the columns do not fill them (4 warps per block, a column per warp).
 int pair_col_grid(int ncols, int ff, int special, int near, bool strays);
+// Far forces (RBE, Ewald) from the structure factor, for launch_final to add.
+void launch_far(const Batch& b, cudaStream_t s, int virial);
 void launch_final(const Batch& b, cudaStream_t s, FinalMode mode, int virial);
 void launch_ke_thermostat(const Batch& b, cudaStream_t s);
 void launch_flush_vscale(const Batch& b, cudaStream_t s);
