@@ -258,6 +258,17 @@ __device__ inline int warp_incl_scan(int v, int lane) {
 
 __device__ inline unsigned lanemask_lt(int lane) { return (1u << lane) - 1u; }
 
+// Sum of v over the block, in a fixed order (lanes by butterfly, warps in turn); every thread gets it.
+__device__ inline double block_sum(double v, double* s_w) {
+  v = warp_sum(v);
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0) s_w[threadIdx.x >> 5] = v;
+  __syncthreads();
+  double t = 0.0;
+  for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += s_w[w];
+  return t;
+}
+
 // Last-block-done pattern: every block of a system calls this after writing its partials; the
 // block that arrives last gets true and may reduce all partials of the system in a fixed order.
 // The counter is reset by the last block, so the pattern needs no host-side clearing.

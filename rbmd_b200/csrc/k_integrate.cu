@@ -264,17 +264,6 @@ __global__ void k_bonded(const SysDev* __restrict__ S, const int2* __restrict__ 
 }
 
 // ------------------------------------------------------------------ final force + kick
-// Sum of v over the block, in a fixed order (lanes by butterfly, warps in turn); every thread gets it.
-__device__ inline double block_sum(double v, double* s_w) {
-  v = warp_sum(v);
-  __syncthreads();
-  if ((threadIdx.x & 31) == 0) s_w[threadIdx.x >> 5] = v;
-  __syncthreads();
-  double t = 0.0;
-  for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += s_w[w];
-  return t;
-}
-
 // Far force of every atom (RBE or Ewald) into ffar.  A block takes kFarAtoms atoms and four threads
 // share an atom's k vectors, a quarter each: the sine / cosine loop is the kernel's time, and one thread
 // per atom made it a chain of P evaluations on an SM per 256 atoms (inside the force assembly, which
@@ -583,9 +572,10 @@ __global__ void __launch_bounds__(kAtomBlock) k_ke_thermostat(const SysDev* __re
     s.atom_part[(size_t)blk * 8] = t;
   }
   if (arrive_last(&st->counter[5], (unsigned)s.blocks_atom)) {
+    double t = 0.0;
+    for (int b = threadIdx.x; b < s.blocks_atom; b += kAtomBlock) t += __ldcg(&s.atom_part[(size_t)b * 8]);
+    t = block_sum(t, s_w);
     if (threadIdx.x == 0) {
-      double t = 0.0;
-      for (int b = 0; b < s.blocks_atom; ++b) t += __ldcg(&s.atom_part[(size_t)b * 8]);
       compute_tempe(s, st, t);
       double c = 1.0;
       if (s.temp_ctrl == RBMD_TC_RESCALE) c = sqrt(s.t_start / st->temperature);
@@ -815,10 +805,13 @@ __global__ void __launch_bounds__(128, 3) k_shake(const SysDev* __restrict__ S, 
     s.tri_part[(size_t)blk * 6 + threadIdx.x] = t;
   }
   if (arrive_last(&st->counter[3], (unsigned)s.blocks_tri)) {
-    if (threadIdx.x < 6) {
-      double t = 0;
-      for (int b = 0; b < s.blocks_tri; ++b) t += __ldcg(&s.tri_part[(size_t)b * 6 + threadIdx.x]);
-      st->shake_virial[threadIdx.x] = t;
+    __shared__ double s_b[4];
+    double t6[6] = {0, 0, 0, 0, 0, 0};
+    for (int b = threadIdx.x; b < s.blocks_tri; b += 128)
+      for (int k = 0; k < 6; ++k) t6[k] += __ldcg(&s.tri_part[(size_t)b * 6 + k]);
+    for (int k = 0; k < 6; ++k) {
+      const double t = block_sum(t6[k], s_b);
+      if (threadIdx.x == 0) st->shake_virial[k] = t;
     }
   }
 }
