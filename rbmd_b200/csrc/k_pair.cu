@@ -682,24 +682,301 @@ __device__ inline void eval_pair_f32(const SysDev& s, int moli, float qi, int js
                                       ntypes, Lx, Ly, Lz, fx, fy, fz, gx, gy, gz, SPECIAL, s.near_tab);
 }
 
+__device__ inline void acc_zero(float (&ff)[6], PairAcc& a) {
+#pragma unroll
+  for (int k = 0; k < 6; ++k) ff[k] = 0.f;
+#pragma unroll
+  for (int k = 0; k < 3; ++k) a.f[k] = a.g[k] = 0.0;
+#pragma unroll
+  for (int k = 0; k < 6; ++k) a.vir[k] = 0.0;
+  a.rho = a.e0 = a.e1 = 0.0;
+}
+
+// What a warp of the lean traversal keeps in shared memory: its pair queue and its segment table.
+template <typename R>
+struct LeanShared {
+  int qj[64];
+  R qr[3][64];
+  int sa[64];   // segment first sorted index
+  int sb[64];   // segment begin in the flattened sequence
+  int se[64];   // segment end in the flattened sequence
+  R so[3][64];  // segment coordinate offsets
+};
+
+// The lean traversal of one atom (sorted index sidx) by one warp; the lanes' sums are left in ff (FP32
+// RBL modes, with tab the FP32 LJ factors of the type pairs) or in a.
+template <typename R, int MODE, bool SPECIAL, bool VIRIAL, bool NEAR>
+__device__ __forceinline__ void lean_atom(const SysDev& s, int sidx, int lane, LeanShared<R>& sh, const float* tab,
+                                          int& i, float (&ff)[6], PairAcc& a) {
+  using R4 = typename Vec4<R>::T;
+  constexpr bool F32 = sizeof(R) == 4 && (MODE == kLJ_RBL || MODE == kCOUL_RBL);
+  const unsigned FULL = 0xffffffffu;
+  const int ntypes = s.ntypes;
+  const int dx = s.dims[0], dy = s.dims[1], dz = s.dims[2];
+  const double d0 = s.d[0], d1 = s.d[1], d2c = s.d[2];
+  const int4 mi = __ldg(&s.smeta[sidx]);
+  i = mi.x;
+  const int ti = mi.y, moli = mi.z;
+  const double4 xi = ldg4(&s.sx[sidx]);
+  const R4 pi4 = load_sorted<R>(s, sidx);
+  const R pix = pi4.x, piy = pi4.y, piz = pi4.z;
+  // home cell by truncation and NOT clamped (InWhichCell, ExecPointLocator.h:271-274): an atom
+  // that a step left outside the box walks the neighbourhood of its unclamped cell, every
+  // neighbour cell wrapped by a true modulo below
+  const int c0 = (int)((xi.x - s.lo[0]) / d0);
+  const int c1 = (int)((xi.y - s.lo[1]) / d1);
+  const int c2 = (int)((xi.z - s.lo[2]) / d2c);
+  const double fpi = (MODE == kEAM_FORCE) ? s.eam_fp[i] : 0.0;
+  int nsp = 0;
+  const int* spi = nullptr;
+  const double* spw = nullptr;
+  if (SPECIAL) {
+    const int b = s.sp_off[i];
+    nsp = s.sp_off[i + 1] - b;
+    spi = s.sp_ids + b;
+    spw = s.sp_w + b;
+  }
+  const bool rbl = (MODE == kLJ_RBL || MODE == kCOUL_RBL ||
+                    ((MODE == kEAM_RHO || MODE == kEAM_FORCE) && s.neigh == RBMD_NEIGH_RBL));
+  const int pice = rbl ? s.pice : 1;
+  int nsh_mod = 0;  // running shell index modulo pice
+  if (rbl && s.rbl_mode == RBMD_RBL_PHILOX && pice > 1) {
+    uint32_t o[4];
+    philox4x32_10((uint32_t)i, 0u, (uint32_t)s.st->step, kTagRblOffset, s.seed_lo, s.seed_hi, o);
+    nsh_mod = (int)(o[0] % (uint32_t)pice);
+  }
+  uint32_t base_mask = 0;  // bits 0, pice, 2 pice, ... below 32
+  for (int k = 0; k < 32; k += pice) base_mask |= (1u << k);
+  const R rc2 = (R)s.rc2, rs2 = (R)s.rs2;
+  const int nc = s.nc, side = 2 * nc + 1, nrows = side * side;
+  // conservative culling radius: cells farther than rc from i (with a margin for atoms outside
+  // their cell: at least the farthest an atom lay outside its binned cell plus the largest SHAKE
+  // displacement since the cell list was built) cannot hold a core or shell atom; cells of atoms
+  // SHAKE wrapped across the box (they sit on the far side of it) are never culled, and beyond
+  // kMaxMigrated of them nothing is
+  const double margin =
+      fmax(0.1 * fmin(d0, fmin(d1, d2c)), 1.001 * ((double)__uint_as_float(s.st->shake_disp_bits) +
+                                                   (double)__uint_as_float(s.st->out_bits)));
+  const int mig_n = s.st->mig_n;
+  const double cut2 = s.rc2;
+  const double lo0 = s.lo[0], lo1 = s.lo[1], lo2 = s.lo[2];
+  const float spice = (float)pice;
+  const float fsa = (float)sqrt(s.alpha), falpha = (float)s.alpha;
+  const float fLx = (float)s.L[0], fLy = (float)s.L[1], fLz = (float)s.L[2];
+  const float frc2 = (float)s.rc2, frs2 = (float)s.rs2;
+  int head = 0, qn = 0;
+
+  auto flush = [&](int cnt) {
+    if (lane < cnt) {
+      const int slot = (head + lane) & 63;
+      int js = sh.qj[slot];
+      const bool core = js >= 0;
+      if (!core) js = ~js;
+      if (F32) {
+        eval_pair_f32<MODE, SPECIAL, NEAR>(s, moli, (float)xi.w, js, core, (float)sh.qr[0][slot],
+                                     (float)sh.qr[1][slot], (float)sh.qr[2][slot], ti, spi, spw, nsp,
+                                     spice, frc2, frs2, fsa, falpha, tab, ntypes, fLx, fLy, fLz, ff[0], ff[1], ff[2], ff[3], ff[4], ff[5]);
+      } else {
+        eval_pair<R, MODE, SPECIAL, VIRIAL, NEAR>(s, i, ti, moli, xi.w, fpi, js, core, sh.qr[0][slot],
+                                            sh.qr[1][slot], sh.qr[2][slot], spi, spw, nsp, (R)pice, a);
+      }
+    }
+    head = (head + cnt) & 63;
+    qn -= cnt;
+  };
+
+  // rows per segment table: 32 of at most two ranges each, or 21 of at most three when the box
+  // holds fewer than 2 nc + 1 cells in z (the table holds 64)
+  const int group = dz >= side ? 32 : 21;
+  for (int r0 = 0; r0 < nrows; r0 += group) {
+    // ---- segment table of rows r0 .. r0 + group - 1 (one row per lane)
+    const int r = r0 + lane;
+    int nseg = 0, cnt = 0;
+    int sa0 = 0, sa1 = 0, sa2 = 0, n0c = 0, n1c = 0, n2c = 0;
+    R oxv = R(0), oyv = R(0), oz0 = R(0), oz1 = R(0), oz2 = R(0);
+    if (lane < group && r < nrows) {
+      const int da = r / side - nc, db = r % side - nc;
+      int n0 = c0 + da, n1 = c1 + db;
+      int w0 = ((n0 % dx) + dx) % dx;
+      int w1 = ((n1 % dy) + dy) % dy;
+      const double ox = d0 * (double)(w0 - n0), oy = d1 * (double)(w1 - n1);
+      oxv = (R)ox;
+      oyv = (R)oy;
+      // squared gap between i and the column of cells (unwrapped frame), shrunk by the margin
+      const double bx0 = lo0 + n0 * d0 - margin, bx1 = lo0 + (n0 + 1) * d0 + margin;
+      const double by0 = lo1 + n1 * d1 - margin, by1 = lo1 + (n1 + 1) * d1 + margin;
+      const double gx = fmax(0.0, fmax(bx0 - xi.x, xi.x - bx1));
+      const double gy = fmax(0.0, fmax(by0 - xi.y, xi.y - by1));
+      const double gxy = gx * gx + gy * gy;
+      int elo = nc + 1, ehi = -nc - 1;
+      if (gxy < cut2) {
+        for (int de = -nc; de <= nc; ++de) {
+          const int n2 = c2 + de;
+          const double bz0 = lo2 + n2 * d2c - margin, bz1 = lo2 + (n2 + 1) * d2c + margin;
+          const double gz = fmax(0.0, fmax(bz0 - xi.z, xi.z - bz1));
+          if (gxy + gz * gz < cut2) {
+            elo = min(elo, de);
+            ehi = max(ehi, de);
+          }
+        }
+      }
+      if (mig_n > kMaxMigrated) {
+        elo = -nc;
+        ehi = nc;
+      } else {
+        for (int m = 0; m < mig_n; ++m) {
+          const int cm = __ldg(&s.st->mig_cell[m]) - dz * (w1 + dy * w0);
+          if (cm < 0 || cm >= dz) continue;  // not in this row's column
+          for (int de = -nc; de <= nc; ++de)
+            if ((((c2 + de) % dz) + dz) % dz == cm) {
+              elo = min(elo, de);
+              ehi = max(ehi, de);
+            }
+        }
+      }
+      {
+        if (elo <= ehi) {
+          // unwrapped z cells [z0, z1] (len <= 2 nc + 1 <= 2 dz - 1 of them) start in the
+          // periodic copy q = floor(z0 / dz); they map to wrapped cells [zw, zw + len) when that
+          // stays below dz, else to [zw, dz), then [0, rest) of the next copy, or [0, dz) and
+          // [0, rest - dz) of the two next when the stencil is longer than the box.  The shift of
+          // a cell is d * (wrapped - unwrapped) = -d dz q, -d dz (q + 1), -d dz (q + 2).
+          const int base = dz * (w1 + dy * w0);
+          const int z0 = c2 + elo, len = ehi - elo + 1;
+          const int zw = ((z0 % dz) + dz) % dz;
+          const int q = (z0 - zw) / dz;
+          sa0 = __ldg(&s.cell_start[base + zw]);
+          oz0 = (R)(-d2c * (double)dz * (double)q);
+          if (zw + len <= dz) {
+            n0c = __ldg(&s.cell_start[base + zw + len]) - sa0;
+            nseg = 1;
+          } else {
+            n0c = __ldg(&s.cell_start[base + dz]) - sa0;
+            const int rest = zw + len - dz;
+            sa1 = __ldg(&s.cell_start[base]);
+            oz1 = (R)(-d2c * (double)dz * (double)(q + 1));
+            if (rest <= dz) {
+              n1c = __ldg(&s.cell_start[base + rest]) - sa1;
+              nseg = 2;
+            } else {
+              n1c = __ldg(&s.cell_start[base + dz]) - sa1;
+              sa2 = sa1;
+              n2c = __ldg(&s.cell_start[base + rest - dz]) - sa2;
+              oz2 = (R)(-d2c * (double)dz * (double)(q + 2));
+              nseg = 3;
+            }
+          }
+          cnt = n0c + n1c + n2c;
+        }
+      }
+    }
+    const int seg_incl = warp_incl_scan(nseg, lane);
+    const int cnt_incl = warp_incl_scan(cnt, lane);
+    const int nsegs = __shfl_sync(FULL, seg_incl, 31);
+    const int total = __shfl_sync(FULL, cnt_incl, 31);
+    {
+      int slot = seg_incl - nseg, beg = cnt_incl - cnt;
+      if (nseg >= 1) {
+        sh.sa[slot] = sa0;
+        sh.sb[slot] = beg;
+        sh.se[slot] = beg + n0c;
+        sh.so[0][slot] = oxv;
+        sh.so[1][slot] = oyv;
+        sh.so[2][slot] = oz0;
+      }
+      if (nseg >= 2) {
+        sh.sa[slot + 1] = sa1;
+        sh.sb[slot + 1] = beg + n0c;
+        sh.se[slot + 1] = beg + n0c + n1c;
+        sh.so[0][slot + 1] = oxv;
+        sh.so[1][slot + 1] = oyv;
+        sh.so[2][slot + 1] = oz1;
+      }
+      if (nseg == 3) {
+        sh.sa[slot + 2] = sa2;
+        sh.sb[slot + 2] = beg + n0c + n1c;
+        sh.se[slot + 2] = beg + n0c + n1c + n2c;
+        sh.so[0][slot + 2] = oxv;
+        sh.so[1][slot + 2] = oyv;
+        sh.so[2][slot + 2] = oz2;
+      }
+    }
+    __syncwarp();
+    // ---- candidates of the flattened sequence, 32 per iteration
+    int seg = 0;
+    for (int base = 0; base < total; base += 32) {
+      const int p = base + lane;
+      const bool valid = p < total;
+      bool core = false, shell = false;
+      R rx = R(0), ry = R(0), rz = R(0);
+      int js = 0;
+      if (valid) {
+        while (p >= sh.se[seg]) ++seg;
+        js = sh.sa[seg] + (p - sh.sb[seg]);
+        const R4 pj = load_sorted<R>(s, js);
+        rx = (pj.x - sh.so[0][seg]) - pix;
+        ry = (pj.y - sh.so[1][seg]) - piy;
+        rz = (pj.z - sh.so[2][seg]) - piz;
+        const R dd = add_rn(add_rn(mul_rn(rx, rx), mul_rn(ry, ry)), mul_rn(rz, rz));
+        if (rbl) {
+          shell = (rc2 - dd > R(0.0001) && dd - rs2 > R(0.0001));
+          core = !shell && (rs2 - dd > R(0.0001) && dd > R(0.0001));
+        } else {
+          core = (rc2 - dd > R(0.0001) && dd > R(0.0001));
+        }
+        if constexpr (sizeof(R) == 4) {
+          if (f32_banded(s, (float)dd))
+            classify_fp64(s, xi.x, xi.y, xi.z, js, (int)rintf((float)(sh.so[0][seg] / d0)),
+                          (int)rintf((float)(sh.so[1][seg] / d1)), (int)rintf((float)(sh.so[2][seg] / d2c)),
+                          rbl, core, shell);
+        }
+      }
+      bool sel = core;
+      if (rbl) {
+        if (pice == 1) {
+          sel = core || shell;
+        } else {
+          const unsigned sm = __ballot_sync(FULL, shell);
+          const int phase = nsh_mod == 0 ? 0 : pice - nsh_mod;
+          const uint32_t mask = phase < 32 ? (base_mask << phase) : 0u;
+          const int pre = __popc(sm & lanemask_lt(lane));
+          sel = core || (shell && ((mask >> pre) & 1u));
+          nsh_mod += __popc(sm);
+          nsh_mod -= pice * (int)((unsigned)nsh_mod / (unsigned)pice);
+        }
+      }
+      const unsigned selm = __ballot_sync(FULL, sel);
+      if (sel) {
+        const int slot = (head + qn + __popc(selm & lanemask_lt(lane))) & 63;
+        sh.qj[slot] = core ? js : ~js;
+        sh.qr[0][slot] = rx;
+        sh.qr[1][slot] = ry;
+        sh.qr[2][slot] = rz;
+      }
+      qn += __popc(selm);
+      __syncwarp();
+      if (qn >= 32) {
+        flush(32);
+        __syncwarp();
+      }
+    }
+    __syncwarp();
+  }
+  if (qn > 0) flush(qn);
+  __syncwarp();
+}
+
 template <typename R, int MODE, bool SPECIAL, bool VIRIAL, bool NEAR = false>
 __global__ void __launch_bounds__(kPairWarps * 32, 3)
 k_pair2(const SysDev* __restrict__ S, const int2* __restrict__ work) {
-  using R4 = typename Vec4<R>::T;
   constexpr bool F32 = sizeof(R) == 4 && (MODE == kLJ_RBL || MODE == kCOUL_RBL);
-  __shared__ int s_qj[kPairWarps][64];
-  __shared__ R s_qr[kPairWarps][3][64];
-  __shared__ int s_sa[kPairWarps][64];   // segment first sorted index
-  __shared__ int s_sb[kPairWarps][64];   // segment begin in the flattened sequence
-  __shared__ int s_se[kPairWarps][64];   // segment end in the flattened sequence
-  __shared__ R s_so[kPairWarps][3][64];  // segment coordinate offsets
+  __shared__ LeanShared<R> s_w[kPairWarps];
   __shared__ float s_tab[2 * kMaxF32Types * kMaxF32Types];  // FP32 LJ table: -24 sqrt(eps eps), sigma^6
   __shared__ double s_red[kPairWarps][9];
 
   const int2 wk = work[blockIdx.x];
   const SysDev& s = S[wk.x];
   const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const unsigned FULL = 0xffffffffu;
   const int n = s.n, ntypes = s.ntypes;
   if (F32) {
     for (int t = threadIdx.x; t < ntypes * ntypes && t < kMaxF32Types * kMaxF32Types; t += blockDim.x) {
@@ -712,277 +989,18 @@ k_pair2(const SysDev* __restrict__ S, const int2* __restrict__ work) {
   }
   const int sidx = wk.y + wid;
   PairAcc a;
-#pragma unroll
-  for (int k = 0; k < 3; ++k) a.f[k] = a.g[k] = 0.0;
-#pragma unroll
-  for (int k = 0; k < 6; ++k) a.vir[k] = 0.0;
-  a.rho = a.e0 = a.e1 = 0.0;
-  float ffx = 0.f, ffy = 0.f, ffz = 0.f, fgx = 0.f, fgy = 0.f, fgz = 0.f;
+  float ff[6];
+  acc_zero(ff, a);
   int i = -1;
-
-  if (sidx < n) {
-    const int dx = s.dims[0], dy = s.dims[1], dz = s.dims[2];
-    const double d0 = s.d[0], d1 = s.d[1], d2c = s.d[2];
-    const int4 mi = __ldg(&s.smeta[sidx]);
-    i = mi.x;
-    const int ti = mi.y, moli = mi.z;
-    const double4 xi = ldg4(&s.sx[sidx]);
-    const R4 pi4 = load_sorted<R>(s, sidx);
-    const R pix = pi4.x, piy = pi4.y, piz = pi4.z;
-    // home cell by truncation and NOT clamped (InWhichCell, ExecPointLocator.h:271-274): an atom
-    // that a step left outside the box walks the neighbourhood of its unclamped cell, every
-    // neighbour cell wrapped by a true modulo below
-    const int c0 = (int)((xi.x - s.lo[0]) / d0);
-    const int c1 = (int)((xi.y - s.lo[1]) / d1);
-    const int c2 = (int)((xi.z - s.lo[2]) / d2c);
-    const double fpi = (MODE == kEAM_FORCE) ? s.eam_fp[i] : 0.0;
-    int nsp = 0;
-    const int* spi = nullptr;
-    const double* spw = nullptr;
-    if (SPECIAL) {
-      const int b = s.sp_off[i];
-      nsp = s.sp_off[i + 1] - b;
-      spi = s.sp_ids + b;
-      spw = s.sp_w + b;
-    }
-    const bool rbl = (MODE == kLJ_RBL || MODE == kCOUL_RBL ||
-                      ((MODE == kEAM_RHO || MODE == kEAM_FORCE) && s.neigh == RBMD_NEIGH_RBL));
-    const int pice = rbl ? s.pice : 1;
-    int nsh_mod = 0;  // running shell index modulo pice
-    if (rbl && s.rbl_mode == RBMD_RBL_PHILOX && pice > 1) {
-      uint32_t o[4];
-      philox4x32_10((uint32_t)i, 0u, (uint32_t)s.st->step, kTagRblOffset, s.seed_lo, s.seed_hi, o);
-      nsh_mod = (int)(o[0] % (uint32_t)pice);
-    }
-    uint32_t base_mask = 0;  // bits 0, pice, 2 pice, ... below 32
-    for (int k = 0; k < 32; k += pice) base_mask |= (1u << k);
-    const R rc2 = (R)s.rc2, rs2 = (R)s.rs2;
-    const int nc = s.nc, side = 2 * nc + 1, nrows = side * side;
-    // conservative culling radius: cells farther than rc from i (with a margin for atoms outside
-    // their cell: at least the farthest an atom lay outside its binned cell plus the largest SHAKE
-    // displacement since the cell list was built) cannot hold a core or shell atom; cells of atoms
-    // SHAKE wrapped across the box (they sit on the far side of it) are never culled, and beyond
-    // kMaxMigrated of them nothing is
-    const double margin =
-        fmax(0.1 * fmin(d0, fmin(d1, d2c)), 1.001 * ((double)__uint_as_float(s.st->shake_disp_bits) +
-                                                     (double)__uint_as_float(s.st->out_bits)));
-    const int mig_n = s.st->mig_n;
-    const double cut2 = s.rc2;
-    const double lo0 = s.lo[0], lo1 = s.lo[1], lo2 = s.lo[2];
-    const float spice = (float)pice;
-    const float fsa = (float)sqrt(s.alpha), falpha = (float)s.alpha;
-    const float fLx = (float)s.L[0], fLy = (float)s.L[1], fLz = (float)s.L[2];
-    const float frc2 = (float)s.rc2, frs2 = (float)s.rs2;
-    int head = 0, qn = 0;
-
-    auto flush = [&](int cnt) {
-      if (lane < cnt) {
-        const int slot = (head + lane) & 63;
-        int js = s_qj[wid][slot];
-        const bool core = js >= 0;
-        if (!core) js = ~js;
-        if (F32) {
-          eval_pair_f32<MODE, SPECIAL, NEAR>(s, moli, (float)xi.w, js, core, (float)s_qr[wid][0][slot],
-                                       (float)s_qr[wid][1][slot], (float)s_qr[wid][2][slot], ti, spi, spw, nsp,
-                                       spice, frc2, frs2, fsa, falpha, s_tab, ntypes, fLx, fLy, fLz, ffx, ffy, ffz,
-                                       fgx, fgy, fgz);
-        } else {
-          eval_pair<R, MODE, SPECIAL, VIRIAL, NEAR>(s, i, ti, moli, xi.w, fpi, js, core, s_qr[wid][0][slot],
-                                              s_qr[wid][1][slot], s_qr[wid][2][slot], spi, spw, nsp, (R)pice, a);
-        }
-      }
-      head = (head + cnt) & 63;
-      qn -= cnt;
-    };
-
-    // rows per segment table: 32 of at most two ranges each, or 21 of at most three when the box
-    // holds fewer than 2 nc + 1 cells in z (the table holds 64)
-    const int group = dz >= side ? 32 : 21;
-    for (int r0 = 0; r0 < nrows; r0 += group) {
-      // ---- segment table of rows r0 .. r0 + group - 1 (one row per lane)
-      const int r = r0 + lane;
-      int nseg = 0, cnt = 0;
-      int sa0 = 0, sa1 = 0, sa2 = 0, n0c = 0, n1c = 0, n2c = 0;
-      R oxv = R(0), oyv = R(0), oz0 = R(0), oz1 = R(0), oz2 = R(0);
-      if (lane < group && r < nrows) {
-        const int da = r / side - nc, db = r % side - nc;
-        int n0 = c0 + da, n1 = c1 + db;
-        int w0 = ((n0 % dx) + dx) % dx;
-        int w1 = ((n1 % dy) + dy) % dy;
-        const double ox = d0 * (double)(w0 - n0), oy = d1 * (double)(w1 - n1);
-        oxv = (R)ox;
-        oyv = (R)oy;
-        // squared gap between i and the column of cells (unwrapped frame), shrunk by the margin
-        const double bx0 = lo0 + n0 * d0 - margin, bx1 = lo0 + (n0 + 1) * d0 + margin;
-        const double by0 = lo1 + n1 * d1 - margin, by1 = lo1 + (n1 + 1) * d1 + margin;
-        const double gx = fmax(0.0, fmax(bx0 - xi.x, xi.x - bx1));
-        const double gy = fmax(0.0, fmax(by0 - xi.y, xi.y - by1));
-        const double gxy = gx * gx + gy * gy;
-        int elo = nc + 1, ehi = -nc - 1;
-        if (gxy < cut2) {
-          for (int de = -nc; de <= nc; ++de) {
-            const int n2 = c2 + de;
-            const double bz0 = lo2 + n2 * d2c - margin, bz1 = lo2 + (n2 + 1) * d2c + margin;
-            const double gz = fmax(0.0, fmax(bz0 - xi.z, xi.z - bz1));
-            if (gxy + gz * gz < cut2) {
-              elo = min(elo, de);
-              ehi = max(ehi, de);
-            }
-          }
-        }
-        if (mig_n > kMaxMigrated) {
-          elo = -nc;
-          ehi = nc;
-        } else {
-          for (int m = 0; m < mig_n; ++m) {
-            const int cm = __ldg(&s.st->mig_cell[m]) - dz * (w1 + dy * w0);
-            if (cm < 0 || cm >= dz) continue;  // not in this row's column
-            for (int de = -nc; de <= nc; ++de)
-              if ((((c2 + de) % dz) + dz) % dz == cm) {
-                elo = min(elo, de);
-                ehi = max(ehi, de);
-              }
-          }
-        }
-        {
-          if (elo <= ehi) {
-            // unwrapped z cells [z0, z1] (len <= 2 nc + 1 <= 2 dz - 1 of them) start in the
-            // periodic copy q = floor(z0 / dz); they map to wrapped cells [zw, zw + len) when that
-            // stays below dz, else to [zw, dz), then [0, rest) of the next copy, or [0, dz) and
-            // [0, rest - dz) of the two next when the stencil is longer than the box.  The shift of
-            // a cell is d * (wrapped - unwrapped) = -d dz q, -d dz (q + 1), -d dz (q + 2).
-            const int base = dz * (w1 + dy * w0);
-            const int z0 = c2 + elo, len = ehi - elo + 1;
-            const int zw = ((z0 % dz) + dz) % dz;
-            const int q = (z0 - zw) / dz;
-            sa0 = __ldg(&s.cell_start[base + zw]);
-            oz0 = (R)(-d2c * (double)dz * (double)q);
-            if (zw + len <= dz) {
-              n0c = __ldg(&s.cell_start[base + zw + len]) - sa0;
-              nseg = 1;
-            } else {
-              n0c = __ldg(&s.cell_start[base + dz]) - sa0;
-              const int rest = zw + len - dz;
-              sa1 = __ldg(&s.cell_start[base]);
-              oz1 = (R)(-d2c * (double)dz * (double)(q + 1));
-              if (rest <= dz) {
-                n1c = __ldg(&s.cell_start[base + rest]) - sa1;
-                nseg = 2;
-              } else {
-                n1c = __ldg(&s.cell_start[base + dz]) - sa1;
-                sa2 = sa1;
-                n2c = __ldg(&s.cell_start[base + rest - dz]) - sa2;
-                oz2 = (R)(-d2c * (double)dz * (double)(q + 2));
-                nseg = 3;
-              }
-            }
-            cnt = n0c + n1c + n2c;
-          }
-        }
-      }
-      const int seg_incl = warp_incl_scan(nseg, lane);
-      const int cnt_incl = warp_incl_scan(cnt, lane);
-      const int nsegs = __shfl_sync(FULL, seg_incl, 31);
-      const int total = __shfl_sync(FULL, cnt_incl, 31);
-      {
-        int slot = seg_incl - nseg, beg = cnt_incl - cnt;
-        if (nseg >= 1) {
-          s_sa[wid][slot] = sa0;
-          s_sb[wid][slot] = beg;
-          s_se[wid][slot] = beg + n0c;
-          s_so[wid][0][slot] = oxv;
-          s_so[wid][1][slot] = oyv;
-          s_so[wid][2][slot] = oz0;
-        }
-        if (nseg >= 2) {
-          s_sa[wid][slot + 1] = sa1;
-          s_sb[wid][slot + 1] = beg + n0c;
-          s_se[wid][slot + 1] = beg + n0c + n1c;
-          s_so[wid][0][slot + 1] = oxv;
-          s_so[wid][1][slot + 1] = oyv;
-          s_so[wid][2][slot + 1] = oz1;
-        }
-        if (nseg == 3) {
-          s_sa[wid][slot + 2] = sa2;
-          s_sb[wid][slot + 2] = beg + n0c + n1c;
-          s_se[wid][slot + 2] = beg + n0c + n1c + n2c;
-          s_so[wid][0][slot + 2] = oxv;
-          s_so[wid][1][slot + 2] = oyv;
-          s_so[wid][2][slot + 2] = oz2;
-        }
-      }
-      __syncwarp();
-      // ---- candidates of the flattened sequence, 32 per iteration
-      int seg = 0;
-      for (int base = 0; base < total; base += 32) {
-        const int p = base + lane;
-        const bool valid = p < total;
-        bool core = false, shell = false;
-        R rx = R(0), ry = R(0), rz = R(0);
-        int js = 0;
-        if (valid) {
-          while (p >= s_se[wid][seg]) ++seg;
-          js = s_sa[wid][seg] + (p - s_sb[wid][seg]);
-          const R4 pj = load_sorted<R>(s, js);
-          rx = (pj.x - s_so[wid][0][seg]) - pix;
-          ry = (pj.y - s_so[wid][1][seg]) - piy;
-          rz = (pj.z - s_so[wid][2][seg]) - piz;
-          const R dd = add_rn(add_rn(mul_rn(rx, rx), mul_rn(ry, ry)), mul_rn(rz, rz));
-          if (rbl) {
-            shell = (rc2 - dd > R(0.0001) && dd - rs2 > R(0.0001));
-            core = !shell && (rs2 - dd > R(0.0001) && dd > R(0.0001));
-          } else {
-            core = (rc2 - dd > R(0.0001) && dd > R(0.0001));
-          }
-          if constexpr (sizeof(R) == 4) {
-            if (f32_banded(s, (float)dd))
-              classify_fp64(s, xi.x, xi.y, xi.z, js, (int)rintf((float)(s_so[wid][0][seg] / d0)),
-                            (int)rintf((float)(s_so[wid][1][seg] / d1)), (int)rintf((float)(s_so[wid][2][seg] / d2c)),
-                            rbl, core, shell);
-          }
-        }
-        bool sel = core;
-        if (rbl) {
-          if (pice == 1) {
-            sel = core || shell;
-          } else {
-            const unsigned sm = __ballot_sync(FULL, shell);
-            const int phase = nsh_mod == 0 ? 0 : pice - nsh_mod;
-            const uint32_t mask = phase < 32 ? (base_mask << phase) : 0u;
-            const int pre = __popc(sm & lanemask_lt(lane));
-            sel = core || (shell && ((mask >> pre) & 1u));
-            nsh_mod += __popc(sm);
-            nsh_mod -= pice * (int)((unsigned)nsh_mod / (unsigned)pice);
-          }
-        }
-        const unsigned selm = __ballot_sync(FULL, sel);
-        if (sel) {
-          const int slot = (head + qn + __popc(selm & lanemask_lt(lane))) & 63;
-          s_qj[wid][slot] = core ? js : ~js;
-          s_qr[wid][0][slot] = rx;
-          s_qr[wid][1][slot] = ry;
-          s_qr[wid][2][slot] = rz;
-        }
-        qn += __popc(selm);
-        __syncwarp();
-        if (qn >= 32) {
-          flush(32);
-          __syncwarp();
-        }
-      }
-      __syncwarp();
-    }
-    if (qn > 0) flush(qn);
-    __syncwarp();
-  }
+  if (sidx < n) lean_atom<R, MODE, SPECIAL, VIRIAL, NEAR>(s, sidx, lane, s_w[wid], s_tab, i, ff, a);
 
   double r9[9];
   if (F32) {
-    r9[0] = warp_sum((double)ffx);
-    r9[1] = warp_sum((double)ffy);
-    r9[2] = warp_sum((double)ffz);
+    r9[0] = warp_sum((double)ff[0]);
+    r9[1] = warp_sum((double)ff[1]);
+    r9[2] = warp_sum((double)ff[2]);
     if (MODE == kCOUL_RBL) {
-      const double q0 = warp_sum((double)fgx), q1 = warp_sum((double)fgy), q2 = warp_sum((double)fgz);
+      const double q0 = warp_sum((double)ff[3]), q1 = warp_sum((double)ff[4]), q2 = warp_sum((double)ff[5]);
       r9[0] = r9[0] + s.qqr2e * q0;
       r9[1] = r9[1] + s.qqr2e * q1;
       r9[2] = r9[2] + s.qqr2e * q2;
@@ -1276,16 +1294,6 @@ __device__ inline void acc_to_r9(const SysDev& s, const double (&c)[6], const Pa
     r9[0] = a.e0;
     r9[1] = a.e1;
   }
-}
-
-__device__ inline void acc_zero(float (&ff)[6], PairAcc& a) {
-#pragma unroll
-  for (int k = 0; k < 6; ++k) ff[k] = 0.f;
-#pragma unroll
-  for (int k = 0; k < 3; ++k) a.f[k] = a.g[k] = 0.0;
-#pragma unroll
-  for (int k = 0; k < 6; ++k) a.vir[k] = 0.0;
-  a.rho = a.e0 = a.e1 = 0.0;
 }
 
 // Adds the accumulators of lanes (a, m), m = 0 .. k - 1 (lane = a + m nat), into lane (a, 0), in a
@@ -1984,61 +1992,41 @@ __device__ inline int col_first_skip(const SysDev& s, int i, int pice) {
   return nm == 0 ? 0 : pice - nm;
 }
 
-// The stray atoms of the batch's columns, before the column kernel: each is walked by the whole
-// warp over its own neighbourhood and its force written (finish_atom), where the column kernel
-// reads it back.  Warps take columns from a work counter (ctr[0]; ctr[1] counts finished warps, and
-// the last one resets both), as the column kernel does.
-// resident blocks per SM the stray pass is compiled for: its walks wait on dependent loads, so it
-// runs more warps per SM than the column kernel, at the price of a few spilled registers (on the
-// saline stream 25.79 ms for both pair launches of a step, against 25.83 ms at the column kernel's
-// 4 blocks and 25.76 ms at 8)
-#ifndef RBMD_STRAY_MIN_BLOCKS
-#define RBMD_STRAY_MIN_BLOCKS 6
-#endif
-
+// The stray atoms, before the column kernel: a block looks 256 atoms over (in cell order), lists its
+// strays, and its warps walk them, one each, by the lean traversal (rows as contiguous ranges, cells
+// beyond rc left out), writing their forces where the column kernel reads them back for the RBL mean.
+// Bound by the latency of a walk's dependent loads, so what counts is that no warp has several strays
+// to walk while others have none and that a walk is short: a warp per column of cells, cell after
+// cell over all (2 nc + 1)^3 of them, took 167 us per step of a 9000-atom water box and 324 us of a
+// 64,000-atom one.
 template <int MODE, bool SPECIAL, bool NEAR>
-__global__ void __launch_bounds__(kColWarps * 32, RBMD_STRAY_MIN_BLOCKS)
-k_pair_col_strays(const SysDev* __restrict__ S, const int2* __restrict__ work, int nwork, unsigned* __restrict__ ctr) {
-  const int lane = threadIdx.x & 31;
-  const unsigned FULL = 0xffffffffu;
-  for (;;) {
-    int wi = 0;
-    if (lane == 0) wi = (int)atomicAdd(&ctr[0], 1u);
-    wi = __shfl_sync(FULL, wi, 0);
-    if (wi >= nwork) break;
-    const int2 wk = __ldg(&work[wi]);
-    const SysDev& s = S[wk.x];
+__global__ void __launch_bounds__(kAtomBlock, 3) k_pair_col_strays(const SysDev* __restrict__ S,
+                                                                   const int2* __restrict__ work) {
+  __shared__ LeanShared<float> s_w[kAtomBlock / 32];
+  __shared__ int s_list[kAtomBlock], s_n;
+  const int2 wk = work[blockIdx.x];
+  const SysDev& s = S[wk.x];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  if (threadIdx.x == 0) s_n = 0;
+  __syncthreads();
+  const int k = wk.y + threadIdx.x;
+  if (k < s.n) {
+    const int c = __ldg(&s.cell_of_atom[__ldg(&s.smeta[k]).x]);
     const int dy = s.dims[1], dz = s.dims[2];
-    const int hx = wk.y / dy, hy = wk.y % dy;
-    const int cbase = dz * (hy + dy * hx);
-    const int a0 = __ldg(&s.cell_start[cbase]), a1 = __ldg(&s.cell_start[cbase + dz]);
-    for (int g0 = a0; g0 < a1; g0 += 32) {
-      const int si = g0 + lane;
-      int i = 0, c = 0;
-      bool stray = false;
-      if (si < a1) {
-        i = __ldg(&s.smeta[si]).x;
-        stray = col_is_stray(s, si, hx, hy, __ldg(&s.cell_of_atom[i]) - cbase);
-        if (stray) c = col_first_skip(s, i, s.pice);
-      }
-      for (unsigned m = __ballot_sync(FULL, stray); m; m &= m - 1) {
-        const int as = __ffs(m) - 1;
-        const int sk = __shfl_sync(FULL, c, as);
-        float ff[6];
-        PairAcc acc;
-        acc_zero(ff, acc);
-        tile_stray<float, MODE, SPECIAL, false, NEAR>(s, g0 + as, sk, s.pice, true, (const float*)s.ljf, 0, nullptr,
-                                                      nullptr, nullptr, nullptr, ff, acc);
-        double cmb[6], r9[9];
-        acc_warp_total<true>(ff, acc, cmb);
-        acc_to_r9<MODE, true, false>(s, cmb, acc, r9);
-        if (lane == as) finish_atom<MODE>(s, i, r9);
-      }
-    }
+    if (col_is_stray(s, k, c / (dz * dy), (c / dz) % dy, c % dz)) s_list[atomicAdd(&s_n, 1)] = k;
   }
-  if (lane == 0 && atomicAdd(&ctr[1], 1u) == gridDim.x * (unsigned)kColWarps - 1u) {
-    ctr[0] = 0u;
-    ctr[1] = 0u;
+  __syncthreads();
+  for (int q = wid; q < s_n; q += kAtomBlock / 32) {
+    float ff[6];
+    PairAcc acc;
+    acc_zero(ff, acc);
+    int i;
+    lean_atom<float, MODE, SPECIAL, false, NEAR>(s, s_list[q], lane, s_w[wid], (const float*)s.ljf, i, ff, acc);
+    double cmb[6], r9[9];
+    acc_warp_total<true>(ff, acc, cmb);
+    acc_to_r9<MODE, true, false>(s, cmb, acc, r9);
+    if (lane == 0) finish_atom<MODE>(s, i, r9);
+    __syncwarp();
   }
 }
 
@@ -2458,8 +2446,7 @@ static void go_near(const Batch& b, cudaStream_t st) {
   if constexpr (kColumn) {
     if (b.dense == 2) {
       if (b.pair.n > 0) {
-        k_pair_col_strays<MODE, SPECIAL, NEAR><<<b.stray_grid, kColWarps * 32, 0, st>>>(b.sys, b.pair.d, b.pair.n,
-                                                                                        b.col_ctr + 2);
+        k_pair_col_strays<MODE, SPECIAL, NEAR><<<b.atom.n, kAtomBlock, 0, st>>>(b.sys, b.atom.d);
         note_launch();
         k_pair_col<MODE, SPECIAL, NEAR><<<b.col_grid, kColWarps * 32, 0, st>>>(b.sys, b.pair.d, b.pair.n, b.col_ctr,
                                                                                band);
@@ -2490,23 +2477,15 @@ static void go(const Batch& b, cudaStream_t st) {
   go_near<R, MODE, SPECIAL, VIRIAL, false>(b, st);
 }
 
-int pair_col_grid(int ncols, int ff, int special, int near, bool strays) {
+int pair_col_grid(int ncols, int ff, int special, int near) {
   int dev = 0, sms = 0, per_sm = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const void* fn;
-  if (strays)
-    fn = ff == RBMD_FF_LJ_CUT ? (const void*)k_pair_col_strays<kLJ_RBL, false, false>
-         : special ? (near ? (const void*)k_pair_col_strays<kCOUL_RBL, true, true>
-                           : (const void*)k_pair_col_strays<kCOUL_RBL, true, false>)
-                   : (near ? (const void*)k_pair_col_strays<kCOUL_RBL, false, true>
-                           : (const void*)k_pair_col_strays<kCOUL_RBL, false, false>);
-  else
-    fn = ff == RBMD_FF_LJ_CUT ? (const void*)k_pair_col<kLJ_RBL, false, false>
-         : special ? (near ? (const void*)k_pair_col<kCOUL_RBL, true, true>
-                           : (const void*)k_pair_col<kCOUL_RBL, true, false>)
-                   : (near ? (const void*)k_pair_col<kCOUL_RBL, false, true>
-                           : (const void*)k_pair_col<kCOUL_RBL, false, false>);
+  const void* fn = ff == RBMD_FF_LJ_CUT ? (const void*)k_pair_col<kLJ_RBL, false, false>
+                   : special ? (near ? (const void*)k_pair_col<kCOUL_RBL, true, true>
+                                     : (const void*)k_pair_col<kCOUL_RBL, true, false>)
+                             : (near ? (const void*)k_pair_col<kCOUL_RBL, false, true>
+                                     : (const void*)k_pair_col<kCOUL_RBL, false, false>);
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kColWarps * 32, 0);
   const int need = (ncols + kColWarps - 1) / kColWarps;
   return std::max(1, std::min(need, std::max(1, sms) * std::max(1, per_sm)));
