@@ -772,9 +772,12 @@ int Context::add_system(const rbmd_system_desc& d, const rbmd_params& p, int32_t
     up(D.z2r_s, d.eam_z2r_spline, sizeof(double) * nz);
   }
   D.atom_part = (double*)dal(sizeof(double) * 8 * D.blocks_atom);
-  // pair-kernel partials: enough blocks for any layout the autotuner may switch to
-  D.vir_part = (double*)dal(sizeof(double) * 9 *
-                            std::max((D.ncell_cap + kCellWarpsHost - 1) / kCellWarpsHost, (n + kPairWarps - 1) / kPairWarps));
+  // pair-kernel partials: enough for any layout the autotuner may switch to (nine per block; the column
+  // kernel three per 32-atom chunk, at most n / 32 + one per column of them)
+  const size_t part_blocks =
+      std::max((D.ncell_cap + kCellWarpsHost - 1) / kCellWarpsHost, (n + kPairWarps - 1) / kPairWarps);
+  const size_t part_chunks = (size_t)n / 32 + (size_t)D.dims[0] * D.dims[1] + 1;
+  D.vir_part = (double*)dal(sizeof(double) * std::max(9 * part_blocks, 3 * part_chunks));
   D.tri_part = (double*)dal(sizeof(double) * 6 * std::max(1, D.blocks_tri));
   D.st = (SysState*)dal(sizeof(SysState));
   if (oom) {
@@ -971,7 +974,13 @@ Context::BatchRec* Context::build_batch(const std::vector<System*>& group, int& 
       br->allocs.push_back(b.col_ctr);
       cudaMemsetAsync(b.col_ctr, 0, 2 * sizeof(unsigned), stream);
     }
-    b.col_grid = pair_col_grid(b.pair.n, b.ff, b.special, b.near);
+    double chunks = 0.0, longest = 0.0;
+    for (System* s : group) {
+      const double nxy = (double)s->dev.dims[0] * s->dev.dims[1], per = s->dev.n / nxy;
+      chunks += nxy * (per / 32.0 + 0.5);
+      longest = std::max(longest, per);
+    }
+    plan_pair_col(b, chunks, longest, g.nc);
   }
   mk(wc, b.cell);
   mk(wr, b.rho);

@@ -22,6 +22,7 @@
 // threshold equivalents of the reference's window tests) so that it makes the same decisions as
 // the CPU oracle on the same positions.
 #include <algorithm>
+#include <cmath>
 #include <mutex>
 
 #include "kernels.h"
@@ -1952,10 +1953,13 @@ k_pair_tile(const SysDev* __restrict__ S, const int2* __restrict__ work, int cap
 // a time from a work counter, longest columns first, so no warp waits for another and the launch's
 // tail is short columns.  The RBL mean force is summed per column and the system's last column
 // adds the partials in column order: the result does not depend on which warp took which column.
-constexpr int kColWarps = 4;     // warps per block
+constexpr int kColWarps = 4;     // warps per block, a chunk each
+constexpr int kColSplit = 8;     // warps per block of the split form, one chunk between them
 constexpr int kColStage = 256;   // staged candidates per warp
 constexpr int kColQ = kColStage;  // the most steps between evaluations: a staged tile
 constexpr int kColQW = kColQ / 32;  // 32-step blocks between evaluations
+constexpr int kColKeep = 12;     // 32-step blocks whose masks a warp of the split form keeps
+constexpr int kColMaxRows = 64;  // traversal rows the split form takes
 constexpr float kColFar = 1e30f;
 // resident blocks per SM: 4 (128 registers per thread) ran the saline stream's column launch in
 // 34.2 ms against 36.1 ms at 5 (96 registers, twice the local-memory traffic of spills)
@@ -2030,46 +2034,74 @@ __global__ void __launch_bounds__(kAtomBlock, 3) k_pair_col_strays(const SysDev*
   }
 }
 
-template <int MODE, bool SPECIAL, bool NEAR>
-__global__ void __launch_bounds__(kColWarps * 32, RBMD_COL_MIN_BLOCKS)
-k_pair_col(const SysDev* __restrict__ S, const int2* __restrict__ work, int nwork, unsigned* __restrict__ ctr,
-           float4 band) {
+// A warp's shared memory.
+template <bool SPLIT>
+struct ColWarp {
+  float4 c[kColStage];  // candidate position - image shift, charge
+  int id[kColStage];    // atom id (LJ/CUT: molecule) | type << kJsBits
+  // per lane and 32-step block, bit t for step t: the selected candidates (core, or a picked shell) and
+  // the picked shells among them, of the tile being evaluated; in the split form also, behind them, the
+  // core and shell masks kept from the first pass
+  unsigned sel[kColQW + (SPLIT ? kColKeep : 0)][32];
+  unsigned pk[kColQW + (SPLIT ? kColKeep : 0)][32];
+  // per lane (home atom): what the evaluation needs, kept out of registers during the walk
+  int4 ai[32];     // type, molecule, special partners, first special slot
+  int2 sp[32];     // first two special partners
+  float2 sw[32];   // and their weights
+  float4 f[32];    // force of the row so far (x, y, z), charge in w
+  float3 ft[32];   // force of the rows before it
+  float shift[3][3];  // per dimension: d (w - n) for w - n = -dims, 0, +dims
+};
+// The split form's, per block: each row's shells per lane, and its force.
+struct ColRow {
+  int shells[32];
+  float3 f[32];
+};
+constexpr size_t col_smem(int nrows) { return kColSplit * sizeof(ColWarp<true>) + (size_t)nrows * sizeof(ColRow); }
+
+template <int MODE, bool SPECIAL, bool NEAR, bool SPLIT>
+__global__ void __launch_bounds__(SPLIT ? kColSplit * 32 : kColWarps * 32, SPLIT ? 2 : RBMD_COL_MIN_BLOCKS)
+k_pair_col(const SysDev* __restrict__ S, const int2* __restrict__ work, int nwork, int nparts,
+           unsigned* __restrict__ ctr, float4 band) {
   static_assert(MODE == kLJ_RBL || MODE == kCOUL_RBL, "column layout: FP32 RBL forces only");
   static_assert(!NEAR || MODE == kCOUL_RBL, "the near-Coulomb table applies to the Coulomb mode");
   static_assert(kColQ % 32 == 0 && kColStage % 32 == 0, "the walk runs in blocks of 32 steps");
-  __shared__ float4 s_c[kColWarps][kColStage];      // candidate position - image shift, charge
-  __shared__ int s_id[kColWarps][kColStage];        // atom id (LJ/CUT: molecule) | type << kJsBits
-  // per lane and 32-step block since the last evaluation, bit t for step t: the selected candidates
-  // (core, or a picked shell) and the picked shells among them
-  __shared__ unsigned s_sel[kColWarps][kColQW][32];
-  __shared__ unsigned s_pk[kColWarps][kColQW][32];
-  // per lane (home atom): what the evaluation needs, kept out of registers during the walk
-  __shared__ int4 s_ai[kColWarps][32];    // type, molecule, special partners, first special slot
-  __shared__ int2 s_sp[kColWarps][32];    // first two special partners
-  __shared__ float2 s_sw[kColWarps][32];  // and their weights
-  __shared__ float4 s_f[kColWarps][32];   // force accumulated so far (x, y, z), charge in w
-  __shared__ float s_shift[kColWarps][3][3];  // per dimension: d (w - n) for w - n = -dims, 0, +dims
-
+  constexpr int kWarps = SPLIT ? kColSplit : kColWarps;
   const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  __shared__ __align__(16) unsigned char s_fixed[SPLIT ? 16 : kColWarps * sizeof(ColWarp<false>)];
+  __shared__ int s_item;
+  extern __shared__ __align__(16) unsigned char s_dyn[];  // split form: kColSplit warps, then the rows
+  ColWarp<SPLIT>& sh = reinterpret_cast<ColWarp<SPLIT>*>(SPLIT ? s_dyn : s_fixed)[wid];
+  ColRow* const s_row = reinterpret_cast<ColRow*>(s_dyn + kColSplit * sizeof(ColWarp<true>));
+
   const unsigned FULL = 0xffffffffu;
   // FP32 band edges of the launch (the union of its systems' bands; a batch shares rc and rs)
   const float b0 = band.x, b1 = band.y, b2 = band.z, b3 = band.w;
-  int cur = -1;  // slot of the system whose image shifts s_shift holds
+  int cur = -1;  // slot of the system whose image shifts sh.shift holds
   for (;;) {
     int wi = 0;
-    if (lane == 0) wi = (int)atomicAdd(&ctr[0], 1u);
-    wi = __shfl_sync(FULL, wi, 0);
-    if (wi >= nwork) break;
-    const int2 wk = __ldg(&work[wi]);
+    if constexpr (SPLIT) {
+      __syncthreads();  // the item before is read, its rows are used
+      if (threadIdx.x == 0) s_item = (int)atomicAdd(&ctr[0], 1u);
+      __syncthreads();
+      wi = s_item;
+    } else {
+      if (lane == 0) wi = (int)atomicAdd(&ctr[0], 1u);
+      wi = __shfl_sync(FULL, wi, 0);
+    }
+    if (wi >= nwork * nparts) break;
+    // item: every nparts-th chunk of a column, from chunk `part` on
+    const int part = wi % nparts;
+    const int2 wk = __ldg(&work[wi / nparts]);
     const SysDev& s = S[wk.x];
     const int dx = s.dims[0], dy = s.dims[1], dz = s.dims[2];
     const int ntypes = s.ntypes;
     if (wk.x != cur) {
       cur = wk.x;
-      __syncwarp();  // the previous column's reads are done
+      __syncwarp();  // the previous item's reads are done
       if (lane < 9) {
         const int dim = lane / 3, t = lane % 3;
-        s_shift[wid][dim][t] = (float)(s.d[dim] * (double)((t - 1) * s.dims[dim]));
+        sh.shift[dim][t] = (float)(s.d[dim] * (double)((t - 1) * s.dims[dim]));
       }
       __syncwarp();
     }
@@ -2085,16 +2117,16 @@ k_pair_col(const SysDev* __restrict__ S, const int2* __restrict__ work, int nwor
     const float mdisp = __uint_as_float(s.st->shake_disp_bits) + __uint_as_float(s.st->out_bits);
     const int mig_n = s.st->mig_n;
     const float mgx = 1e-3f * fdx + mdisp, mgy = 1e-3f * fdy + mdisp, mgz = 1e-3f * fdz + mdisp;
-    double red0 = 0.0, red1 = 0.0, red2 = 0.0;  // this lane's atoms' forces (the RBL mean)
 
     const int col = wk.y;
     {
       const int hx = col / dy, hy = col % dy;
       const int cbase = dz * (hy + dy * hx);
       const int a0 = __ldg(&s.cell_start[cbase]), a1 = __ldg(&s.cell_start[cbase + dz]);
-      for (int g0 = a0; g0 < a1; g0 += 32) {
+      for (int g0 = a0 + 32 * part; g0 < a1; g0 += 32 * nparts) {
         const int si = g0 + lane;
         const bool valid = si < a1;
+        double red0 = 0.0, red1 = 0.0, red2 = 0.0;  // this lane's atom's force (the RBL mean)
         int i = 0, zl = 0;
         float4 p4 = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         bool stray = false;
@@ -2121,16 +2153,25 @@ k_pair_col(const SysDev* __restrict__ S, const int2* __restrict__ work, int nwor
               w1 = (float)__ldg(&s.sp_w[spb + 1]);
             }
           }
-          s_ai[wid][lane] = make_int4(mi.y, mi.z, nsp, spb);
-          s_sp[wid][lane] = make_int2(sp0, sp1);
-          s_sw[wid][lane] = make_float2(w0, w1);
+          sh.ai[lane] = make_int4(mi.y, mi.z, nsp, spb);
+          sh.sp[lane] = make_int2(sp0, sp1);
+          sh.sw[lane] = make_float2(w0, w1);
         } else {  // a lane without an atom still runs the evaluation rounds (adding nothing): its
                   // record must hold valid indices (type 0, no special partners)
-          s_ai[wid][lane] = make_int4(0, -1, 0, 0);
-          s_sp[wid][lane] = make_int2(-1, -1);
-          s_sw[wid][lane] = make_float2(1.0f, 1.0f);
+          sh.ai[lane] = make_int4(0, -1, 0, 0);
+          sh.sp[lane] = make_int2(-1, -1);
+          sh.sw[lane] = make_float2(1.0f, 1.0f);
         }
-        s_f[wid][lane] = make_float4(0.0f, 0.0f, 0.0f, p4.w);
+        sh.f[lane] = make_float4(0.0f, 0.0f, 0.0f, p4.w);
+        sh.ft[lane] = make_float3(0.0f, 0.0f, 0.0f);
+        if constexpr (SPLIT) {
+          __syncthreads();  // the chunk before has read the rows
+          for (int t = threadIdx.x; t < nrows * 32; t += kWarps * 32) {
+            s_row[t >> 5].shells[lane] = 0;
+            s_row[t >> 5].f[lane] = make_float3(0.0f, 0.0f, 0.0f);
+          }
+          __syncthreads();
+        }
 
         // ---- an atom outside its cell: walked by k_pair_col_strays before this launch, which wrote
         // its force
@@ -2150,34 +2191,34 @@ k_pair_col(const SysDev* __restrict__ S, const int2* __restrict__ work, int nwor
         // stage entry `base` (the candidates are still in the stage)
         auto flush = [&](int nblk, int base) {
           int qn = 0;
-          for (int bk = 0; bk < nblk; ++bk) qn += __popc(s_sel[wid][bk][lane]);
+          for (int bk = 0; bk < nblk; ++bk) qn += __popc(sh.sel[bk][lane]);
           const int rounds = __reduce_max_sync(FULL, qn);
           if (rounds == 0) return;
-          const int4 ai = s_ai[wid][lane];
-          const int2 sp = s_sp[wid][lane];
-          const float2 sw = s_sw[wid][lane];
-          float4 fa = s_f[wid][lane];
+          const int4 ai = sh.ai[lane];
+          const int2 sp = sh.sp[lane];
+          const float2 sw = sh.sw[lane];
+          float4 fa = sh.f[lane];
           const float spice = (float)pice, fsa = s.fsa, falpha_l2 = s.falpha_l2, fqq = s.fqq;
           const float* const ntab = s.near_tab;  // RBMD_NEAR_TABLE: the reference's G table
           int wc = 0;  // block of the next selected candidate, its remaining bits and its picks
-          unsigned mc = s_sel[wid][0][lane], pc = s_pk[wid][0][lane];
+          unsigned mc = sh.sel[0][lane], pc = sh.pk[0][lane];
           // two rounds per iteration: independent pairs for the scheduler to interleave
 #pragma unroll 2
           for (int k = 0; k < rounds; ++k) {
             if (k < qn) {
               while (mc == 0u) {
                 ++wc;
-                mc = s_sel[wid][wc][lane];
-                pc = s_pk[wid][wc][lane];
+                mc = sh.sel[wc][lane];
+                pc = sh.pk[wc][lane];
               }
               const int b = __ffs(mc) - 1;
               mc &= mc - 1u;
               const int e = base + 32 * wc + b;
               const bool core = ((pc >> b) & 1u) == 0u;
-              const float4 pj = s_c[wid][e];
+              const float4 pj = sh.c[e];
               const float rx = pj.x - pix, ry = pj.y - piy, rz = pj.z - piz;
               const float d2 = tile_d2(rx, ry, rz);
-              const int idt = s_id[wid][e];
+              const int idt = sh.id[e];
               const int idj = idt & kJsMask, tj = idt >> kJsBits;
               float w = 1.0f;
               if (SPECIAL) {
@@ -2201,190 +2242,243 @@ k_pair_col(const SysDev* __restrict__ S, const int2* __restrict__ work, int nwor
               fa.z += f * rz;
             }
           }
-          s_f[wid][lane] = fa;
+          sh.f[lane] = fa;
         };
 
         if (zmax >= 0) {
           const float xr = pix - (float)s.lo[0], yr = piy - (float)s.lo[1], zr = piz - (float)s.lo[2];
           const int u0 = zmin - nc, u1 = zmax + nc;  // the chunk's z cells, unwrapped, -dz < u0, u1 < 2 dz
-          for (int r = 0; r < nrows; ++r) {
-            const int da = r / side - nc, db = r % side - nc;
-            const int n0 = hx + da, n1 = hy + db;  // unwrapped column of the row (nc < dims)
-            const int w0c = n0 < 0 ? n0 + dx : (n0 >= dx ? n0 - dx : n0);
-            const int w1c = n1 < 0 ? n1 + dy : (n1 >= dy ? n1 - dy : n1);
-            const int t0c = n0 < 0 ? 2 : (n0 >= dx ? 0 : 1), t1c = n1 < 0 ? 2 : (n1 >= dy ? 0 : 1);
-            const int base = dz * (w1c + dy * w0c);
-            // the row's union: unwrapped z cells u0 .. u1 in up to three segments (images -1, 0, +1:
-            // below the box, inside, above), segment k holding sorted indices sa_k .., union entries ob_k ..
-            int sa0 = 0, sa1, sa2 = 0, ob1, ob2, len = 0;
-            if (u0 < 0) {  // below the box: cells u0 + dz .. dz - 1
-              sa0 = __ldg(&s.cell_start[base + u0 + dz]);
-              len = __ldg(&s.cell_start[base + dz]) - sa0;
-            }
-            ob1 = len;
-            {  // inside: cells max(u0, 0) .. min(u1, dz - 1)
-              sa1 = __ldg(&s.cell_start[base + max(u0, 0)]);
-              len += __ldg(&s.cell_start[base + min(u1, dz - 1) + 1]) - sa1;
-            }
-            ob2 = len;
-            if (u1 >= dz) {  // above the box: cells 0 .. u1 - dz
-              sa2 = __ldg(&s.cell_start[base]);
-              len += __ldg(&s.cell_start[base + u1 - dz + 1]) - sa2;
-            }
-            // union entries before unwrapped cell u (u0 <= u <= u1 + 1)
-            auto ucount = [&](int u) -> int {
-              if (u > u1) return len;
-              if (u < 0) return __ldg(&s.cell_start[base + u + dz]) - sa0;
-              if (u < dz) return ob1 + __ldg(&s.cell_start[base + u]) - sa1;
-              return ob2 + __ldg(&s.cell_start[base + u - dz]) - sa2;
-            };
-            // this lane's window, trimmed to the z cells that can hold an atom within rc: the x / y
-            // gaps to the row's column (shrunk by the margin) leave a z half-width sqrt(rc^2 - g^2)
-            // (grown by it)
-            int wb = 0, wl = 0;
-            if (act) {
-              int zlo = zl + nc + 1, zhi = zl - nc - 1;  // empty
-              const float gx = fmaxf(0.0f, fmaxf((float)n0 * fdx - xr, xr - (float)(n0 + 1) * fdx) - mgx);
-              const float gy = fmaxf(0.0f, fmaxf((float)n1 * fdy - yr, yr - (float)(n1 + 1) * fdy) - mgy);
-              const float g2 = __fmaf_rn(gx, gx, gy * gy);
-              if (g2 < frc2) {
-                const float h = sqrtf(frc2 - g2) + mgz;
-                zlo = max((int)floorf((zr - h) / fdz), zl - nc);
-                zhi = min((int)floorf((zr + h) / fdz), zl + nc);
+          // split form: the warps take the rows in turn, first counting every row's shells (and keeping
+          // the masks while there is room), then, with the counts of the rows before known, picking
+          // and evaluating
+          const int c_first = c;
+          for (int pass = SPLIT ? 0 : 1; pass < 2; ++pass) {
+            int kept = 0, counted = 0;  // blocks of masks kept so far; rows whose shells c has passed
+            for (int r = SPLIT ? wid : 0; r < nrows; r += SPLIT ? kWarps : 1) {
+              int shells = 0;
+              if (SPLIT && pass == 1) {
+                if (counted == 0) c = c_first;
+                int before = 0;
+                for (; counted < r; ++counted) before += s_row[counted].shells[lane];
+                c -= before;
+                if (c < 0) c += (-c + pice - 1) / pice * pice;
               }
-              if (mig_n > kMaxMigrated) {
-                zlo = zl - nc;
-                zhi = zl + nc;
-              } else {
-                for (int m = 0; m < mig_n; ++m) {  // the stencil's visits of a recorded cell stay in
-                  const int zm = __ldg(&s.st->mig_cell[m]) - base;
-                  if (zm < 0 || zm >= dz) continue;  // not in this row's column
-                  for (int u = zm - dz; u <= zm + dz; u += dz)
-                    if (u >= zl - nc && u <= zl + nc) {
-                      zlo = min(zlo, u);
-                      zhi = max(zhi, u);
-                    }
+              const int da = r / side - nc, db = r % side - nc;
+              const int n0 = hx + da, n1 = hy + db;  // unwrapped column of the row (nc < dims)
+              const int w0c = n0 < 0 ? n0 + dx : (n0 >= dx ? n0 - dx : n0);
+              const int w1c = n1 < 0 ? n1 + dy : (n1 >= dy ? n1 - dy : n1);
+              const int t0c = n0 < 0 ? 2 : (n0 >= dx ? 0 : 1), t1c = n1 < 0 ? 2 : (n1 >= dy ? 0 : 1);
+              const int base = dz * (w1c + dy * w0c);
+              // the row's union: unwrapped z cells u0 .. u1 in up to three segments (images -1, 0, +1:
+              // below the box, inside, above), segment k holding sorted indices sa_k .., union entries ob_k ..
+              int sa0 = 0, sa1, sa2 = 0, ob1, ob2, len = 0;
+              if (u0 < 0) {  // below the box: cells u0 + dz .. dz - 1
+                sa0 = __ldg(&s.cell_start[base + u0 + dz]);
+                len = __ldg(&s.cell_start[base + dz]) - sa0;
+              }
+              ob1 = len;
+              {  // inside: cells max(u0, 0) .. min(u1, dz - 1)
+                sa1 = __ldg(&s.cell_start[base + max(u0, 0)]);
+                len += __ldg(&s.cell_start[base + min(u1, dz - 1) + 1]) - sa1;
+              }
+              ob2 = len;
+              if (u1 >= dz) {  // above the box: cells 0 .. u1 - dz
+                sa2 = __ldg(&s.cell_start[base]);
+                len += __ldg(&s.cell_start[base + u1 - dz + 1]) - sa2;
+              }
+              // union entries before unwrapped cell u (u0 <= u <= u1 + 1)
+              auto ucount = [&](int u) -> int {
+                if (u > u1) return len;
+                if (u < 0) return __ldg(&s.cell_start[base + u + dz]) - sa0;
+                if (u < dz) return ob1 + __ldg(&s.cell_start[base + u]) - sa1;
+                return ob2 + __ldg(&s.cell_start[base + u - dz]) - sa2;
+              };
+              // this lane's window, trimmed to the z cells that can hold an atom within rc: the x / y
+              // gaps to the row's column (shrunk by the margin) leave a z half-width sqrt(rc^2 - g^2)
+              // (grown by it)
+              int wb = 0, wl = 0;
+              if (act) {
+                int zlo = zl + nc + 1, zhi = zl - nc - 1;  // empty
+                const float gx = fmaxf(0.0f, fmaxf((float)n0 * fdx - xr, xr - (float)(n0 + 1) * fdx) - mgx);
+                const float gy = fmaxf(0.0f, fmaxf((float)n1 * fdy - yr, yr - (float)(n1 + 1) * fdy) - mgy);
+                const float g2 = __fmaf_rn(gx, gx, gy * gy);
+                if (g2 < frc2) {
+                  const float h = sqrtf(frc2 - g2) + mgz;
+                  zlo = max((int)floorf((zr - h) / fdz), zl - nc);
+                  zhi = min((int)floorf((zr + h) / fdz), zl + nc);
                 }
-              }
-              if (zlo <= zhi) {
-                wb = ucount(zlo);
-                wl = ucount(zhi + 1) - wb;
-              }
-            }
-            if (__reduce_max_sync(FULL, wl) == 0) continue;
-            // walks the windows of the lanes `in`; their starts lie within kColStage - 32 entries of
-            // each other, so every staged tile covers at least one block of 32 steps
-            auto walk = [&](bool in) {
-              const int ml = __reduce_max_sync(FULL, in ? wl : 0);
-              if (ml == 0) return;
-              const int gbb = __reduce_min_sync(FULL, in ? wb : 0x7fffffff);
-              const int spr = __reduce_max_sync(FULL, in ? wb : gbb) - gbb;
-              const int T = (kColStage - spr) & ~31;  // steps per staged tile, whole blocks
-              const float shx = s_shift[wid][0][t0c], shy = s_shift[wid][1][t1c];
-              // lanes not walking step through the stage too, from a position that matches nothing
-              const float wpx = in ? pix : -kColFar, wpy = in ? piy : -kColFar, wpz = in ? piz : -kColFar;
-              const int i0 = in ? wb - gbb : 0;
-              const int wlen = in ? wl : 0;  // steps of this lane's own window
-              for (int t0 = 0; t0 < ml; t0 += T) {
-                const int tl = min(T, ml - t0);
-                const int nb = (tl + 31) >> 5;  // blocks of this tile
-                const int need = spr + tl;      // entries of the tile's windows; up to spr + 32 nb (<=
-                                                // kColStage) are read, the rest staged as far away
-                const int ub = gbb + t0;        // union index of stage entry 0
-                for (int e = lane; e < spr + 32 * nb; e += 32) {
-                  const int g = ub + e;
-                  float4 cv = make_float4(kColFar, kColFar, kColFar, 0.0f);
-                  int idt = 0;
-                  if (g < len && e < need) {
-                    const int zc = g < ob1 ? 2 : (g < ob2 ? 1 : 0);  // z shift code: below 2, inside 1, above 0
-                    const int js = g < ob1 ? sa0 + g : (g < ob2 ? sa1 + (g - ob1) : sa2 + (g - ob2));
-                    const float4 pj = __ldg(&s.sxf[js]);
-                    const int4 mj = __ldg(&s.smeta[js]);
-                    cv = make_float4(pj.x - shx, pj.y - shy, pj.z - s_shift[wid][2][zc], pj.w);
-                    idt = (MODE == kLJ_RBL ? mj.z : mj.x) | (mj.y << kJsBits);
+                if (mig_n > kMaxMigrated) {
+                  zlo = zl - nc;
+                  zhi = zl + nc;
+                } else {
+                  for (int m = 0; m < mig_n; ++m) {  // the stencil's visits of a recorded cell stay in
+                    const int zm = __ldg(&s.st->mig_cell[m]) - base;
+                    if (zm < 0 || zm >= dz) continue;  // not in this row's column
+                    for (int u = zm - dz; u <= zm + dz; u += dz)
+                      if (u >= zl - nc && u <= zl + nc) {
+                        zlo = min(zlo, u);
+                        zhi = max(zhi, u);
+                      }
                   }
-                  s_c[wid][e] = cv;
-                  s_id[wid][e] = idt;
                 }
-                __syncwarp();
-                // the walk: blocks of 32 steps, each step a compare into two bit masks, the picks
-                // and the FP64 re-classification once per block
-                for (int q0 = 0; q0 < nb; q0 += kColQW) {  // at most kColQ steps between evaluations
-                  const int nblk = min(kColQW, nb - q0);
-                  for (int bk = 0; bk < nblk; ++bk) {
-                    const int ib = i0 + 32 * (q0 + bk);  // this lane's stage entry at the block's first step
-                    unsigned cm = 0u, sm = 0u;
-                    auto step = [&](int st) {
-                      const float4 cj = s_c[wid][ib + st];
-                      const float ex = cj.x - wpx, ey = cj.y - wpy, ez = cj.z - wpz;
-                      const float dd = tile_d2(ex, ey, ez);
-                      // x alone: core (or the atom itself, dropped at evaluation); y alone: shell;
-                      // both: within a rounding band of rs^2 or rc^2, classified again in FP64
-                      const bool x = ((dd <= b1) | (dd >= b2)) & (dd <= b3);
-                      const bool y = (dd >= b0) & (dd <= b3);
-                      cm |= x ? (1u << st) : 0u;
-                      sm |= y ? (1u << st) : 0u;
-                    };
-                    const int rem = tl - 32 * (q0 + bk);  // steps of the block: 32 but in the tile's last
-                    if (rem >= 32) {
-#pragma unroll
-                      for (int st = 0; st < 32; ++st) step(st);
-                    } else {
-#pragma unroll 4
-                      for (int st = 0; st < rem; ++st) step(st);
-                    }
-                    // only this lane's own window counts: past its end (the lanes step together) lie
-                    // cells beyond rc or outside the stencil
-                    const int left = wlen - (t0 + 32 * (q0 + bk));
-                    const unsigned vm = left >= 32 ? 0xffffffffu : (left > 0 ? (1u << left) - 1u : 0u);
-                    cm &= vm;
-                    sm &= vm;
-                    for (unsigned bm = cm & sm; bm != 0u; bm &= bm - 1u) {
-                      // a banded candidate from its stage slot: union index, segment, sorted index, image
-                      const int st = __ffs(bm) - 1;
-                      const int g = ub + ib + st;
-                      const int zc = g < ob1 ? 2 : (g < ob2 ? 1 : 0);
+                if (zlo <= zhi) {
+                  wb = ucount(zlo);
+                  wl = ucount(zhi + 1) - wb;
+                }
+              }
+              if (__reduce_max_sync(FULL, wl) == 0) continue;
+              // walks the windows of the lanes `in`; their starts lie within kColStage - 32 entries of
+              // each other, so every staged tile covers at least one block of 32 steps
+              auto walk = [&](bool in) {
+                const int ml = __reduce_max_sync(FULL, in ? wl : 0);
+                if (ml == 0) return;
+                const int gbb = __reduce_min_sync(FULL, in ? wb : 0x7fffffff);
+                const int spr = __reduce_max_sync(FULL, in ? wb : gbb) - gbb;
+                const int T = (kColStage - spr) & ~31;  // steps per staged tile, whole blocks
+                const float shx = sh.shift[0][t0c], shy = sh.shift[1][t1c];
+                // lanes not walking step through the stage too, from a position that matches nothing
+                const float wpx = in ? pix : -kColFar, wpy = in ? piy : -kColFar, wpz = in ? piz : -kColFar;
+                const int i0 = in ? wb - gbb : 0;
+                const int wlen = in ? wl : 0;  // steps of this lane's own window
+                for (int t0 = 0; t0 < ml; t0 += T) {
+                  const int tl = min(T, ml - t0);
+                  const int nb = (tl + 31) >> 5;  // blocks of this tile
+                  const int need = spr + tl;      // entries of the tile's windows; up to spr + 32 nb (<=
+                                                  // kColStage) are read, the rest staged as far away
+                  const int ub = gbb + t0;        // union index of stage entry 0
+                  for (int e = lane; e < spr + 32 * nb; e += 32) {
+                    const int g = ub + e;
+                    float4 cv = make_float4(kColFar, kColFar, kColFar, 0.0f);
+                    int idt = 0;
+                    if (g < len && e < need) {
+                      const int zc = g < ob1 ? 2 : (g < ob2 ? 1 : 0);  // z shift code: below 2, inside 1, above 0
                       const int js = g < ob1 ? sa0 + g : (g < ob2 ? sa1 + (g - ob1) : sa2 + (g - ob2));
-                      const unsigned cs2 = col_classify_fp64(&s, si, js, (t0c - 1) * dx, (t1c - 1) * dy, (zc - 1) * dz);
-                      const unsigned bit = 1u << st;
-                      cm = (cs2 & 1u) ? (cm | bit) : (cm & ~bit);
-                      sm = (cs2 & 2u) ? (sm | bit) : (sm & ~bit);
+                      const float4 pj = __ldg(&s.sxf[js]);
+                      const int4 mj = __ldg(&s.smeta[js]);
+                      cv = make_float4(pj.x - shx, pj.y - shy, pj.z - sh.shift[2][zc], pj.w);
+                      idt = (MODE == kLJ_RBL ? mj.z : mj.x) | (mj.y << kJsBits);
+                    }
+                    sh.c[e] = cv;
+                    sh.id[e] = idt;
+                  }
+                  __syncwarp();
+                  // the walk: blocks of 32 steps, each step a compare into two bit masks, the picks
+                  // and the FP64 re-classification once per block
+                  const bool keep = SPLIT && kept + nb <= kColKeep;  // the same in both passes
+                  const unsigned keep0 = kColQW + kept;
+                  if (keep) kept += nb;
+                  for (int bk = 0; bk < nb; ++bk) {  // nb <= kColQW: a tile is evaluated at once
+                    const int ib = i0 + 32 * bk;  // this lane's stage entry at the block's first step
+                    unsigned cm = 0u, sm = 0u;
+                    if (SPLIT && pass == 1 && keep) {
+                      cm = sh.sel[keep0 + bk][lane];
+                      sm = sh.pk[keep0 + bk][lane];
+                    } else {
+                      auto step = [&](int st) {
+                        const float4 cj = sh.c[ib + st];
+                        const float ex = cj.x - wpx, ey = cj.y - wpy, ez = cj.z - wpz;
+                        const float dd = tile_d2(ex, ey, ez);
+                        // x alone: core (or the atom itself, dropped at evaluation); y alone: shell;
+                        // both: within a rounding band of rs^2 or rc^2, classified again in FP64
+                        const bool x = ((dd <= b1) | (dd >= b2)) & (dd <= b3);
+                        const bool y = (dd >= b0) & (dd <= b3);
+                        cm |= x ? (1u << st) : 0u;
+                        sm |= y ? (1u << st) : 0u;
+                      };
+                      const int rem = tl - 32 * bk;  // steps of the block: 32 but in the tile's last
+                      if (rem >= 32) {
+#pragma unroll
+                        for (int st = 0; st < 32; ++st) step(st);
+                      } else {
+#pragma unroll 4
+                        for (int st = 0; st < rem; ++st) step(st);
+                      }
+                      // only this lane's own window counts: past its end (the lanes step together) lie
+                      // cells beyond rc or outside the stencil
+                      const int left = wlen - (t0 + 32 * bk);
+                      const unsigned vm = left >= 32 ? 0xffffffffu : (left > 0 ? (1u << left) - 1u : 0u);
+                      cm &= vm;
+                      sm &= vm;
+                      for (unsigned bm = cm & sm; bm != 0u; bm &= bm - 1u) {
+                        // a banded candidate from its stage slot: union index, segment, sorted index, image
+                        const int st = __ffs(bm) - 1;
+                        const int g = ub + ib + st;
+                        const int zc = g < ob1 ? 2 : (g < ob2 ? 1 : 0);
+                        const int js = g < ob1 ? sa0 + g : (g < ob2 ? sa1 + (g - ob1) : sa2 + (g - ob2));
+                        const unsigned cs2 =
+                            col_classify_fp64(&s, si, js, (t0c - 1) * dx, (t1c - 1) * dy, (zc - 1) * dz);
+                        const unsigned bit = 1u << st;
+                        cm = (cs2 & 1u) ? (cm | bit) : (cm & ~bit);
+                        sm = (cs2 & 2u) ? (sm | bit) : (sm & ~bit);
+                      }
+                    }
+                    if (SPLIT && pass == 0) {
+                      shells += __popc(sm);
+                      if (keep) {
+                        sh.sel[keep0 + bk][lane] = cm;
+                        sh.pk[keep0 + bk][lane] = sm;
+                      }
+                      continue;
                     }
                     // every pice-th shell in traversal order, c shells still to skip before the next
                     const unsigned pm = lgp >= 0 ? pick_shells_pow2(sm, lgp, c) : pick_shells(sm, pice, c);
-                    s_sel[wid][bk][lane] = cm | pm;
-                    s_pk[wid][bk][lane] = pm;
+                    sh.sel[bk][lane] = cm | pm;
+                    sh.pk[bk][lane] = pm;
                   }
-                  flush(nblk, i0 + 32 * q0);
+                  if (!SPLIT || pass == 1) flush(nb, i0);
+                  __syncwarp();  // the stage is rewritten by the next tile or row
                 }
-                __syncwarp();  // the stage is rewritten by the next tile or row
-              }
-            };
-            const int gmin = __reduce_min_sync(FULL, wl > 0 ? wb : 0x7fffffff);
-            const int gmax = __reduce_max_sync(FULL, wl > 0 ? wb : -1);
-            if (gmax - gmin <= kColStage - 32) {
-              walk(wl > 0);
-            } else {
-              // windows far apart (a sparse home column next to dense ones): the chunk's home cells
-              // take turns, and single lanes where one cell's trimmed windows are still too far apart
-              for (int zg = zmin; zg <= zmax; ++zg) {
-                const bool in = wl > 0 && zl == zg;
-                const int lo = __reduce_min_sync(FULL, in ? wb : 0x7fffffff);
-                const int hi = __reduce_max_sync(FULL, in ? wb : -1);
-                if (hi < 0) continue;
-                if (hi - lo <= kColStage - 32) {
-                  walk(in);
-                } else {
-                  for (unsigned m = __ballot_sync(FULL, in); m; m &= m - 1) walk(in && lane == __ffs(m) - 1);
+              };
+              const int gmin = __reduce_min_sync(FULL, wl > 0 ? wb : 0x7fffffff);
+              const int gmax = __reduce_max_sync(FULL, wl > 0 ? wb : -1);
+              if (gmax - gmin <= kColStage - 32) {
+                walk(wl > 0);
+              } else {
+                // windows far apart (a sparse home column next to dense ones): the chunk's home cells
+                // take turns, and single lanes where one cell's trimmed windows are still too far apart
+                for (int zg = zmin; zg <= zmax; ++zg) {
+                  const bool in = wl > 0 && zl == zg;
+                  const int lo = __reduce_min_sync(FULL, in ? wb : 0x7fffffff);
+                  const int hi = __reduce_max_sync(FULL, in ? wb : -1);
+                  if (hi < 0) continue;
+                  if (hi - lo <= kColStage - 32) {
+                    walk(in);
+                  } else {
+                    for (unsigned m = __ballot_sync(FULL, in); m; m &= m - 1) walk(in && lane == __ffs(m) - 1);
+                  }
                 }
               }
+              if (SPLIT && pass == 0) {
+                s_row[r].shells[lane] = shells;
+                continue;
+              }
+              // the row's force joins the rows before it: an atom's sum is formed row by row in either form
+              const float4 fr = sh.f[lane];
+              if constexpr (SPLIT) {
+                s_row[r].f[lane] = make_float3(fr.x, fr.y, fr.z);
+                if (pass == 1) counted = r + 1;  // picking passed c over the row's shells
+              } else {
+                const float3 ft = sh.ft[lane];
+                sh.ft[lane] = make_float3(ft.x + fr.x, ft.y + fr.y, ft.z + fr.z);
+              }
+              sh.f[lane] = make_float4(0.0f, 0.0f, 0.0f, fr.w);
             }
+            if constexpr (SPLIT) __syncthreads();  // every row counted; every row evaluated
           }
         }
+        if constexpr (SPLIT) {
+          if (wid != 0) continue;  // the first warp adds the rows up
+          float3 ft = make_float3(0.0f, 0.0f, 0.0f);
+          for (int r = 0; r < nrows; ++r) {
+            const float3 fr = s_row[r].f[lane];
+            ft = make_float3(ft.x + fr.x, ft.y + fr.y, ft.z + fr.z);
+          }
+          sh.ft[lane] = ft;
+        }
         if (act) {
-          const float4 fa = s_f[wid][lane];  // Coulomb already scaled by qqr2e inside the pair factor
+          const float3 fa = sh.ft[lane];  // Coulomb already scaled by qqr2e inside the pair factor
           double r9[9];
-  #pragma unroll
+#pragma unroll
           for (int q = 0; q < 9; ++q) r9[q] = 0.0;
           r9[0] = (double)fa.x;
           r9[1] = (double)fa.y;
@@ -2394,30 +2488,40 @@ k_pair_col(const SysDev* __restrict__ S, const int2* __restrict__ work, int nwor
           red1 += r9[1];
           red2 += r9[2];
         }
+        // RBL mean force: a partial per chunk, at a place that is the chunk's own (columns before it
+        // hold at most a0 / 32 + col chunks)
+        red0 = warp_sum(red0);
+        red1 = warp_sum(red1);
+        red2 = warp_sum(red2);
+        if (lane == 0) {
+          double* p = s.vir_part + 3 * ((size_t)(a0 >> 5) + col + ((g0 - a0) >> 5));
+          p[0] = red0;
+          p[1] = red1;
+          p[2] = red2;
+        }
       }
     }
-    // RBL mean force: a partial per column; the column of the system that completes last adds them
-    // in column order (lane k takes columns k, k + 32, ..., then the fixed butterfly)
-    red0 = warp_sum(red0);
-    red1 = warp_sum(red1);
-    red2 = warp_sum(red2);
+    // the item of the system that completes last adds the chunks' partials: lane k takes columns k,
+    // k + 32, ... in order, each column's chunks in order, then the fixed butterfly
+    if (SPLIT && wid != 0) continue;
     const int ncols = dx * dy;
     int last = 0;
     if (lane == 0) {
-      s.vir_part[(size_t)col * 3 + 0] = red0;
-      s.vir_part[(size_t)col * 3 + 1] = red1;
-      s.vir_part[(size_t)col * 3 + 2] = red2;
       __threadfence();
-      last = atomicAdd(&s.st->counter[0], 1u) == (unsigned)(ncols - 1);
+      last = atomicAdd(&s.st->counter[0], 1u) == (unsigned)(ncols * nparts - 1);
       if (last) s.st->counter[0] = 0u;
     }
     if (__shfl_sync(FULL, last, 0)) {
       __threadfence();
       double t0 = 0.0, t1 = 0.0, t2 = 0.0;
       for (int c = lane; c < ncols; c += 32) {
-        t0 += __ldcg(&s.vir_part[(size_t)c * 3 + 0]);
-        t1 += __ldcg(&s.vir_part[(size_t)c * 3 + 1]);
-        t2 += __ldcg(&s.vir_part[(size_t)c * 3 + 2]);
+        const int e0 = __ldg(&s.cell_start[dz * c]), e1 = __ldg(&s.cell_start[dz * (c + 1)]);
+        const double* p = s.vir_part + 3 * ((size_t)(e0 >> 5) + c);
+        for (int q = 0; q < (e1 - e0 + 31) >> 5; ++q) {
+          t0 += __ldcg(&p[3 * q]);
+          t1 += __ldcg(&p[3 * q + 1]);
+          t2 += __ldcg(&p[3 * q + 2]);
+        }
       }
       t0 = warp_sum(t0);
       t1 = warp_sum(t1);
@@ -2428,9 +2532,9 @@ k_pair_col(const SysDev* __restrict__ S, const int2* __restrict__ work, int nwor
         s.st->fmean[2] = t2 / s.n;
       }
     }
-  }  // next column
+  }  // next item
   // the last warp of the launch to finish resets the work counters for the next launch
-  if (lane == 0 && atomicAdd(&ctr[1], 1u) == gridDim.x * (unsigned)kColWarps - 1u) {
+  if (lane == 0 && atomicAdd(&ctr[1], 1u) == gridDim.x * (unsigned)kWarps - 1u) {
     ctr[0] = 0u;
     ctr[1] = 0u;
   }
@@ -2448,8 +2552,12 @@ static void go_near(const Batch& b, cudaStream_t st) {
       if (b.pair.n > 0) {
         k_pair_col_strays<MODE, SPECIAL, NEAR><<<b.atom.n, kAtomBlock, 0, st>>>(b.sys, b.atom.d);
         note_launch();
-        k_pair_col<MODE, SPECIAL, NEAR><<<b.col_grid, kColWarps * 32, 0, st>>>(b.sys, b.pair.d, b.pair.n, b.col_ctr,
-                                                                               band);
+        if (b.col_split)
+          k_pair_col<MODE, SPECIAL, NEAR, true><<<b.col_grid, kColSplit * 32, col_smem(b.col_rows), st>>>(
+              b.sys, b.pair.d, b.pair.n, b.col_parts, b.col_ctr, band);
+        else
+          k_pair_col<MODE, SPECIAL, NEAR, false><<<b.col_grid, kColWarps * 32, 0, st>>>(
+              b.sys, b.pair.d, b.pair.n, b.col_parts, b.col_ctr, band);
         note_launch();
       }
       return;
@@ -2477,18 +2585,35 @@ static void go(const Batch& b, cudaStream_t st) {
   go_near<R, MODE, SPECIAL, VIRIAL, false>(b, st);
 }
 
-int pair_col_grid(int ncols, int ff, int special, int near) {
+template <bool SPLIT>
+static const void* col_kernel(const Batch& b) {
+  if (b.ff == RBMD_FF_LJ_CUT) return (const void*)k_pair_col<kLJ_RBL, false, false, SPLIT>;
+  if (b.special)
+    return b.near ? (const void*)k_pair_col<kCOUL_RBL, true, true, SPLIT>
+                  : (const void*)k_pair_col<kCOUL_RBL, true, false, SPLIT>;
+  return b.near ? (const void*)k_pair_col<kCOUL_RBL, false, true, SPLIT>
+                : (const void*)k_pair_col<kCOUL_RBL, false, false, SPLIT>;
+}
+
+void plan_pair_col(Batch& b, double chunks, double longest, int nc) {
+  const int side = 2 * nc + 1;
+  b.col_rows = side * side;
+  b.col_parts = std::max(1, std::min(1024, (int)std::ceil(1.2 * longest / 32.0)));
+  // Up to about one chunk per resident warp (148 SMs x 16) the split form's eight warps per chunk are
+  // faster: 177 -> 56 us (1200 atoms of saline), 245 -> 145 us (9000), 467 -> 449 us (64,000, 2140
+  // chunks); above, its second staging costs more than it spreads (3420 -> 5460 us for 985,000 atoms).
+  b.col_split = b.col_rows <= kColMaxRows && chunks < 2200;
   int dev = 0, sms = 0, per_sm = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const void* fn = ff == RBMD_FF_LJ_CUT ? (const void*)k_pair_col<kLJ_RBL, false, false>
-                   : special ? (near ? (const void*)k_pair_col<kCOUL_RBL, true, true>
-                                     : (const void*)k_pair_col<kCOUL_RBL, true, false>)
-                             : (near ? (const void*)k_pair_col<kCOUL_RBL, false, true>
-                                     : (const void*)k_pair_col<kCOUL_RBL, false, false>);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kColWarps * 32, 0);
-  const int need = (ncols + kColWarps - 1) / kColWarps;
-  return std::max(1, std::min(need, std::max(1, sms) * std::max(1, per_sm)));
+  const void* fn = b.col_split ? col_kernel<true>(b) : col_kernel<false>(b);
+  const size_t smem = b.col_split ? col_smem(b.col_rows) : 0;
+  const int warps = b.col_split ? kColSplit : kColWarps;
+  if (b.col_split) cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, warps * 32, smem);
+  const long long items = (long long)b.pair.n * b.col_parts;
+  const long long need = b.col_split ? items : (items + kColWarps - 1) / kColWarps;
+  b.col_grid = (int)std::max(1LL, std::min(need, (long long)std::max(1, sms) * std::max(1, per_sm)));
 }
 
 template <typename R, bool VIRIAL>

@@ -21,10 +21,11 @@ struct Batch {
   Work atom, pair, cell, rho, tri, term, kred, draw;
   Work pair_cells;           // column layout: the tile kernel's cell table (energies, other modes)
   // column layout: pair.d lists every column (slot, column index), most atoms per column first;
-  // the persistent column kernel's warps take them in that order from col_ctr[0] (col_ctr[1] counts
-  // the warps that are done; the last one resets both), col_grid blocks
+  // the persistent column kernel takes them in that order from col_ctr[0] (col_ctr[1] counts the warps
+  // that are done; the last one resets both), every column in col_parts items, col_grid blocks;
+  // col_split: eight warps share a chunk of 32 atoms, by its col_rows traversal rows
   unsigned* col_ctr = nullptr;
-  int col_grid = 0;
+  int col_grid = 0, col_parts = 1, col_split = 0, col_rows = 0;
   // uniform switches of the batch (a batch never mixes them)
   int ff = 0, neigh = 0, coul = 0, prec = 0, temp_ctrl = 0, special = 0;
   int has_shake = 0, has_bonded = 0;
@@ -53,9 +54,9 @@ void launch_rbe_sample(const Batch& b, cudaStream_t s);
 void launch_rho(const Batch& b, cudaStream_t s, int ewald);
 void launch_bonded(const Batch& b, cudaStream_t s, int virial);
 void launch_pair(const Batch& b, cudaStream_t s, int virial);
-// Blocks of the persistent column kernel for `ncols` columns: resident blocks per SM x SMs of the
-// current device, fewer when the columns do not fill them (4 warps per block, a column per warp).
-int pair_col_grid(int ncols, int ff, int special, int near);
+// How the column kernel takes a batch (col_* of Batch): chunks is the number of 32-atom chunks its columns
+// hold on average, longest the atoms of its longest columns, nc the cells per cut-off.
+void plan_pair_col(Batch& b, double chunks, double longest, int nc);
 // Far forces (RBE, Ewald) from the structure factor, for launch_final to add.
 void launch_far(const Batch& b, cudaStream_t s, int virial);
 void launch_final(const Batch& b, cudaStream_t s, FinalMode mode, int virial);
