@@ -21,6 +21,7 @@ constexpr int kCellBlock = 256;        // cells per work item of the cell kernel
 constexpr int kBuildCells = 32;        // cells per block of the cell-list build
 constexpr int kCellBigGrid = 16384;    // cells of a system above which counts are added up in two levels
 constexpr int kRbeSlack = 64;          // Metropolis proposal slots tried beyond the samples still to draw
+constexpr int kEamRow = 8;             // doubles per row of the device's rhor and z2r tables
 constexpr int kQueue = 64;             // per-warp pair queue of the pair kernel
 constexpr int kMaxF32Types = 16;       // atom types of the FP32 (mixed) pair table
 
@@ -122,7 +123,7 @@ struct SysDev {
   float fsa, falpha_l2, fqq, fpad;
   double dt, t_start, t_stop, t_damp;
   int64_t num_steps;
-  double eam_dr, eam_drho, eam_rhomax, eam_cut;
+  double eam_dr, eam_rdr, eam_drho, eam_rhomax, eam_cut;
   double rbe_sigma[3];
   // Pair classification thresholds, exact equivalents of the reference's tests on d2 in each
   // precision: d2 <= c[0]  <=>  rc2 - d2 > 1e-4;  d2 >= c[1]  <=>  d2 - rs2 > 1e-4;
@@ -204,9 +205,9 @@ struct SysDev {
   int pad_e;
   // EAM
   double* frho_s;
-  double* rhor_s;
-  double* z2r_s;
-  double* eam_fp;      // [n]
+  double* rhor_s;      // rows of kEamRow: c[3..6], c[0..2], 0
+  double* z2r_s;       // likewise
+  double* eam_fp;      // [n] in cell order
   // reductions
   double* pair_part;   // [blocks_pair * 4]
   double* atom_part;   // [blocks_atom * 8]

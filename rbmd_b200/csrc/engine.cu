@@ -271,7 +271,7 @@ int64_t Context::estimate_bytes(const rbmd_system_desc& d, const rbmd_params& p)
   if (p.force_field == RBMD_FF_EAM) {
     size_t nf, nr, nz;
     eam_table_sizes(d, &nf, &nr, &nz);
-    b += (int64_t)(nf + nr + nz) * 8;
+    b += (int64_t)(nf + (nr + nz) / 7 * kEamRow) * 8;
   }
   if (p.precision == RBMD_PREC_MIXED) b += (int64_t)d.n_types * d.n_types * 8;  // FP32 LJ factors
   if (p.near_table == RBMD_NEAR_TABLE) b += (int64_t)kNearKeys * 4;
@@ -753,23 +753,35 @@ int Context::add_system(const rbmd_system_desc& d, const rbmd_params& p, int32_t
       up(D.rbe_tab, rbe_tab.data(), sizeof(double) * rbe_tab.size());
     }
   }
+  std::vector<double> hrhor, hz2r;  // until the upload is done
   if (p.force_field == RBMD_FF_EAM) {
     D.eam_nrho = d.eam_nrho;
     D.eam_nr = d.eam_nr;
     D.eam_drho = d.eam_drho;
     D.eam_dr = d.eam_dr;
+    D.eam_rdr = 1.0 / d.eam_dr;
     D.eam_rhomax = d.eam_rhomax;
     D.eam_cut = d.eam_cut;
     D.eam_per_type = d.eam_per_type;
     size_t nf, nr, nz;
     eam_table_sizes(d, &nf, &nr, &nz);
     D.frho_s = (double*)dal(sizeof(double) * nf);
-    D.rhor_s = (double*)dal(sizeof(double) * nr);
-    D.z2r_s = (double*)dal(sizeof(double) * nz);
+    // rhor and z2r in rows of two 32-byte halves, the cubic and its derivative
+    auto halves = [](const double* rows, size_t n7, std::vector<double>& out) {
+      out.assign(n7 / 7 * kEamRow, 0.0);
+      for (size_t r = 0; r < n7 / 7; ++r) {
+        for (int k = 0; k < 4; ++k) out[r * kEamRow + k] = rows[r * 7 + 3 + k];
+        for (int k = 0; k < 3; ++k) out[r * kEamRow + 4 + k] = rows[r * 7 + k];
+      }
+    };
+    halves(d.eam_rhor_spline, nr, hrhor);
+    halves(d.eam_z2r_spline, nz, hz2r);
+    D.rhor_s = (double*)dal(sizeof(double) * hrhor.size());
+    D.z2r_s = (double*)dal(sizeof(double) * hz2r.size());
     D.eam_fp = (double*)dal(sizeof(double) * n);
     up(D.frho_s, d.eam_frho_spline, sizeof(double) * nf);
-    up(D.rhor_s, d.eam_rhor_spline, sizeof(double) * nr);
-    up(D.z2r_s, d.eam_z2r_spline, sizeof(double) * nz);
+    up(D.rhor_s, hrhor.data(), sizeof(double) * hrhor.size());
+    up(D.z2r_s, hz2r.data(), sizeof(double) * hz2r.size());
   }
   D.atom_part = (double*)dal(sizeof(double) * 8 * D.blocks_atom);
   // pair-kernel partials: enough for any layout the autotuner may switch to (nine per block; the column

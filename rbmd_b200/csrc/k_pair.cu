@@ -91,7 +91,7 @@ __device__ __forceinline__ float near_table_g(const float* __restrict__ tab, flo
 }
 
 // EAM spline row evaluation (ExecForceFunction::ComputeEAMrho / ComputeEAMforce)
-__device__ inline void eam_row(const double* tab, double r, double rdr, int nr, int& m, double& p) {
+__device__ inline void eam_row(double r, double rdr, int nr, int& m, double& p) {
   p = r * rdr + 1.0;
   m = (int)p;
   m = min(m, nr - 1);
@@ -101,17 +101,37 @@ __device__ inline void eam_row(const double* tab, double r, double rdr, int nr, 
 
 // EAM tables of a type and of a type pair: one table of each kind for every type (funcfl, the
 // reference's EAM), or per type (setfl): frho / rhor by type, z2r by pair i >= j at i (i+1)/2 + j
-// (LAMMPS pair eam/alloy's type2frho, type2rhor, type2z2r).
+// (LAMMPS pair eam/alloy's type2frho, type2rhor, type2z2r).  The EAM passes are bound by the gathers of
+// the pairs' rows (every lane its own), so a row of rhor and z2r is stored as two 32-byte halves -- the
+// cubic c[3..6], then its derivative c[0..2] -- and each half is one load: 32,000 atoms' force pass
+// takes three such loads per pair where it took 13 of 8 bytes.
 __device__ inline const double* eam_frho(const SysDev& s, int t) {
   return s.eam_per_type ? s.frho_s + (size_t)t * 7 * (s.eam_nrho + 1) : s.frho_s;
 }
 __device__ inline const double* eam_rhor(const SysDev& s, int t) {
-  return s.eam_per_type ? s.rhor_s + (size_t)t * 7 * (s.eam_nr + 1) : s.rhor_s;
+  return s.eam_per_type ? s.rhor_s + (size_t)t * kEamRow * (s.eam_nr + 1) : s.rhor_s;
 }
 __device__ inline const double* eam_z2r(const SysDev& s, int a, int b) {
   if (!s.eam_per_type) return s.z2r_s;
   const int hi = max(a, b), lo = min(a, b);
-  return s.z2r_s + (size_t)(hi * (hi + 1) / 2 + lo) * 7 * (s.eam_nr + 1);
+  return s.z2r_s + (size_t)(hi * (hi + 1) / 2 + lo) * kEamRow * (s.eam_nr + 1);
+}
+// The cubic of a row (its value), or its derivative, at p.
+struct EamHalf {
+  double a, b, c, d;
+};
+__device__ __forceinline__ EamHalf eam_half(const double* row) {
+  EamHalf h;
+  asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(h.a), "=d"(h.b), "=d"(h.c), "=d"(h.d) : "l"(row));
+  return h;
+}
+__device__ __forceinline__ double eam_value(const double* row, double p) {
+  const EamHalf h = eam_half(row);
+  return ((h.a * p + h.b) * p + h.c) * p + h.d;
+}
+__device__ __forceinline__ double eam_slope(const double* row, double p) {
+  const EamHalf h = eam_half(row + 4);
+  return (h.a * p + h.b) * p + h.c;
 }
 
 struct PairAcc {
@@ -126,16 +146,18 @@ template <typename R, int MODE, bool SPECIAL, bool VIRIAL, bool NEAR = false>
 __device__ inline void eval_pair(const SysDev& s, int i, int ti, int moli, double qi, double fpi,
                                  int js, bool core, R rx, R ry, R rz, const int* spi, const double* spw,
                                  int nsp, R pice, PairAcc& a) {
-  const int4 mj = __ldg(&s.smeta[js]);  // atom id, type, molecule
+  constexpr bool kEam = MODE == kEAM_RHO || MODE == kEAM_FORCE || MODE == kEAM_ENERGY;
+  int4 mj = make_int4(0, 0, 0, 0);  // atom id, type, molecule (EAM: the type, where tables are per type)
+  if (!kEam || s.eam_per_type) mj = __ldg(&s.smeta[js]);
   const R Lx = (R)s.L[0], Ly = (R)s.L[1], Lz = (R)s.L[2];
-  if (MODE == kEAM_RHO || MODE == kEAM_FORCE || MODE == kEAM_ENERGY) {
+  if (kEam) {
     rx = -rx; ry = -ry; rz = -rz;  // MinDistanceVec(p_i, p_j)
   }
   min_image(rx, ry, rz, Lx, Ly, Lz);
   const R d2 = rx * rx + ry * ry + rz * rz;
   const R rc2 = (R)s.rc2, rs2 = (R)s.rs2;
 
-  if (MODE == kEAM_RHO || MODE == kEAM_FORCE || MODE == kEAM_ENERGY) {
+  if (kEam) {
     const double rsq = (double)d2;
     const double cut = (MODE == kEAM_ENERGY) ? s.eam_cut : s.rc;
     bool ok = core ? (rsq < cut * cut && rsq > 0.01) : (rsq < s.rc * s.rc && rsq > s.rs2);
@@ -143,29 +165,26 @@ __device__ inline void eval_pair(const SysDev& s, int i, int ti, int moli, doubl
     const double rr = sqrt(rsq);
     int m;
     double p;
-    eam_row(s.rhor_s, rr, 1.0 / s.eam_dr, s.eam_nr, m, p);
+    eam_row(rr, s.eam_rdr, s.eam_nr, m, p);
     const double scale = core ? 1.0 : (double)pice;
     const int tj = mj.y;
     if (MODE == kEAM_RHO || MODE == kEAM_ENERGY) {
-      const double* c = eam_rhor(s, tj) + 7 * m;  // the density the neighbour's type contributes
-      a.rho += scale * (((__ldg(c + 3) * p + __ldg(c + 4)) * p + __ldg(c + 5)) * p + __ldg(c + 6));
+      a.rho += scale * eam_value(eam_rhor(s, tj) + kEamRow * m, p);  // what the neighbour's type contributes
       if (MODE == kEAM_ENERGY) {
-        const double* z = eam_z2r(s, ti, tj) + 7 * m;
-        double z2 = ((__ldg(z + 3) * p + __ldg(z + 4)) * p + __ldg(z + 5)) * p + __ldg(z + 6);
+        const double z2 = eam_value(eam_z2r(s, ti, tj) + kEamRow * m, p);
         a.e1 += 0.5 * (z2 * (1.0 / rr));
       }
     } else {
-      const double* ci = eam_rhor(s, ti) + 7 * m;
-      const double rhoip = (__ldg(ci) * p + __ldg(ci + 1)) * p + __ldg(ci + 2);
-      const double* cj = eam_rhor(s, tj) + 7 * m;
-      const double rhojp = (__ldg(cj) * p + __ldg(cj + 1)) * p + __ldg(cj + 2);
-      const double* cz = eam_z2r(s, ti, tj) + 7 * m;
-      const double z2p = (__ldg(cz) * p + __ldg(cz + 1)) * p + __ldg(cz + 2);
-      const double z2 = ((__ldg(cz + 3) * p + __ldg(cz + 4)) * p + __ldg(cz + 5)) * p + __ldg(cz + 6);
+      const double fpj = __ldg(&s.eam_fp[js]);
+      const double rhoip = eam_slope(eam_rhor(s, ti) + kEamRow * m, p);
+      const double rhojp = !s.eam_per_type || ti == tj ? rhoip : eam_slope(eam_rhor(s, tj) + kEamRow * m, p);
+      const double* cz = eam_z2r(s, ti, tj) + kEamRow * m;
+      const double z2p = eam_slope(cz, p);
+      const double z2 = eam_value(cz, p);
       const double recip = 1.0 / rr;
       const double phi = z2 * recip;
       const double phip = z2p * recip - phi * recip;
-      const double psip = fpi * rhojp + __ldg(&s.eam_fp[mj.x]) * rhoip + phip;
+      const double psip = fpi * rhojp + fpj * rhoip + phip;
       const double fpair = -psip * recip;
       a.f[0] += scale * ((double)rx * fpair);
       a.f[1] += scale * ((double)ry * fpair);
@@ -346,7 +365,7 @@ k_pair(const SysDev* __restrict__ S, const int2* __restrict__ work, int cap, int
     int c0 = (int)((xi.x - s.lo[0]) / s.d[0]);
     int c1 = (int)((xi.y - s.lo[1]) / s.d[1]);
     int c2 = (int)((xi.z - s.lo[2]) / s.d[2]);
-    const double fpi = (MODE == kEAM_FORCE) ? s.eam_fp[i] : 0.0;
+    const double fpi = (MODE == kEAM_FORCE) ? s.eam_fp[sidx] : 0.0;
     // special list of i (first 16 entries in shared memory)
     int nsp = 0;
     const int* spi = nullptr;
@@ -558,7 +577,7 @@ k_pair(const SysDev* __restrict__ S, const int2* __restrict__ work, int cap, int
       p -= m;
       p = fmin(p, 1.0);
       const double* c = eam_frho(s, s.meta[i].x) + 7 * m;
-      s.eam_fp[i] = (c[0] * p + c[1]) * p + c[2];
+      s.eam_fp[sidx] = (c[0] * p + c[1]) * p + c[2];
     } else if (MODE == kEAM_ENERGY) {
       const double rho = r9[0];
       double p = rho * (1.0 / s.eam_drho) + 1.0;
@@ -727,7 +746,7 @@ __device__ __forceinline__ void lean_atom(const SysDev& s, int sidx, int lane, L
   const int c0 = (int)((xi.x - s.lo[0]) / d0);
   const int c1 = (int)((xi.y - s.lo[1]) / d1);
   const int c2 = (int)((xi.z - s.lo[2]) / d2c);
-  const double fpi = (MODE == kEAM_FORCE) ? s.eam_fp[i] : 0.0;
+  const double fpi = (MODE == kEAM_FORCE) ? s.eam_fp[sidx] : 0.0;
   int nsp = 0;
   const int* spi = nullptr;
   const double* spw = nullptr;
@@ -1036,7 +1055,7 @@ k_pair2(const SysDev* __restrict__ S, const int2* __restrict__ work) {
       p = fmin(p, 1.0);
       const double* c = eam_frho(s, s.meta[i].x) + 7 * m;
       if (MODE == kEAM_RHO) {
-        s.eam_fp[i] = (c[0] * p + c[1]) * p + c[2];
+        s.eam_fp[sidx] = (c[0] * p + c[1]) * p + c[2];
       } else {
         const double fpv = (c[0] * p + c[1]) * p + c[2];
         double phi = ((c[3] * p + c[4]) * p + c[5]) * p + c[6];
@@ -1249,7 +1268,7 @@ __device__ inline void finish_atom(const SysDev& s, int i, double (&r9)[9]) {
     p = fmin(p, 1.0);
     const double* c = eam_frho(s, s.meta[i].x) + 7 * m;
     if (MODE == kEAM_RHO) {
-      s.eam_fp[i] = (c[0] * p + c[1]) * p + c[2];
+      s.eam_fp[s.rank[i]] = (c[0] * p + c[1]) * p + c[2];
     } else {
       const double fpv = (c[0] * p + c[1]) * p + c[2];
       double phi = ((c[3] * p + c[4]) * p + c[5]) * p + c[6];
@@ -1359,7 +1378,7 @@ __device__ void tile_stray(const SysDev& s, int si, int skip, int pice, bool rbl
   const int i = mi.x, ti = mi.y, moli = mi.z;
   const double4 xd = ldg4(&s.sx[si]);
   const R4 p4 = load_sorted<R>(s, si);
-  const double fpi = (MODE == kEAM_FORCE) ? s.eam_fp[i] : 0.0;
+  const double fpi = (MODE == kEAM_FORCE) ? s.eam_fp[si] : 0.0;
   int nsp = 0;
   const int* spi = nullptr;
   const double* spw = nullptr;
@@ -1529,7 +1548,7 @@ k_pair_tile(const SysDev* __restrict__ S, const int2* __restrict__ work, int cap
       const double qi = xd.w;
       const bool stray = (int)((xd.x - s.lo[0]) / s.d[0]) != hx || (int)((xd.y - s.lo[1]) / s.d[1]) != hy ||
                          (int)((xd.z - s.lo[2]) / s.d[2]) != hz;
-      const double fpi = (MODE == kEAM_FORCE) ? s.eam_fp[i] : 0.0;
+      const double fpi = (MODE == kEAM_FORCE) ? s.eam_fp[si] : 0.0;
       int nsp = 0;
       const int* spi = nullptr;
       const double* spw = nullptr;
