@@ -723,6 +723,13 @@ struct LeanShared {
   R so[3][64];  // segment coordinate offsets
 };
 
+// Cell n of a dimension of d cells wrapped into it, by a true modulo where one image is not enough.
+__device__ __forceinline__ int wrap_cell(int n, int d) {
+  int w = n < 0 ? n + d : (n >= d ? n - d : n);
+  if ((unsigned)w >= (unsigned)d) w = ((n % d) + d) % d;
+  return w;
+}
+
 // The lean traversal of one atom (sorted index sidx) by one warp; the lanes' sums are left in ff (FP32
 // RBL modes, with tab the FP32 LJ factors of the type pairs) or in a.
 template <typename R, int MODE, bool SPECIAL, bool VIRIAL, bool NEAR>
@@ -769,17 +776,19 @@ __device__ __forceinline__ void lean_atom(const SysDev& s, int sidx, int lane, L
   for (int k = 0; k < 32; k += pice) base_mask |= (1u << k);
   const R rc2 = (R)s.rc2, rs2 = (R)s.rs2;
   const int nc = s.nc, side = 2 * nc + 1, nrows = side * side;
-  // conservative culling radius: cells farther than rc from i (with a margin for atoms outside
-  // their cell: at least the farthest an atom lay outside its binned cell plus the largest SHAKE
-  // displacement since the cell list was built) cannot hold a core or shell atom; cells of atoms
-  // SHAKE wrapped across the box (they sit on the far side of it) are never culled, and beyond
-  // kMaxMigrated of them nothing is
-  const double margin =
-      fmax(0.1 * fmin(d0, fmin(d1, d2c)), 1.001 * ((double)__uint_as_float(s.st->shake_disp_bits) +
-                                                   (double)__uint_as_float(s.st->out_bits)));
+  // conservative culling: cells farther than rc from i (with a margin for atoms outside their cell: at
+  // least the farthest an atom lay outside its binned cell plus the largest SHAKE displacement since
+  // the cell list was built) cannot hold a core or shell atom; cells of atoms SHAKE wrapped across the
+  // box (they sit on the far side of it) are never culled, and beyond kMaxMigrated of them nothing is.
+  // In FP32, whose rounding (a millionth of the box covers it) is added to the margin.
+  const float fd0 = (float)d0, fd1 = (float)d1, fd2 = (float)d2c;
+  const float margin = fmaxf(0.1f * fminf(fd0, fminf(fd1, fd2)),
+                             1.001f * (__uint_as_float(s.st->shake_disp_bits) + __uint_as_float(s.st->out_bits))) +
+                       1e-6f * (float)fmax(fabs(xi.x - s.lo[0]) + s.L[0], fmax(fabs(xi.y - s.lo[1]) + s.L[1],
+                                                                             fabs(xi.z - s.lo[2]) + s.L[2]));
   const int mig_n = s.st->mig_n;
-  const double cut2 = s.rc2;
-  const double lo0 = s.lo[0], lo1 = s.lo[1], lo2 = s.lo[2];
+  const float cut2 = 1.0001f * (float)s.rc2;
+  const float xr = (float)(xi.x - s.lo[0]), yr = (float)(xi.y - s.lo[1]), zr = (float)(xi.z - s.lo[2]);
   const float spice = (float)pice;
   const float fsa = (float)sqrt(s.alpha), falpha = (float)s.alpha;
   const float fLx = (float)s.L[0], fLy = (float)s.L[1], fLz = (float)s.L[2];
@@ -816,29 +825,21 @@ __device__ __forceinline__ void lean_atom(const SysDev& s, int sidx, int lane, L
     R oxv = R(0), oyv = R(0), oz0 = R(0), oz1 = R(0), oz2 = R(0);
     if (lane < group && r < nrows) {
       const int da = r / side - nc, db = r % side - nc;
-      int n0 = c0 + da, n1 = c1 + db;
-      int w0 = ((n0 % dx) + dx) % dx;
-      int w1 = ((n1 % dy) + dy) % dy;
-      const double ox = d0 * (double)(w0 - n0), oy = d1 * (double)(w1 - n1);
-      oxv = (R)ox;
-      oyv = (R)oy;
-      // squared gap between i and the column of cells (unwrapped frame), shrunk by the margin
-      const double bx0 = lo0 + n0 * d0 - margin, bx1 = lo0 + (n0 + 1) * d0 + margin;
-      const double by0 = lo1 + n1 * d1 - margin, by1 = lo1 + (n1 + 1) * d1 + margin;
-      const double gx = fmax(0.0, fmax(bx0 - xi.x, xi.x - bx1));
-      const double gy = fmax(0.0, fmax(by0 - xi.y, xi.y - by1));
-      const double gxy = gx * gx + gy * gy;
+      const int n0 = c0 + da, n1 = c1 + db;
+      const int w0 = wrap_cell(n0, dx), w1 = wrap_cell(n1, dy);
+      oxv = (R)(d0 * (double)(w0 - n0));
+      oyv = (R)(d1 * (double)(w1 - n1));
+      // gap between i and the column of cells (unwrapped frame), shrunk by the margin; it leaves a z
+      // half-width sqrt(rc^2 - gap^2)
+      const float gx = fmaxf(0.0f, fmaxf((float)n0 * fd0 - xr, xr - (float)(n0 + 1) * fd0) - margin);
+      const float gy = fmaxf(0.0f, fmaxf((float)n1 * fd1 - yr, yr - (float)(n1 + 1) * fd1) - margin);
+      const float gxy = gx * gx + gy * gy;
       int elo = nc + 1, ehi = -nc - 1;
       if (gxy < cut2) {
-        for (int de = -nc; de <= nc; ++de) {
-          const int n2 = c2 + de;
-          const double bz0 = lo2 + n2 * d2c - margin, bz1 = lo2 + (n2 + 1) * d2c + margin;
-          const double gz = fmax(0.0, fmax(bz0 - xi.z, xi.z - bz1));
-          if (gxy + gz * gz < cut2) {
-            elo = min(elo, de);
-            ehi = max(ehi, de);
-          }
-        }
+        const float h = sqrtf(cut2 - gxy) + margin;
+        // clamped before the conversion: a margin beyond every cell (or a NaN) takes the whole stencil
+        elo = (int)fminf(fmaxf(floorf((zr - h) / fd2) - (float)c2, (float)-nc), (float)(nc + 1));
+        ehi = (int)fmaxf(fminf(floorf((zr + h) / fd2) - (float)c2, (float)nc), (float)(-nc - 1));
       }
       if (mig_n > kMaxMigrated) {
         elo = -nc;
@@ -848,7 +849,7 @@ __device__ __forceinline__ void lean_atom(const SysDev& s, int sidx, int lane, L
           const int cm = __ldg(&s.st->mig_cell[m]) - dz * (w1 + dy * w0);
           if (cm < 0 || cm >= dz) continue;  // not in this row's column
           for (int de = -nc; de <= nc; ++de)
-            if ((((c2 + de) % dz) + dz) % dz == cm) {
+            if (wrap_cell(c2 + de, dz) == cm) {
               elo = min(elo, de);
               ehi = max(ehi, de);
             }
@@ -863,8 +864,8 @@ __device__ __forceinline__ void lean_atom(const SysDev& s, int sidx, int lane, L
           // a cell is d * (wrapped - unwrapped) = -d dz q, -d dz (q + 1), -d dz (q + 2).
           const int base = dz * (w1 + dy * w0);
           const int z0 = c2 + elo, len = ehi - elo + 1;
-          const int zw = ((z0 % dz) + dz) % dz;
-          const int q = (z0 - zw) / dz;
+          const int zw = wrap_cell(z0, dz);
+          const int q = zw == z0 ? 0 : (z0 - zw) / dz;
           sa0 = __ldg(&s.cell_start[base + zw]);
           oz0 = (R)(-d2c * (double)dz * (double)q);
           if (zw + len <= dz) {
