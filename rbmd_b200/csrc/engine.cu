@@ -120,6 +120,9 @@ T thr_above(T c, T e) {
 Context::Context(const rbmd_device_cfg& c) : cfg(c) {
   cudaSetDevice(cfg.device);
   cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking);
+  cudaStreamCreateWithFlags(&side_, cudaStreamNonBlocking);
+  cudaEventCreateWithFlags(&fork_ev_, cudaEventDisableTiming);
+  cudaEventCreateWithFlags(&join_ev_, cudaEventDisableTiming);
   cudaMemPoolProps props;
   std::memset(&props, 0, sizeof(props));
   props.allocType = cudaMemAllocationTypePinned;
@@ -172,6 +175,9 @@ Context::~Context() {
       cudaEventDestroy(e.first);
       cudaEventDestroy(e.second);
     }
+  cudaEventDestroy(fork_ev_);
+  cudaEventDestroy(join_ev_);
+  cudaStreamDestroy(side_);
   cudaStreamDestroy(stream);
 }
 
@@ -1071,30 +1077,60 @@ void Context::timed(const char* name, double units, F&& fn) {
   r.units.push_back(units);
 }
 
-void Context::enqueue_forces(const Batch& b, FinalMode mode, int virial) {
-  timed("cells", 0, [&] { launch_cells(b, stream); });
-  if (b.coul == RBMD_COUL_RBE) timed("rbe_sample", 0, [&] { launch_rbe_sample(b, stream); });
-  if (b.coul != RBMD_COUL_NONE) timed("rho", 0, [&] { launch_rho(b, stream, b.coul == RBMD_COUL_EWALD); });
-  if (b.has_bonded) timed("bonded", 0, [&] { launch_bonded(b, stream, virial); });
+// The side stream goes on from this point of the main stream, or the main stream waits for it.  The
+// k-space chain (samples, structure factor, far force) and the bonded terms only read positions and
+// write arrays of their own until the force assembly, so they run beside the cell list and the pair
+// kernel: a step of a small system is a string of kernels that each leave most of the chip idle.  While
+// profiling everything stays on the main stream, where the timing events are.
+cudaStream_t Context::fork_side() {
+  if (prof.on) return stream;
+  cudaEventRecord(fork_ev_, stream);
+  cudaStreamWaitEvent(side_, fork_ev_, 0);
+  return side_;
+}
+void Context::join_side(cudaStream_t side) {
+  if (side == stream) return;
+  cudaEventRecord(join_ev_, side);
+  cudaStreamWaitEvent(stream, join_ev_, 0);
+}
+
+// From the cell list on: k-space and bonded terms beside the pair forces, then the assembly.
+void Context::enqueue_assembly(const Batch& b, FinalMode mode, int virial) {
+  cudaStream_t side = stream;
+  if (b.coul != RBMD_COUL_NONE || b.has_bonded) {
+    side = fork_side();
+    if (b.coul != RBMD_COUL_NONE) {
+      timed("rho", 0, [&] { launch_rho(b, side, b.coul == RBMD_COUL_EWALD); });
+      timed("far", (double)b.natoms, [&] { launch_far(b, side, virial); });
+    }
+    if (b.has_bonded) timed("bonded", 0, [&] { launch_bonded(b, side, virial); });
+  }
   timed(pair_name(b), (double)b.natoms, [&] { launch_pair(b, stream, virial); });
-  timed("far", (double)b.natoms, [&] { launch_far(b, stream, virial); });
+  join_side(side);
   timed("final", (double)b.natoms, [&] { launch_final(b, stream, mode, virial); });
+}
+
+void Context::enqueue_forces(const Batch& b, FinalMode mode, int virial) {
+  if (b.coul == RBMD_COUL_RBE) {  // the next fork orders what follows on the side stream after it
+    cudaStream_t side = fork_side();
+    timed("rbe_sample", 0, [&] { launch_rbe_sample(b, side); });
+  }
+  timed("cells", 0, [&] { launch_cells(b, stream); });
+  enqueue_assembly(b, mode, virial);
 }
 
 void Context::enqueue_step(const Batch& b) {
   if (b.npt == 2) timed("mtk", 0, [&] { launch_mtk_begin(b, stream); });
   else timed("nhc", 0, [&] { launch_nhc_a(b, stream); });
+  if (b.coul == RBMD_COUL_RBE) {  // needs the step's number and box only
+    cudaStream_t side = fork_side();
+    timed("rbe_sample", 0, [&] { launch_rbe_sample(b, side); });
+  }
   timed("kick_drift", 0, [&] { launch_kick_drift(b, stream); });
   timed("cells", 0, [&] { launch_cells_build(b, stream); });
   if (b.has_shake) timed("shake", 0, [&] { launch_shake(b, stream); });
-  if (b.coul == RBMD_COUL_RBE) timed("rbe_sample", 0, [&] { launch_rbe_sample(b, stream); });
-  if (b.coul != RBMD_COUL_NONE) timed("rho", 0, [&] { launch_rho(b, stream, b.coul == RBMD_COUL_EWALD); });
   // NPT: the barostat needs the virial of this evaluation
-  const int vir = b.npt;
-  if (b.has_bonded) timed("bonded", 0, [&] { launch_bonded(b, stream, vir); });
-  timed(pair_name(b), (double)b.natoms, [&] { launch_pair(b, stream, vir); });
-  timed("far", (double)b.natoms, [&] { launch_far(b, stream, vir); });
-  timed("final", (double)b.natoms, [&] { launch_final(b, stream, kFinalKick, vir); });
+  enqueue_assembly(b, kFinalKick, b.npt);
   if (b.has_shake) {
     timed("rattle", 0, [&] { launch_rattle(b, stream); });
     if (b.temp_ctrl != RBMD_TC_NOSE_HOOVER) timed("ke", 0, [&] { launch_ke_thermostat(b, stream); });
@@ -1342,18 +1378,15 @@ int Context::get_thermo_many(const int32_t* ids, int nsys, rbmd_thermo* outs) {
                       stream);
     cudaMemsetAsync(&D.st->virial[0], 0, sizeof(double) * 6, stream);
   }
+  const bool profiling = prof.on;  // the profile is of the steps' launches
+  prof.on = false;
   for (BatchRec* br : bs) {
     const Batch& b = br->b;
-    launch_cells(b, stream);
-    if (b.coul == RBMD_COUL_RBE) launch_rbe_sample(b, stream);
-    if (b.coul != RBMD_COUL_NONE) launch_rho(b, stream, b.coul == RBMD_COUL_EWALD);
-    if (b.has_bonded) launch_bonded(b, stream, 1);
-    launch_far(b, stream, 1);
-    launch_pair(b, stream, 1);
-    launch_final(b, stream, kFinalForceOnly, 1);
+    enqueue_forces(b, kFinalForceOnly, 1);
     launch_energy(b, stream);
     if (b.coul != RBMD_COUL_NONE) launch_ewald_energy(b, stream);
   }
+  prof.on = profiling;
   for (auto& p : ps) {
     const SysDev& D = p.s->dev;
     cudaMemcpyAsync(D.f, p.fsave, sizeof(double4) * D.n, cudaMemcpyDeviceToDevice, stream);

@@ -171,11 +171,16 @@ class Context {
   void drop_batches_with(int id);
   void enqueue_step(const Batch& b);
   void enqueue_forces(const Batch& b, FinalMode mode, int virial);
+  void enqueue_assembly(const Batch& b, FinalMode mode, int virial);
+  cudaStream_t fork_side();
+  void join_side(cudaStream_t side);
   template <class F> void timed(const char* name, double units, F&& fn);
   int check_cuda(const char* where);
 
   std::vector<System*> systems_;
   std::vector<int> free_slots_;
+  cudaStream_t side_ = nullptr;  // beside `stream` within an evaluation; always joined before its end
+  cudaEvent_t fork_ev_ = nullptr, join_ev_ = nullptr;
   SysDev* d_sys_ = nullptr;
   cudaMemPool_t pool_ = nullptr;
   int slot_cap_ = 0;
