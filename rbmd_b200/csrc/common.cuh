@@ -23,6 +23,7 @@ constexpr int kCellBigGrid = 16384;    // cells of a system above which counts a
 constexpr int kRbeSlack = 64;          // Metropolis proposal slots tried beyond the samples still to draw
 constexpr int kEamRow = 8;             // doubles per row of the device's rhor and z2r tables
 constexpr int kQueue = 64;             // per-warp pair queue of the pair kernel
+constexpr int kMaxLjdTypes = 64;       // atom types of the FP64 pair table (64 KB)
 constexpr int kMaxF32Types = 16;       // atom types of the FP32 (mixed) pair table
 
 // device error word bits (rbmd_thermo.status)
@@ -121,6 +122,7 @@ struct SysDev {
   // FP32 constants of the mixed-precision pair evaluation: sqrt(alpha), alpha log2(e) (so that
   // exp(-alpha d2) = 2^(-falpha_l2 d2)) and qqr2e, each rounded once from FP64
   float fsa, falpha_l2, fqq, fpad;
+  double sa;  // sqrt(alpha)
   double dt, t_start, t_stop, t_damp;
   int64_t num_steps;
   double eam_dr, eam_rdr, eam_drho, eam_rhomax, eam_cut;
@@ -163,6 +165,7 @@ struct SysDev {
   // per-type tables
   double* eps;
   double* sig;
+  double2* ljd;  // by type pair: -24 sqrt(eps_a eps_b) and ((sig_a + sig_b) / 2)^6; nullptr above kMaxLjdTypes
   float2* ljf;  // mixed precision, [ntypes^2] by type pair a ntypes + b: -24 sqrt(eps_a eps_b) and
                 // ((sig_a + sig_b) / 2)^6, each rounded once from FP64
   float* near_tab;  // RBMD_NEAR_TABLE with RBL Coulomb: G by key [kNearKeys]; nullptr: analytic G

@@ -279,7 +279,8 @@ int64_t Context::estimate_bytes(const rbmd_system_desc& d, const rbmd_params& p)
     eam_table_sizes(d, &nf, &nr, &nz);
     b += (int64_t)(nf + (nr + nz) / 7 * kEamRow) * 8;
   }
-  if (p.precision == RBMD_PREC_MIXED) b += (int64_t)d.n_types * d.n_types * 8;  // FP32 LJ factors
+  if (d.n_types <= kMaxLjdTypes) b += (int64_t)d.n_types * d.n_types * 16;      // LJ factors
+  if (p.precision == RBMD_PREC_MIXED) b += (int64_t)d.n_types * d.n_types * 8;  // and in FP32
   if (p.near_table == RBMD_NEAR_TABLE) b += (int64_t)kNearKeys * 4;
   b += ((n + kPairWarps - 1) / kPairWarps) * 72 + ((n + kAtomBlock - 1) / kAtomBlock) * 64 + 4096;
   return b;
@@ -432,6 +433,7 @@ int Context::add_system(const rbmd_system_desc& d, const rbmd_params& p, int32_t
   D.S = s->dv.S_rbe;
   D.qqr2e = u.qqr2e;
   D.fsa = (float)std::sqrt(p.alpha);
+  D.sa = std::sqrt(p.alpha);
   D.falpha_l2 = (float)(p.alpha * 1.4426950408889634);
   D.fqq = (float)u.qqr2e;
   D.fmt2v = u.fmt2v;
@@ -670,6 +672,17 @@ int Context::add_system(const rbmd_system_desc& d, const rbmd_params& p, int32_t
   D.smeta = (int4*)dal(sizeof(int4) * n);
   D.eps = (double*)dal(sizeof(double) * d.n_types);
   D.sig = (double*)dal(sizeof(double) * d.n_types);
+  std::vector<double2> hljd;
+  if (d.n_types <= kMaxLjdTypes) {
+    hljd.resize((size_t)d.n_types * d.n_types);
+    for (int a = 0; a < d.n_types; ++a)
+      for (int b = 0; b < d.n_types; ++b) {
+        const double sg = (d.sigma[a] + d.sigma[b]) / 2;
+        hljd[(size_t)a * d.n_types + b] =
+            make_double2(-24.0 * std::sqrt(d.epsilon[a] * d.epsilon[b]), sg * sg * sg * sg * sg * sg);
+      }
+    D.ljd = (double2*)dal(sizeof(double2) * hljd.size());
+  }
   std::vector<float2> hlj;
   if (D.prec == RBMD_PREC_MIXED) {  // at most kMaxF32Types types (checked above)
     hlj.resize((size_t)d.n_types * d.n_types);
@@ -811,6 +824,7 @@ int Context::add_system(const rbmd_system_desc& d, const rbmd_params& p, int32_t
   up(D.eps, d.epsilon, sizeof(double) * d.n_types);
   up(D.sig, d.sigma, sizeof(double) * d.n_types);
   up(D.ljf, hlj.data(), sizeof(float2) * hlj.size());
+  up(D.ljd, hljd.data(), sizeof(double2) * hljd.size());
   up(D.near_tab, hnear.data(), sizeof(float) * hnear.size());
   up(D.mol_off, mol_off.data(), sizeof(int) * mol_off.size());
   up(D.mol_atoms, mol_atoms.data(), sizeof(int) * n);

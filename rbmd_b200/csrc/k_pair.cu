@@ -75,6 +75,7 @@ __device__ __forceinline__ void classify_fp64(const SysDev& s, double pix, doubl
   core = rbl ? (dd <= s.cls_d[2] && dd > 0.0001) : (dd <= s.cls_d[0] && dd > 0.0001);
 }
 
+constexpr double kSqrtPif = 1.7724538755670267;  // sqrt(kPif)
 __device__ inline double r_sqrt(double x) { return sqrt(x); }
 __device__ inline float r_sqrt(float x) { return sqrtf(x); }
 __device__ inline double r_exp(double x) { return exp(x); }
@@ -195,21 +196,41 @@ __device__ inline void eval_pair(const SysDev& s, int i, int ti, int moli, doubl
 
   if (MODE == kLJ_RBL && moli == mj.z) return;  // same-molecule skip, RunWorklet.cpp:1874-1876
   const int tj = mj.y;
-  const R eps_i = (R)__ldg(&s.eps[ti]), eps_j = (R)__ldg(&s.eps[tj]);
-  const R sig_ij = ((R)__ldg(&s.sig[ti]) + (R)__ldg(&s.sig[tj])) / R(2);
   R w = R(1);
   if (SPECIAL) {
     for (int k = 0; k < nsp; ++k)
       if (spi[k] == mj.x) w = (R)spw[k];
   }
-  const R s6 = sig_ij * sig_ij * sig_ij * sig_ij * sig_ij * sig_ij;
+  // -24 sqrt(eps_i eps_j) and sigma_ij^6 of the type pair, from the table in FP64
+  R clj = R(0), s6 = R(0);
+  constexpr bool kLjForce = MODE != kLIST && MODE != kENERGY;
+  if (kLjForce) {
+    if (sizeof(R) == 8 && s.ljd) {
+      const double2 t = __ldg(&s.ljd[ti * s.ntypes + tj]);
+      clj = (R)t.x;
+      s6 = (R)t.y;
+    } else {
+      const R sig_ij = ((R)__ldg(&s.sig[ti]) + (R)__ldg(&s.sig[tj])) / R(2);
+      clj = R(-24) * r_sqrt((R)__ldg(&s.eps[ti]) * (R)__ldg(&s.eps[tj]));
+      s6 = sig_ij * sig_ij * sig_ij * sig_ij * sig_ij * sig_ij;
+    }
+  }
+  // one root and one division per pair; 1 / r and 1 / r^2 serve every term
+  constexpr bool kCoul = MODE == kCOUL_RBL || MODE == kCOUL_VERLET;
+  const R dis = kCoul ? r_sqrt(d2) : R(0);
+  const R rinv = kCoul ? R(1) / dis : R(0);
+  const R inv2 = kCoul ? rinv * rinv : R(1) / d2;
   auto lj = [&](R cut2lo, R cut2hi) -> R {  // force / r_vector factor (0 outside the window)
     if (d2 < cut2hi && d2 > cut2lo) {
-      const R dis6 = d2 * d2 * d2;
-      const R sd6 = s6 / dis6;
-      return R(-24) * r_sqrt(eps_i * eps_j) * ((R(2) * sd6 - R(1)) * sd6) / d2;
+      const R sd6 = s6 * (inv2 * inv2 * inv2);
+      return clj * ((R(2) * sd6 - R(1)) * sd6) * inv2;
     }
     return R(0);
+  };
+  // erfc(sqrt(a) r) / r^2 + 2 sqrt(a) exp(-a r^2) / (sqrt(pi) r)
+  const R sa = (R)s.sa;
+  auto g_erfc = [&]() -> R {
+    return r_erfc(sa * dis) * inv2 + (R)(2.0 / kSqrtPif) * sa * r_exp(-(R)s.alpha * d2) * rinv;
   };
 
   if (MODE == kLJ_RBL) {
@@ -222,7 +243,6 @@ __device__ inline void eval_pair(const SysDev& s, int i, int ti, int moli, doubl
   if (MODE == kLIST) return;
 
   const R qj = (R)__ldg(reinterpret_cast<const double*>(&s.sx[js]) + 3);
-  const R alpha = (R)s.alpha;
   if (MODE == kCOUL_RBL) {
     const R fl = core ? w * lj(R(0.0001), rs2) : w * (pice * lj(rs2, rc2));
     a.f[0] += (double)(fl * rx);
@@ -231,15 +251,10 @@ __device__ inline void eval_pair(const SysDev& s, int i, int ti, int moli, doubl
     const bool in = core ? (d2 < rc2 && d2 > R(0.0001))
                          : (SPECIAL ? (d2 < rc2 && d2 > rs2) : (d2 < rc2 && d2 > R(0.0001)));
     if (in) {
-      const R dis = r_sqrt(d2);
       R g;
-      if constexpr (NEAR) {  // RBMD_NEAR_TABLE
-        g = (R)near_table_g(s.near_tab, (float)dis);
-      } else {
-        const R sa = r_sqrt(alpha);
-        g = r_erfc(sa * dis) / d2 + R(2) * sa * r_exp(-alpha * d2) / ((R)sqrt(kPif) * dis);
-      }
-      R fc = -(R)qi * qj * g / dis;
+      if constexpr (NEAR) g = (R)near_table_g(s.near_tab, (float)dis);  // RBMD_NEAR_TABLE
+      else g = g_erfc();
+      R fc = -(R)qi * qj * g * rinv;
       if (!core) fc *= pice;
       a.g[0] += (double)(fc * rx);
       a.g[1] += (double)(fc * ry);
@@ -261,15 +276,12 @@ __device__ inline void eval_pair(const SysDev& s, int i, int ti, int moli, doubl
     }
     return;
   }
-  R fcs = R(0), fbs = R(0);
-  R dis = r_sqrt(d2);
-  if (d2 < rc2 && d2 > R(0.0001)) {
-    const R sa = r_sqrt(alpha);
-    const R g = r_erfc(sa * dis) / d2 + R(2) * sa * r_exp(-alpha * d2) / ((R)sqrt(kPif) * dis);
-    fcs = -(R)qi * qj * g / dis;
-    fbs = -(R)qi * qj / (dis * dis * dis);
-  }
   if (MODE == kCOUL_VERLET) {
+    R fcs = R(0), fbs = R(0);
+    if (d2 < rc2 && d2 > R(0.0001)) {
+      fcs = -(R)qi * qj * g_erfc() * rinv;
+      fbs = -(R)qi * qj * (inv2 * rinv);
+    }
     const R qq = (R)s.qqr2e;
     const R fp = SPECIAL ? qq * (fcs - (R(1) - w) * fbs) + w * flj : qq * fcs + flj;
     a.f[0] += (double)(fp * rx);
