@@ -114,14 +114,14 @@ class Context:
 
     def forces(self, sid):
         n = self._sizes[sid][0]
-        f = np.zeros((n, 3))
+        f = np.empty((n, 3))
         self._check(lib().rbmd_get_forces(self.h, sid, _dp(f)))
         return f
 
     def state(self, sid):
         n = self._sizes[sid][0]
-        x, v = np.zeros((n, 3)), np.zeros((n, 3))
-        img = np.zeros((n, 3), np.int32)
+        x, v = np.empty((n, 3)), np.empty((n, 3))
+        img = np.empty((n, 3), np.int32)
         self._check(lib().rbmd_get_state(self.h, sid, _dp(x), _dp(v), _ip(img)))
         return x, v, img
 

@@ -163,6 +163,9 @@ class Context {
   };
   int ensure_slots(int need);
   int upload_record(System* s);
+  int read_back(void* dst, const void* src, size_t bytes);
+  int read3(const double4* src, double* dst, int n);        // nothing for a null dst
+  int write3(double4* dst, const double* src, int n);
   int refresh(System* s);
   void set_layout(System* s, int layout);
   std::vector<int> usable_layouts(const System* s) const;
@@ -179,6 +182,9 @@ class Context {
 
   std::vector<System*> systems_;
   std::vector<int> free_slots_;
+  static constexpr size_t kStageMin = 128 << 10, kStageHalf = 512 << 10;
+  void* stage_ = nullptr;        // pinned, 2 x kStageHalf, from the first large read-back on
+  cudaEvent_t stage_ev_[2] = {nullptr, nullptr};
   cudaStream_t side_ = nullptr;  // beside `stream` within an evaluation; always joined before its end
   cudaEvent_t fork_ev_ = nullptr, join_ev_ = nullptr;
   SysDev* d_sys_ = nullptr;

@@ -259,4 +259,31 @@ void launch_snapshot_pack(const SysDev* sys, int slot, int n, void* out, cudaStr
   note_launch();
 }
 
+// The host's rows of three doubles from and to the device's double4 records (whose fourth component,
+// charge or mass, stays): packed here, a read-back crosses PCIe as the caller's array holds it.
+__global__ void k_pack3(const double4* __restrict__ src, double* __restrict__ dst, int n) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const double4 p = src[i];
+  dst[3 * (size_t)i] = p.x;
+  dst[3 * (size_t)i + 1] = p.y;
+  dst[3 * (size_t)i + 2] = p.z;
+}
+
+__global__ void k_unpack3(double4* __restrict__ dst, const double* __restrict__ src, int n) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  dst[i] = make_double4(src[3 * (size_t)i], src[3 * (size_t)i + 1], src[3 * (size_t)i + 2], dst[i].w);
+}
+
+void launch_pack3(const double4* src, double* dst, int n, cudaStream_t s) {
+  k_pack3<<<(n + kObsThreads - 1) / kObsThreads, kObsThreads, 0, s>>>(src, dst, n);
+  note_launch();
+}
+
+void launch_unpack3(double4* dst, const double* src, int n, cudaStream_t s) {
+  k_unpack3<<<(n + kObsThreads - 1) / kObsThreads, kObsThreads, 0, s>>>(dst, src, n);
+  note_launch();
+}
+
 }  // namespace rbmd

@@ -115,6 +115,10 @@ void launch_rdf_count(const SysDev* sys, int slot, const int* centers, int nc, c
 size_t snapshot_bytes(int n);
 void launch_snapshot_pack(const SysDev* sys, int slot, int n, void* out, cudaStream_t s);
 
+// Rows of three doubles packed from, or written into, the first three components of double4 records.
+void launch_pack3(const double4* src, double* dst, int n, cudaStream_t s);
+void launch_unpack3(double4* dst, const double* src, int n, cudaStream_t s);
+
 constexpr int kCellWarpsHost = 4;  // home cells per block of the tile pair kernel
 constexpr double kTileMinPerCell = 3.0;  // mean atoms per cell from which the tile kernel is used
 
