@@ -19,6 +19,8 @@ constexpr int kRhoChunk = 256;         // most atoms per block of the structure-
 constexpr int kFarAtoms = 64;          // atoms per block of the far-force kernel (four threads each)
 constexpr int kCellBlock = 256;        // cells per work item of the cell kernels
 constexpr int kBuildCells = 32;        // cells per block of the cell-list build
+constexpr int kBuildFew = 8;           // and in systems of up to kFewCells cells
+constexpr int kFewCells = 1024;
 constexpr int kCellBigGrid = 16384;    // cells of a system above which counts are added up in two levels
 constexpr int kRbeSlack = 64;          // Metropolis proposal slots tried beyond the samples still to draw
 constexpr int kEamRow = 8;             // doubles per row of the device's rhor and z2r tables

@@ -967,6 +967,7 @@ Context::BatchRec* Context::build_batch(const std::vector<System*>& group, int& 
     slots.push_back(s->slot);
     br->ids.push_back(s->id);
     if (D.ncell_cap > kCellBigGrid) b.big_cells = 1;
+    if (D.ncell_cap <= kFewCells) b.few_cells = 1;
     b.max_P = std::max(b.max_P, std::max(D.P, D.nk_ewald));
     b.natoms += D.n;
     for (int k = 0; k < D.n; k += kAtomBlock) wa.push_back(make_int2(s->slot, k));

@@ -21,11 +21,12 @@ __global__ void k_cells_count(const SysDev* __restrict__ S, const int2* __restri
   bin_atom(s, i, pc);
 }
 
-// kBuildCells cells per block: one warp scans their counts.  A block per work item (kCellBlock cells)
-// meant 8-16 cells per warp one after the other, and 1 or 2 blocks for a box of a few hundred cells.
+// kBuildCells cells per block (one warp scans their counts), kBuildFew in systems of few cells, so that a
+// box of a few hundred cells has a warp per cell and blocks for a third of the chip: with 32 cells per
+// block the kernel took 9 us for 512 cells of 18 atoms and 58 us for 27 cells of 167.
 constexpr int kBuildThreads = 256;
-constexpr int kBuildSplit = kCellBlock / kBuildCells;
-static_assert(kCellBlock % kBuildCells == 0, "a work item is a whole number of build blocks");
+static_assert(kCellBlock % kBuildCells == 0 && kBuildCells % kBuildFew == 0 && kBuildCells == 32 && kBuildFew % 4 == 0,
+              "a work item is a whole number of build blocks, a block's counts start on 16 bytes");
 
 // Atoms per group of kBuildCells cells, for systems of more than kCellBigGrid cells.
 __global__ void k_cells_group_sums(const SysDev* __restrict__ S, const int2* __restrict__ work) {
@@ -38,26 +39,28 @@ __global__ void k_cells_group_sums(const SysDev* __restrict__ S, const int2* __r
   if ((threadIdx.x & 31) == 0 && c < s.ncell) s.cell_gsum[c / kBuildCells] = sum;
 }
 
-// One block per kBuildCells cells.  Bound by latency: the loads of the preceding counts (at most
+// One block per kBuildCells (or kBuildFew) cells.  Bound by latency: the loads of the preceding counts (at most
 // kCellBigGrid / (4 x 256) 16-byte loads per thread; above that the group sums of the kernel before),
 // then one dependent gather per atom.  A cell's ids are taken by 8 lanes where buckets are small (cells
 // of a few atoms) and by a warp otherwise; each lane ranks its ids against the whole bucket, so cells
-// of hundreds of atoms need no serial sort.  `blocks` is the number of blocks per system where the work
-// table covers a single system's present cells only, 0 where it covers the ncell_cap of each.
+// of hundreds of atoms need no serial sort.  `items` is the number of work items where the table covers a
+// single system's present cells only, 0 where it covers the ncell_cap of each system.
 __global__ void __launch_bounds__(kBuildThreads) k_cells_build(const SysDev* __restrict__ S,
-                                                             const int2* __restrict__ work, int big, int blocks) {
+                                                             const int2* __restrict__ work, int big, int items) {
   const int2 w = work[blockIdx.x];
   const SysDev& s = S[w.x];
   SysState* st = s.st;
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-  const int c0 = w.y + blockIdx.y * kBuildCells;
+  const int per = s.ncell_cap <= kFewCells ? kBuildFew : kBuildCells;
+  if ((int)blockIdx.y * per >= kCellBlock) return;  // the grid is for the smaller blocks
+  const int c0 = w.y + blockIdx.y * per;
   const int par = st->cell_epoch & 1;
   const int* count = s.cell_count + (size_t)par * s.cell_stride;
   int* other = s.cell_count + (size_t)(par ^ 1) * s.cell_stride;
   __shared__ int s_sum[kBuildThreads / 32], s_start[kBuildCells], s_cnt[kBuildCells];
   if (c0 < s.ncell) {  // block-uniform
     int sum = 0;
-    if (big) {
+    if (big && per == kBuildCells) {
       for (int g = tid; g < c0 / kBuildCells; g += kBuildThreads) sum += s.cell_gsum[g];
     } else {
       const int4* c4 = reinterpret_cast<const int4*>(count);  // c0 is a multiple of 4
@@ -73,12 +76,13 @@ __global__ void __launch_bounds__(kBuildThreads) k_cells_build(const SysDev* __r
       int base = lane < kBuildThreads / 32 ? s_sum[lane] : 0;
       base = __reduce_add_sync(0xffffffffu, base);
       const int c = c0 + lane;
-      const int cnt = c < s.ncell ? count[c] : 0;
+      const bool mine = lane < per && c < s.ncell;
+      const int cnt = mine ? count[c] : 0;
       const int incl = warp_incl_scan(cnt, lane);
       s_start[lane] = base + incl - cnt;
       s_cnt[lane] = cnt;
-      if (c < s.ncell) s.cell_start[c] = base + incl - cnt;
-      if (c == s.ncell - 1) s.cell_start[s.ncell] = base + incl;
+      if (mine) s.cell_start[c] = base + incl - cnt;
+      if (mine && c == s.ncell - 1) s.cell_start[s.ncell] = base + incl;
     }
     __syncthreads();
     const int cap = s.cell_cap;
@@ -93,12 +97,16 @@ __global__ void __launch_bounds__(kBuildThreads) k_cells_build(const SysDev* __r
       const int4 m = s.meta[i];
       s.smeta[k] = make_int4(i, m.x, m.y, m.z);
     };
-    for (int cc = tid / lanes; cc < kBuildCells; cc += kBuildThreads / lanes) {
+    for (int cc = tid / lanes; cc < per; cc += kBuildThreads / lanes) {
       const int c = c0 + cc, cnt = s_cnt[cc], in = min(cnt, cap);
       const int* ids = s.cell_bucket + (size_t)c * cap;
       auto rank_of = [&](int id) {
-        int r = 0;
-        for (int j = 0; j < in; ++j) r += ids[j] < id ? 1 : 0;
+        int r = 0, j = 0;
+        for (; j + 4 <= in; j += 4) {  // a bucket starts on 16 bytes
+          const int4 v = *reinterpret_cast<const int4*>(ids + j);
+          r += (v.x < id ? 1 : 0) + (v.y < id ? 1 : 0) + (v.z < id ? 1 : 0) + (v.w < id ? 1 : 0);
+        }
+        for (; j < in; ++j) r += ids[j] < id ? 1 : 0;
         return r;
       };
       if (cnt <= cap) {
@@ -128,12 +136,12 @@ __global__ void __launch_bounds__(kBuildThreads) k_cells_build(const SysDev* __r
       st->ovf_n[par ^ 1] = 0;
     }
   }
-  if (blocks == 0) blocks = (s.ncell_cap + kCellBlock - 1) / kCellBlock * kBuildSplit;
-  if (tid < kBuildCells && c0 + tid < s.ncell_cap) other[c0 + tid] = 0;
+  if (items == 0) items = (s.ncell_cap + kCellBlock - 1) / kCellBlock;
+  if (tid < per && c0 + tid < s.ncell_cap) other[c0 + tid] = 0;
   if (c0 == 0)
-    for (int c = blocks * kBuildCells + tid; c < s.ncell_cap; c += kBuildThreads) other[c] = 0;
+    for (int c = items * kCellBlock + tid; c < s.ncell_cap; c += kBuildThreads) other[c] = 0;
   // every block has read this list's buffer index: the next list takes the other buffer
-  if (arrive_last(&st->counter[7], (unsigned)blocks) && tid == 0) st->cell_epoch ^= 1;
+  if (arrive_last(&st->counter[7], (unsigned)(items * (kCellBlock / per))) && tid == 0) st->cell_epoch ^= 1;
 }
 
 void launch_cells_build(const Batch& b, cudaStream_t st) {
@@ -141,8 +149,8 @@ void launch_cells_build(const Batch& b, cudaStream_t st) {
     k_cells_group_sums<<<b.cell.n, kCellBlock, 0, st>>>(b.sys, b.cell.d);
     note_launch();
   }
-  k_cells_build<<<dim3(b.cell.n, kBuildSplit), kBuildThreads, 0, st>>>(b.sys, b.cell.d, b.big_cells,
-                                                                           b.cell_blocks);
+  const dim3 grid(b.cell.n, kCellBlock / (b.few_cells ? kBuildFew : kBuildCells));
+  k_cells_build<<<grid, kBuildThreads, 0, st>>>(b.sys, b.cell.d, b.big_cells, b.cell_items);
   note_launch();
 }
 

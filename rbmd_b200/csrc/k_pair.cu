@@ -2820,7 +2820,8 @@ int launch_rbl_lists_static(const SysDev* sys, int slot, int n, int ncell, int d
   b.cell.d = w_cell;
   b.cell.n = nc;
   b.big_cells = ncell > kCellBigGrid;
-  b.cell_blocks = nc * (kCellBlock / kBuildCells);
+  b.few_cells = 1;  // the system's own record says; a block too many ends at once
+  b.cell_items = nc;
   launch_cells(b, st);
   if (dense)
     k_pair_tile<double, kLIST, false, false><<<np, kCellWarps * 32, 0, st>>>(sys, w_pair, cap, out->n_core,

@@ -34,7 +34,8 @@ struct Batch {
   int npt = 0;               // NPT barostat: 0 none, 1 Berendsen (end of step), 2 MTK (around the integrator)
   int near = 0;              // RBL Coulomb with the reference's near-Coulomb table (RBMD_NEAR_TABLE)
   int big_cells = 0;         // a system has more than kCellBigGrid cells
-  int cell_blocks = 0;       // one system whose cell table covers its present cells only: its build blocks
+  int few_cells = 0;         // a system has at most kFewCells cells
+  int cell_items = 0;        // one system whose cell table covers its present cells only: its entries
   int max_P = 0;             // largest P (or Ewald nk) in the batch
   float band[4] = {0, 0, 0, 0};  // FP32 classification bands: union over the batch (same rc, rs)
   long long natoms = 0;      // atoms over all systems of the batch
