@@ -724,6 +724,115 @@ __device__ inline void acc_zero(float (&ff)[6], PairAcc& a) {
   a.rho = a.e0 = a.e1 = 0.0;
 }
 
+// Cell n of a dimension of d cells wrapped into it, by a true modulo where one image is not enough.
+__device__ __forceinline__ int wrap_cell(int n, int d) {
+  int w = n < 0 ? n + d : (n >= d ? n - d : n);
+  if ((unsigned)w >= (unsigned)d) w = ((n % d) + d) % d;
+  return w;
+}
+
+// An atom's home cell and what culling its stencil needs.  The home cell is by truncation and NOT
+// clamped (InWhichCell, ExecPointLocator.h:271-274): an atom that a step left outside the box walks the
+// neighbourhood of its unclamped cell, every neighbour cell wrapped by a true modulo.
+struct LeanHome {
+  int c0, c1, c2;
+  float fd0, fd1, fd2;  // cell widths
+  float xr, yr, zr;     // position in the box
+  float margin;
+};
+// A traversal row (fixed x and y cell offset): up to three ranges of the cell-ordered arrays, first index
+// and length, and the shift in cells (wrapped - unwrapped) of x, y and each range's z.
+struct LeanRow {
+  int sx, sy, sz0, sz1, sz2, a0, a1, a2, n0, n1, n2;
+};
+
+// Conservative culling: cells farther than rc from the atom (with a margin for atoms outside their cell: at
+// least the farthest an atom lay outside its binned cell plus the largest SHAKE displacement since the
+// cell list was built) cannot hold a core or shell atom; cells of atoms SHAKE wrapped across the box
+// (they sit on the far side of it) are never culled, and beyond kMaxMigrated of them nothing is.  In
+// FP32, whose rounding (a millionth of the box covers it) is added to the margin.
+__device__ __forceinline__ LeanHome lean_home(const SysDev& s, const double4& xi, int c0, int c1, int c2) {
+  LeanHome h;
+  h.c0 = c0;
+  h.c1 = c1;
+  h.c2 = c2;
+  h.fd0 = (float)s.d[0];
+  h.fd1 = (float)s.d[1];
+  h.fd2 = (float)s.d[2];
+  h.margin = fmaxf(0.1f * fminf(h.fd0, fminf(h.fd1, h.fd2)),
+                   1.001f * (__uint_as_float(s.st->shake_disp_bits) + __uint_as_float(s.st->out_bits))) +
+             1e-6f * (float)fmax(fabs(xi.x - s.lo[0]) + s.L[0], fmax(fabs(xi.y - s.lo[1]) + s.L[1],
+                                                                   fabs(xi.z - s.lo[2]) + s.L[2]));
+  h.xr = (float)(xi.x - s.lo[0]);
+  h.yr = (float)(xi.y - s.lo[1]);
+  h.zr = (float)(xi.z - s.lo[2]);
+  return h;
+}
+
+// Row (da, db) of the stencil, trimmed; returns its number of candidates.
+__device__ __forceinline__ int lean_row(const SysDev& s, const LeanHome& h, int da, int db, LeanRow& w) {
+  const int dx = s.dims[0], dy = s.dims[1], dz = s.dims[2], nc = s.nc;
+  const float cut2 = 1.0001f * (float)s.rc2;
+  const int mig_n = s.st->mig_n;
+  const int n0 = h.c0 + da, n1 = h.c1 + db;
+  const int w0 = wrap_cell(n0, dx), w1 = wrap_cell(n1, dy);
+  w.sx = w0 - n0;
+  w.sy = w1 - n1;
+  w.sz0 = w.sz1 = w.sz2 = w.a0 = w.a1 = w.a2 = w.n0 = w.n1 = w.n2 = 0;
+  // gap between the atom and the column of cells (unwrapped frame), shrunk by the margin; it leaves a z
+  // half-width sqrt(rc^2 - gap^2)
+  const float gx = fmaxf(0.0f, fmaxf((float)n0 * h.fd0 - h.xr, h.xr - (float)(n0 + 1) * h.fd0) - h.margin);
+  const float gy = fmaxf(0.0f, fmaxf((float)n1 * h.fd1 - h.yr, h.yr - (float)(n1 + 1) * h.fd1) - h.margin);
+  const float gxy = gx * gx + gy * gy;
+  int elo = nc + 1, ehi = -nc - 1;
+  if (gxy < cut2) {
+    const float hw = sqrtf(cut2 - gxy) + h.margin;
+    // clamped before the conversion: a margin beyond every cell (or a NaN) takes the whole stencil
+    elo = (int)fminf(fmaxf(floorf((h.zr - hw) / h.fd2) - (float)h.c2, (float)-nc), (float)(nc + 1));
+    ehi = (int)fmaxf(fminf(floorf((h.zr + hw) / h.fd2) - (float)h.c2, (float)nc), (float)(-nc - 1));
+  }
+  const int base = dz * (w1 + dy * w0);
+  if (mig_n > kMaxMigrated) {
+    elo = -nc;
+    ehi = nc;
+  } else {
+    for (int m = 0; m < mig_n; ++m) {
+      const int cm = __ldg(&s.st->mig_cell[m]) - base;
+      if (cm < 0 || cm >= dz) continue;  // not in this row's column
+      for (int de = -nc; de <= nc; ++de)
+        if (wrap_cell(h.c2 + de, dz) == cm) {
+          elo = min(elo, de);
+          ehi = max(ehi, de);
+        }
+    }
+  }
+  if (elo > ehi) return 0;
+  // unwrapped z cells [z0, z1] (len <= 2 nc + 1 <= 2 dz - 1 of them) start in the periodic copy
+  // q = floor(z0 / dz); they map to wrapped cells [zw, zw + len) when that stays below dz, else to
+  // [zw, dz), then [0, rest) of the next copy, or [0, dz) and [0, rest - dz) of the two next when the
+  // stencil is longer than the box
+  const int z0 = h.c2 + elo, len = ehi - elo + 1;
+  const int zw = wrap_cell(z0, dz);
+  w.sz0 = zw - z0;
+  w.sz1 = w.sz0 - dz;
+  w.sz2 = w.sz1 - dz;
+  w.a0 = __ldg(&s.cell_start[base + zw]);
+  if (zw + len <= dz) {
+    w.n0 = __ldg(&s.cell_start[base + zw + len]) - w.a0;
+  } else {
+    w.n0 = __ldg(&s.cell_start[base + dz]) - w.a0;
+    const int rest = zw + len - dz;
+    w.a1 = w.a2 = __ldg(&s.cell_start[base]);
+    if (rest <= dz) {
+      w.n1 = __ldg(&s.cell_start[base + rest]) - w.a1;
+    } else {
+      w.n1 = __ldg(&s.cell_start[base + dz]) - w.a1;
+      w.n2 = __ldg(&s.cell_start[base + rest - dz]) - w.a2;
+    }
+  }
+  return w.n0 + w.n1 + w.n2;
+}
+
 // What a warp of the lean traversal keeps in shared memory: its pair queue and its segment table.
 template <typename R>
 struct LeanShared {
@@ -735,13 +844,6 @@ struct LeanShared {
   R so[3][64];  // segment coordinate offsets
 };
 
-// Cell n of a dimension of d cells wrapped into it, by a true modulo where one image is not enough.
-__device__ __forceinline__ int wrap_cell(int n, int d) {
-  int w = n < 0 ? n + d : (n >= d ? n - d : n);
-  if ((unsigned)w >= (unsigned)d) w = ((n % d) + d) % d;
-  return w;
-}
-
 // The lean traversal of one atom (sorted index sidx) by one warp; the lanes' sums are left in ff (FP32
 // RBL modes, with tab the FP32 LJ factors of the type pairs) or in a.
 template <typename R, int MODE, bool SPECIAL, bool VIRIAL, bool NEAR>
@@ -751,7 +853,7 @@ __device__ __forceinline__ void lean_atom(const SysDev& s, int sidx, int lane, L
   constexpr bool F32 = sizeof(R) == 4 && (MODE == kLJ_RBL || MODE == kCOUL_RBL);
   const unsigned FULL = 0xffffffffu;
   const int ntypes = s.ntypes;
-  const int dx = s.dims[0], dy = s.dims[1], dz = s.dims[2];
+  const int dz = s.dims[2];
   const double d0 = s.d[0], d1 = s.d[1], d2c = s.d[2];
   const int4 mi = __ldg(&s.smeta[sidx]);
   i = mi.x;
@@ -759,12 +861,8 @@ __device__ __forceinline__ void lean_atom(const SysDev& s, int sidx, int lane, L
   const double4 xi = ldg4(&s.sx[sidx]);
   const R4 pi4 = load_sorted<R>(s, sidx);
   const R pix = pi4.x, piy = pi4.y, piz = pi4.z;
-  // home cell by truncation and NOT clamped (InWhichCell, ExecPointLocator.h:271-274): an atom
-  // that a step left outside the box walks the neighbourhood of its unclamped cell, every
-  // neighbour cell wrapped by a true modulo below
-  const int c0 = (int)((xi.x - s.lo[0]) / d0);
-  const int c1 = (int)((xi.y - s.lo[1]) / d1);
-  const int c2 = (int)((xi.z - s.lo[2]) / d2c);
+  const LeanHome home = lean_home(s, xi, (int)((xi.x - s.lo[0]) / d0), (int)((xi.y - s.lo[1]) / d1),
+                                  (int)((xi.z - s.lo[2]) / d2c));
   const double fpi = (MODE == kEAM_FORCE) ? s.eam_fp[sidx] : 0.0;
   int nsp = 0;
   const int* spi = nullptr;
@@ -788,19 +886,6 @@ __device__ __forceinline__ void lean_atom(const SysDev& s, int sidx, int lane, L
   for (int k = 0; k < 32; k += pice) base_mask |= (1u << k);
   const R rc2 = (R)s.rc2, rs2 = (R)s.rs2;
   const int nc = s.nc, side = 2 * nc + 1, nrows = side * side;
-  // conservative culling: cells farther than rc from i (with a margin for atoms outside their cell: at
-  // least the farthest an atom lay outside its binned cell plus the largest SHAKE displacement since
-  // the cell list was built) cannot hold a core or shell atom; cells of atoms SHAKE wrapped across the
-  // box (they sit on the far side of it) are never culled, and beyond kMaxMigrated of them nothing is.
-  // In FP32, whose rounding (a millionth of the box covers it) is added to the margin.
-  const float fd0 = (float)d0, fd1 = (float)d1, fd2 = (float)d2c;
-  const float margin = fmaxf(0.1f * fminf(fd0, fminf(fd1, fd2)),
-                             1.001f * (__uint_as_float(s.st->shake_disp_bits) + __uint_as_float(s.st->out_bits))) +
-                       1e-6f * (float)fmax(fabs(xi.x - s.lo[0]) + s.L[0], fmax(fabs(xi.y - s.lo[1]) + s.L[1],
-                                                                             fabs(xi.z - s.lo[2]) + s.L[2]));
-  const int mig_n = s.st->mig_n;
-  const float cut2 = 1.0001f * (float)s.rc2;
-  const float xr = (float)(xi.x - s.lo[0]), yr = (float)(xi.y - s.lo[1]), zr = (float)(xi.z - s.lo[2]);
   const float spice = (float)pice;
   const float fsa = (float)sqrt(s.alpha), falpha = (float)s.alpha;
   const float fLx = (float)s.L[0], fLy = (float)s.L[1], fLz = (float)s.L[2];
@@ -832,77 +917,11 @@ __device__ __forceinline__ void lean_atom(const SysDev& s, int sidx, int lane, L
   for (int r0 = 0; r0 < nrows; r0 += group) {
     // ---- segment table of rows r0 .. r0 + group - 1 (one row per lane)
     const int r = r0 + lane;
-    int nseg = 0, cnt = 0;
-    int sa0 = 0, sa1 = 0, sa2 = 0, n0c = 0, n1c = 0, n2c = 0;
-    R oxv = R(0), oyv = R(0), oz0 = R(0), oz1 = R(0), oz2 = R(0);
-    if (lane < group && r < nrows) {
-      const int da = r / side - nc, db = r % side - nc;
-      const int n0 = c0 + da, n1 = c1 + db;
-      const int w0 = wrap_cell(n0, dx), w1 = wrap_cell(n1, dy);
-      oxv = (R)(d0 * (double)(w0 - n0));
-      oyv = (R)(d1 * (double)(w1 - n1));
-      // gap between i and the column of cells (unwrapped frame), shrunk by the margin; it leaves a z
-      // half-width sqrt(rc^2 - gap^2)
-      const float gx = fmaxf(0.0f, fmaxf((float)n0 * fd0 - xr, xr - (float)(n0 + 1) * fd0) - margin);
-      const float gy = fmaxf(0.0f, fmaxf((float)n1 * fd1 - yr, yr - (float)(n1 + 1) * fd1) - margin);
-      const float gxy = gx * gx + gy * gy;
-      int elo = nc + 1, ehi = -nc - 1;
-      if (gxy < cut2) {
-        const float h = sqrtf(cut2 - gxy) + margin;
-        // clamped before the conversion: a margin beyond every cell (or a NaN) takes the whole stencil
-        elo = (int)fminf(fmaxf(floorf((zr - h) / fd2) - (float)c2, (float)-nc), (float)(nc + 1));
-        ehi = (int)fmaxf(fminf(floorf((zr + h) / fd2) - (float)c2, (float)nc), (float)(-nc - 1));
-      }
-      if (mig_n > kMaxMigrated) {
-        elo = -nc;
-        ehi = nc;
-      } else {
-        for (int m = 0; m < mig_n; ++m) {
-          const int cm = __ldg(&s.st->mig_cell[m]) - dz * (w1 + dy * w0);
-          if (cm < 0 || cm >= dz) continue;  // not in this row's column
-          for (int de = -nc; de <= nc; ++de)
-            if (wrap_cell(c2 + de, dz) == cm) {
-              elo = min(elo, de);
-              ehi = max(ehi, de);
-            }
-        }
-      }
-      {
-        if (elo <= ehi) {
-          // unwrapped z cells [z0, z1] (len <= 2 nc + 1 <= 2 dz - 1 of them) start in the
-          // periodic copy q = floor(z0 / dz); they map to wrapped cells [zw, zw + len) when that
-          // stays below dz, else to [zw, dz), then [0, rest) of the next copy, or [0, dz) and
-          // [0, rest - dz) of the two next when the stencil is longer than the box.  The shift of
-          // a cell is d * (wrapped - unwrapped) = -d dz q, -d dz (q + 1), -d dz (q + 2).
-          const int base = dz * (w1 + dy * w0);
-          const int z0 = c2 + elo, len = ehi - elo + 1;
-          const int zw = wrap_cell(z0, dz);
-          const int q = zw == z0 ? 0 : (z0 - zw) / dz;
-          sa0 = __ldg(&s.cell_start[base + zw]);
-          oz0 = (R)(-d2c * (double)dz * (double)q);
-          if (zw + len <= dz) {
-            n0c = __ldg(&s.cell_start[base + zw + len]) - sa0;
-            nseg = 1;
-          } else {
-            n0c = __ldg(&s.cell_start[base + dz]) - sa0;
-            const int rest = zw + len - dz;
-            sa1 = __ldg(&s.cell_start[base]);
-            oz1 = (R)(-d2c * (double)dz * (double)(q + 1));
-            if (rest <= dz) {
-              n1c = __ldg(&s.cell_start[base + rest]) - sa1;
-              nseg = 2;
-            } else {
-              n1c = __ldg(&s.cell_start[base + dz]) - sa1;
-              sa2 = sa1;
-              n2c = __ldg(&s.cell_start[base + rest - dz]) - sa2;
-              oz2 = (R)(-d2c * (double)dz * (double)(q + 2));
-              nseg = 3;
-            }
-          }
-          cnt = n0c + n1c + n2c;
-        }
-      }
-    }
+    LeanRow w{};
+    int cnt = 0;
+    if (lane < group && r < nrows) cnt = lean_row(s, home, r / side - nc, r % side - nc, w);
+    const int nseg = cnt == 0 ? 0 : (w.n2 ? 3 : (w.n1 ? 2 : 1));
+    const R oxv = (R)(d0 * (double)w.sx), oyv = (R)(d1 * (double)w.sy);
     const int seg_incl = warp_incl_scan(nseg, lane);
     const int cnt_incl = warp_incl_scan(cnt, lane);
     const int nsegs = __shfl_sync(FULL, seg_incl, 31);
@@ -910,28 +929,28 @@ __device__ __forceinline__ void lean_atom(const SysDev& s, int sidx, int lane, L
     {
       int slot = seg_incl - nseg, beg = cnt_incl - cnt;
       if (nseg >= 1) {
-        sh.sa[slot] = sa0;
+        sh.sa[slot] = w.a0;
         sh.sb[slot] = beg;
-        sh.se[slot] = beg + n0c;
+        sh.se[slot] = beg + w.n0;
         sh.so[0][slot] = oxv;
         sh.so[1][slot] = oyv;
-        sh.so[2][slot] = oz0;
+        sh.so[2][slot] = (R)(d2c * (double)w.sz0);
       }
       if (nseg >= 2) {
-        sh.sa[slot + 1] = sa1;
-        sh.sb[slot + 1] = beg + n0c;
-        sh.se[slot + 1] = beg + n0c + n1c;
+        sh.sa[slot + 1] = w.a1;
+        sh.sb[slot + 1] = beg + w.n0;
+        sh.se[slot + 1] = beg + w.n0 + w.n1;
         sh.so[0][slot + 1] = oxv;
         sh.so[1][slot + 1] = oyv;
-        sh.so[2][slot + 1] = oz1;
+        sh.so[2][slot + 1] = (R)(d2c * (double)w.sz1);
       }
       if (nseg == 3) {
-        sh.sa[slot + 2] = sa2;
-        sh.sb[slot + 2] = beg + n0c + n1c;
-        sh.se[slot + 2] = beg + n0c + n1c + n2c;
+        sh.sa[slot + 2] = w.a2;
+        sh.sb[slot + 2] = beg + w.n0 + w.n1;
+        sh.se[slot + 2] = beg + w.n0 + w.n1 + w.n2;
         sh.so[0][slot + 2] = oxv;
         sh.so[1][slot + 2] = oyv;
-        sh.so[2][slot + 2] = oz2;
+        sh.so[2][slot + 2] = (R)(d2c * (double)w.sz2);
       }
     }
     __syncwarp();
@@ -2029,20 +2048,27 @@ __device__ inline int col_first_skip(const SysDev& s, int i, int pice) {
 }
 
 // The stray atoms, before the column kernel: a block looks 256 atoms over (in cell order), lists its
-// strays, and its warps walk them, one each, by the lean traversal (rows as contiguous ranges, cells
-// beyond rc left out), writing their forces where the column kernel reads them back for the RBL mean.
-// Bound by the latency of a walk's dependent loads, so what counts is that no warp has several strays
-// to walk while others have none and that a walk is short: a warp per column of cells, cell after
-// cell over all (2 nc + 1)^3 of them, took 167 us per step of a 9000-atom water box and 324 us of a
-// 64,000-atom one.
+// strays and walks them one after the other, its eight warps sharing a stray's traversal rows: first
+// counting every row's shells, then, with the counts of the rows before known, picking and evaluating.
+// Their forces are written where the column kernel reads them back for the RBL mean.  Strays are few
+// (one atom in a thousand), so the pass lasts as long as one walk: 45 us when a warp walked a stray by
+// itself, and 167 us (9000 atoms) to 324 us (64,000) when a warp per column of cells walked its strays cell
+// after cell.
+constexpr int kStrayRows = 512;  // rows counted at a time
+constexpr int kStrayQ = 64;      // a warp's queue of selected pairs
+
 template <int MODE, bool SPECIAL, bool NEAR>
 __global__ void __launch_bounds__(kAtomBlock, 3) k_pair_col_strays(const SysDev* __restrict__ S,
                                                                    const int2* __restrict__ work) {
-  __shared__ LeanShared<float> s_w[kAtomBlock / 32];
+  constexpr int kWarps = kAtomBlock / 32;
   __shared__ int s_list[kAtomBlock], s_n;
+  __shared__ int s_rank[kStrayRows];  // a row's shells, then the shells before it
+  __shared__ float4 s_q[kWarps][kStrayQ];  // displacement, sorted index (~ for a shell) as bits
+  __shared__ double s_f[kWarps][6];
   const int2 wk = work[blockIdx.x];
   const SysDev& s = S[wk.x];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const unsigned FULL = 0xffffffffu;
   if (threadIdx.x == 0) s_n = 0;
   __syncthreads();
   const int k = wk.y + threadIdx.x;
@@ -2052,17 +2078,118 @@ __global__ void __launch_bounds__(kAtomBlock, 3) k_pair_col_strays(const SysDev*
     if (col_is_stray(s, k, c / (dz * dy), (c / dz) % dy, c % dz)) s_list[atomicAdd(&s_n, 1)] = k;
   }
   __syncthreads();
-  for (int q = wid; q < s_n; q += kAtomBlock / 32) {
-    float ff[6];
-    PairAcc acc;
-    acc_zero(ff, acc);
-    int i;
-    lean_atom<float, MODE, SPECIAL, false, NEAR>(s, s_list[q], lane, s_w[wid], (const float*)s.ljf, i, ff, acc);
-    double cmb[6], r9[9];
-    acc_warp_total<true>(ff, acc, cmb);
-    acc_to_r9<MODE, true, false>(s, cmb, acc, r9);
-    if (lane == 0) finish_atom<MODE>(s, i, r9);
-    __syncwarp();
+  const int nc = s.nc, side = 2 * nc + 1, nrows = side * side, pice = s.pice;
+  for (int q = 0; q < s_n; ++q) {
+    const int si = s_list[q];
+    const int4 mi = __ldg(&s.smeta[si]);
+    const double4 xi = ldg4(&s.sx[si]);
+    const float4 pi = __ldg(&s.sxf[si]);
+    const LeanHome home = lean_home(s, xi, (int)((xi.x - s.lo[0]) / s.d[0]), (int)((xi.y - s.lo[1]) / s.d[1]),
+                                    (int)((xi.z - s.lo[2]) / s.d[2]));
+    const int first = col_first_skip(s, mi.x, pice);  // rank of the first pick
+    int nsp = 0;
+    const int* spi = nullptr;
+    const double* spw = nullptr;
+    if (SPECIAL) {
+      const int b = s.sp_off[mi.x];
+      nsp = s.sp_off[mi.x + 1] - b;
+      spi = s.sp_ids + b;
+      spw = s.sp_w + b;
+    }
+    float ff[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    int qn = 0;
+    auto flush = [&]() {
+      __syncwarp();
+      for (int t = lane; t < qn; t += 32) {
+        const float4 e = s_q[wid][t];
+        const int h = __float_as_int(e.w);
+        eval_pair_f32<MODE, SPECIAL, NEAR>(s, mi.z, (float)xi.w, h >= 0 ? h : ~h, h >= 0, e.x, e.y, e.z, mi.y, spi, spw,
+                                           nsp, (float)pice, (float)s.rc2, (float)s.rs2, s.fsa, (float)s.alpha,
+                                           (const float*)s.ljf, s.ntypes, (float)s.L[0], (float)s.L[1], (float)s.L[2],
+                                           ff[0], ff[1], ff[2], ff[3], ff[4], ff[5]);
+      }
+      __syncwarp();
+      qn = 0;
+    };
+    // this lane's candidate p of row w (of len): its class and displacement
+    auto classify = [&](const LeanRow& w, int len, int p, bool& core, bool& shell, int& js, float& rx, float& ry,
+                        float& rz) {
+      core = shell = false;
+      if (p >= len) return;
+      js = p < w.n0 ? w.a0 + p : (p < w.n0 + w.n1 ? w.a1 + (p - w.n0) : w.a2 + (p - w.n0 - w.n1));
+      const int sz = p < w.n0 ? w.sz0 : (p < w.n0 + w.n1 ? w.sz1 : w.sz2);
+      const float4 pj = __ldg(&s.sxf[js]);
+      rx = (pj.x - (float)(s.d[0] * (double)w.sx)) - pi.x;
+      ry = (pj.y - (float)(s.d[1] * (double)w.sy)) - pi.y;
+      rz = (pj.z - (float)(s.d[2] * (double)sz)) - pi.z;
+      const float dd = add_rn(add_rn(mul_rn(rx, rx), mul_rn(ry, ry)), mul_rn(rz, rz));
+      shell = (float)s.rc2 - dd > 0.0001f && dd - (float)s.rs2 > 0.0001f;
+      core = !shell && (float)s.rs2 - dd > 0.0001f && dd > 0.0001f;
+      if (f32_banded(s, dd)) classify_fp64(s, xi.x, xi.y, xi.z, js, w.sx, w.sy, sz, true, core, shell);
+    };
+    int before = 0;  // shells of the row groups before
+    for (int r0 = 0; r0 < nrows; r0 += kStrayRows) {
+      const int rn = min(kStrayRows, nrows - r0);
+      LeanRow w;
+      bool core, shell;
+      int js = 0;
+      float rx = 0.f, ry = 0.f, rz = 0.f;
+      __syncthreads();  // the ranks of the group (or stray) before are used
+      if (pice > 1)
+        for (int r = wid; r < rn; r += kWarps) {
+          const int len = lean_row(s, home, (r0 + r) / side - nc, (r0 + r) % side - nc, w);
+          int shells = 0;
+          for (int p0 = 0; p0 < len; p0 += 32) {
+            classify(w, len, p0 + lane, core, shell, js, rx, ry, rz);
+            shells += __popc(__ballot_sync(FULL, shell));
+          }
+          if (lane == 0) s_rank[r] = shells;
+        }
+      __syncthreads();
+      if (pice > 1 && wid == 0) {
+        int run = before;
+        for (int b = 0; b < rn; b += 32) {
+          const int v = b + lane < rn ? s_rank[b + lane] : 0;
+          const int incl = warp_incl_scan(v, lane);
+          if (b + lane < rn) s_rank[b + lane] = run + incl - v;
+          run += __shfl_sync(FULL, incl, 31);
+        }
+        before = run;  // only this warp's is read
+      }
+      __syncthreads();
+      for (int r = wid; r < rn; r += kWarps) {
+        const int len = lean_row(s, home, (r0 + r) / side - nc, (r0 + r) % side - nc, w);
+        int rank = pice > 1 ? s_rank[r] : 0;
+        for (int p0 = 0; p0 < len; p0 += 32) {
+          classify(w, len, p0 + lane, core, shell, js, rx, ry, rz);
+          bool pick = shell;
+          if (pice > 1) {
+            const unsigned sm = __ballot_sync(FULL, shell);
+            pick = shell && (rank + __popc(sm & lanemask_lt(lane))) % pice == first;
+            rank += __popc(sm);
+          }
+          const unsigned sel = __ballot_sync(FULL, core | pick);
+          if (qn + __popc(sel) > kStrayQ) flush();
+          if (core | pick)
+            s_q[wid][qn + __popc(sel & lanemask_lt(lane))] = make_float4(rx, ry, rz, __int_as_float(core ? js : ~js));
+          qn += __popc(sel);
+        }
+      }
+    }
+    flush();
+    for (int t = 0; t < 6; ++t) {
+      const double v = warp_sum((double)ff[t]);
+      if (lane == 0) s_f[wid][t] = v;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      double c[6] = {0, 0, 0, 0, 0, 0}, r9[9];
+      for (int w = 0; w < kWarps; ++w)
+        for (int t = 0; t < 6; ++t) c[t] += s_f[w][t];
+      PairAcc none;
+      acc_to_r9<MODE, true, false>(s, c, none, r9);
+      finish_atom<MODE>(s, mi.x, r9);
+    }
   }
 }
 
@@ -2099,12 +2226,13 @@ k_pair_col(const SysDev* __restrict__ S, const int2* __restrict__ work, int nwor
   static_assert(!NEAR || MODE == kCOUL_RBL, "the near-Coulomb table applies to the Coulomb mode");
   static_assert(kColQ % 32 == 0 && kColStage % 32 == 0, "the walk runs in blocks of 32 steps");
   constexpr int kWarps = SPLIT ? kColSplit : kColWarps;
+  using Mine = ColWarp<SPLIT>;
   const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  __shared__ __align__(16) unsigned char s_fixed[SPLIT ? 16 : kColWarps * sizeof(ColWarp<false>)];
+  __shared__ __align__(16) unsigned char s_fixed[SPLIT ? 16 : kColWarps * sizeof(Mine)];
   __shared__ int s_item;
-  extern __shared__ __align__(16) unsigned char s_dyn[];  // split form: kColSplit warps, then the rows
-  ColWarp<SPLIT>& sh = reinterpret_cast<ColWarp<SPLIT>*>(SPLIT ? s_dyn : s_fixed)[wid];
-  ColRow* const s_row = reinterpret_cast<ColRow*>(s_dyn + kColSplit * sizeof(ColWarp<true>));
+  extern __shared__ __align__(16) unsigned char s_dyn[];  // split form: the warps, then the rows
+  Mine& sh = reinterpret_cast<Mine*>(SPLIT ? s_dyn : s_fixed)[wid];
+  ColRow* const s_row = reinterpret_cast<ColRow*>(s_dyn + kWarps * sizeof(Mine));
 
   const unsigned FULL = 0xffffffffu;
   // FP32 band edges of the launch (the union of its systems' bands; a batch shares rc and rs)
@@ -2632,8 +2760,9 @@ void plan_pair_col(Batch& b, double chunks, double longest, int nc) {
   b.col_rows = side * side;
   b.col_parts = std::max(1, std::min(1024, (int)std::ceil(1.2 * longest / 32.0)));
   // Up to about one chunk per resident warp (148 SMs x 16) the split form's eight warps per chunk are
-  // faster: 177 -> 56 us (1200 atoms of saline), 245 -> 145 us (9000), 467 -> 449 us (64,000, 2140
+  // faster: 177 -> 56 us (1200 atoms of saline), 216 -> 118 us (9000), 456 -> 439 us (64,000, 2140
   // chunks); above, its second staging costs more than it spreads (3420 -> 5460 us for 985,000 atoms).
+  // Four warps per chunk were no better anywhere (78, 117 and 469 us).
   b.col_split = b.col_rows <= kColMaxRows && chunks < 2200;
   int dev = 0, sms = 0, per_sm = 0;
   cudaGetDevice(&dev);
