@@ -198,7 +198,7 @@ def kernel_profile(ctx, ids, systems):
     ctx.step(ids, 2)
     ctx.sync()
     out = {}
-    for name in ("nhc", "kick_drift", "cells", "shake", "rbe_sample", "rho", "far", "bonded", "pair_col", "pair_tile",
+    for name in ("nhc", "kick_drift", "cells", "shake", "rbe_sample", "rho", "far", "bonded", "intra", "pair_col", "pair_tile",
                  "pair_lean", "pair_atom", "final", "rattle"):
         ms, n, units = ctx.profile_get(name)
         if n:

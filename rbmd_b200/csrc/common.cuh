@@ -145,8 +145,8 @@ struct SysDev {
   double4* x;          // x, y, z, charge
   double4* v;          // vx, vy, vz, mass
   double4* f;          // force
-  double4* ffar;       // far force (RBE, Ewald)
-  double* far_vir;     // [6 per kFarAtoms atoms] its virial partials
+  double4* ffar;       // far force (RBE, Ewald) and intramolecular terms
+  double* far_vir;     // [6 per kFarAtoms atoms] the far force's virial partials, then [6 blocks_atom] the exclusion's
   double4* xold;       // pre-drift positions (SHAKE)
   double4* vold;       // pre-kick velocities (SHAKE first half)
   double4* vold2;      // pre-kick velocities (RATTLE)
@@ -215,7 +215,7 @@ struct SysDev {
   double* eam_fp;      // [n] in cell order
   // reductions
   double* pair_part;   // [blocks_pair * 4]
-  double* atom_part;   // [blocks_atom * 8]
+  double* atom_part;   // [blocks_atom]
   double* vir_part;    // [blocks_pair * 9] pair-kernel partials
   double* tri_part;    // [blocks_tri * 6] SHAKE virial partials
   SysState* st;

@@ -273,7 +273,7 @@ int64_t Context::estimate_bytes(const rbmd_system_desc& d, const rbmd_params& p)
                           ? (int64_t)(2 * p.kmax[0] + 1) * (2 * p.kmax[1] + 1) * (2 * p.kmax[2] + 1)
                           : 0;
   const int64_t brho = (n + rho_chunk((int)n) - 1) / rho_chunk((int)n);
-  if (p.coulomb != RBMD_COUL_NONE) b += n * 32 + (n + kFarAtoms - 1) / kFarAtoms * 48;  // far forces and virial
+  if (p.coulomb != RBMD_COUL_NONE) b += n * 32 + (n + kFarAtoms - 1) / kFarAtoms * 60;  // far forces and virial
   b += nk * 48 + nke * 48 + brho * 16 * std::max(nk, nke);
   b += (int64_t)(d.n_bonds * 2 + d.n_angles * 3 + d.n_dihedrals * 4) * 48 +
        (int64_t)(d.n_bonds + d.n_angles + d.n_dihedrals) * 76;
@@ -762,7 +762,7 @@ int Context::add_system(const rbmd_system_desc& d, const rbmd_params& p, int32_t
   }
   if (D.coul != RBMD_COUL_NONE) {
     D.ffar = (double4*)dal(sizeof(double4) * n);
-    D.far_vir = (double*)dal(sizeof(double) * 6 * ((n + kFarAtoms - 1) / kFarAtoms));
+    D.far_vir = (double*)dal(sizeof(double) * 6 * ((n + kFarAtoms - 1) / kFarAtoms + D.blocks_atom));
     D.km = (int*)dal(sizeof(int) * 3 * std::max(1, D.P));
     D.kv = (double4*)dal(sizeof(double4) * std::max(1, nk_force));
     D.rhok = (double*)dal(sizeof(double) * 2 * std::max(1, nk_force));
@@ -806,7 +806,7 @@ int Context::add_system(const rbmd_system_desc& d, const rbmd_params& p, int32_t
     up(D.rhor_s, hrhor.data(), sizeof(double) * hrhor.size());
     up(D.z2r_s, hz2r.data(), sizeof(double) * hz2r.size());
   }
-  D.atom_part = (double*)dal(sizeof(double) * 8 * D.blocks_atom);
+  D.atom_part = (double*)dal(sizeof(double) * D.blocks_atom);
   // pair-kernel partials: enough for any layout the autotuner may switch to (nine per block; the column
   // kernel three per 32-atom chunk, at most n / 32 + one per column of them)
   const size_t part_blocks =
@@ -1123,6 +1123,7 @@ void Context::enqueue_assembly(const Batch& b, FinalMode mode, int virial) {
       timed("far", (double)b.natoms, [&] { launch_far(b, side, virial); });
     }
     if (b.has_bonded) timed("bonded", 0, [&] { launch_bonded(b, side, virial); });
+    timed("intra", (double)b.natoms, [&] { launch_intra(b, side, virial); });
   }
   timed(pair_name(b), (double)b.natoms, [&] { launch_pair(b, stream, virial); });
   join_side(side);

@@ -375,40 +375,20 @@ __global__ void __launch_bounds__(kAtomBlock, 4) k_far(const SysDev* __restrict_
   }
 }
 
-// Force assembly, half kick, kinetic energy and, in the system's last block, the thermostat.  Bound by
-// memory (240 B per atom and the gathers of the bonded terms).
+// Intramolecular Coulomb exclusion and bonded terms of every atom, added to its far force.  Chains of
+// dependent gathers (molecule, partner, special list, term slots, term forces) of 10 us that need only
+// positions: beside the pair kernel they cost nothing, in the force assembly they were the wait of it
+// (17 us for 9000 atoms of water against 8 us without them).
 template <bool VIRIAL>
-__global__ void __launch_bounds__(kAtomBlock, 4)
-k_final(const SysDev* __restrict__ S, const int2* __restrict__ work, int mode) {
+__global__ void __launch_bounds__(kAtomBlock) k_intra(const SysDev* __restrict__ S, const int2* __restrict__ work) {
   const int2 wk = work[blockIdx.x];
   const SysDev& s = S[wk.x];
   const int i = wk.y + threadIdx.x;
-  const bool act = i < s.n;
-  SysState* st = s.st;
-  __shared__ double s_part[kAtomBlock / 32][8];
-
-  double4 xi = act ? s.x[i] : make_double4(0, 0, 0, 0);
-  double F[3] = {0, 0, 0};
-  if (act) {
-    const double4 fn = s.f[i];
-    F[0] = fn.x;
-    F[1] = fn.y;
-    F[2] = fn.z;
-  }
-  if (s.neigh == RBMD_NEIGH_RBL) {
-    // SumRBLCorrForce: near_i - mean(near), ExecutionMD.cpp:663-667, 820-826, 1097-1099
-    F[0] -= st->fmean[0];
-    F[1] -= st->fmean[1];
-    F[2] -= st->fmean[2];
-  }
   double vir[6] = {0, 0, 0, 0, 0, 0};
-  if (act && s.coul != RBMD_COUL_NONE) {  // far force (k_far)
+  if (i < s.n) {
+    const double4 xi = s.x[i];
     const double4 ff = s.ffar[i];
-    F[0] = ff.x + F[0];
-    F[1] = ff.y + F[1];
-    F[2] = ff.z + F[2];
-  }
-  if (act) {
+    double F[3] = {ff.x, ff.y, ff.z};
     // ---- intramolecular Coulomb exclusion (CVFF + RBL + special bonds)
     if (s.ff == RBMD_FF_CVFF && s.neigh == RBMD_NEIGH_RBL && s.special) {
       const int4 mi = s.meta[i];
@@ -446,6 +426,50 @@ k_final(const SysDev* __restrict__ S, const int2* __restrict__ work, int mode) {
         F[2] += tf.z;
       }
     }
+    s.ffar[i] = make_double4(F[0], F[1], F[2], 0.0);
+  }
+  if (VIRIAL) {
+    __shared__ double s_w[kAtomBlock / 32];
+    double* out = s.far_vir + 6 * ((size_t)((s.n + kFarAtoms - 1) / kFarAtoms) + wk.y / kAtomBlock);
+    for (int k = 0; k < 6; ++k) {
+      const double t = block_sum(vir[k], s_w);
+      if (threadIdx.x == 0) out[k] = t;
+    }
+  }
+}
+
+// Force assembly, half kick, kinetic energy and, in the system's last block, the thermostat.  Bound by
+// memory (200 B per atom).
+template <bool VIRIAL>
+__global__ void __launch_bounds__(kAtomBlock, 4)
+k_final(const SysDev* __restrict__ S, const int2* __restrict__ work, int mode) {
+  const int2 wk = work[blockIdx.x];
+  const SysDev& s = S[wk.x];
+  const int i = wk.y + threadIdx.x;
+  const bool act = i < s.n;
+  SysState* st = s.st;
+  __shared__ double s_w[kAtomBlock / 32];
+
+  double F[3] = {0, 0, 0};
+  if (act) {
+    const double4 fn = s.f[i];
+    F[0] = fn.x;
+    F[1] = fn.y;
+    F[2] = fn.z;
+  }
+  if (s.neigh == RBMD_NEIGH_RBL) {
+    // SumRBLCorrForce: near_i - mean(near), ExecutionMD.cpp:663-667, 820-826, 1097-1099
+    F[0] -= st->fmean[0];
+    F[1] -= st->fmean[1];
+    F[2] -= st->fmean[2];
+  }
+  if (act && s.coul != RBMD_COUL_NONE) {  // far force, intramolecular terms (k_far, k_intra)
+    const double4 ff = s.ffar[i];
+    F[0] = ff.x + F[0];
+    F[1] = ff.y + F[1];
+    F[2] = ff.z + F[2];
+  }
+  if (act) {
     s.f[i] = make_double4(F[0], F[1], F[2], 0.0);
     if (!(isfinite(F[0]) && isfinite(F[1]) && isfinite(F[2]))) atomicOr(&st->status, kErrNonFinite);
   }
@@ -471,32 +495,22 @@ k_final(const SysDev* __restrict__ S, const int2* __restrict__ work, int mode) {
   }
   // ---- block partials and the system epilogue
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  double r8[8];
-  r8[0] = warp_sum(ke);
-#pragma unroll
-  for (int k = 0; k < 6; ++k) r8[1 + k] = VIRIAL ? warp_sum(vir[k]) : 0.0;
-  r8[7] = 0.0;
-  if (lane == 0)
-    for (int k = 0; k < 8; ++k) s_part[wid][k] = r8[k];
+  ke = warp_sum(ke);
+  if (lane == 0) s_w[wid] = ke;
   __syncthreads();
-  const int blk = wk.y / kAtomBlock;
-  if (threadIdx.x < 8) {
+  if (threadIdx.x == 0) {
     double t = 0.0;
-    for (int w = 0; w < kAtomBlock / 32; ++w) t += s_part[w][threadIdx.x];
-    s.atom_part[(size_t)blk * 8 + threadIdx.x] = t;
+    for (int w = 0; w < kAtomBlock / 32; ++w) t += s_w[w];
+    s.atom_part[wk.y / kAtomBlock] = t;
   }
   if (arrive_last(&st->counter[2], (unsigned)s.blocks_atom)) {
-    double* s_w = &s_part[0][0];  // block_sum's scratch
-    double s_tot[7] = {0, 0, 0, 0, 0, 0, 0}, tv[6] = {0, 0, 0, 0, 0, 0};
-    const int nsum = VIRIAL ? 7 : 1;
-    for (int k = 0; k < nsum; ++k) {
-      double t = 0.0;
-      for (int b = threadIdx.x; b < s.blocks_atom; b += kAtomBlock) t += __ldcg(&s.atom_part[(size_t)b * 8 + k]);
-      s_tot[k] = block_sum(t, s_w);
-    }
-    if (VIRIAL) {  // the bonded terms' virial and the far force's
+    double tv[6] = {0, 0, 0, 0, 0, 0}, ke_sum = 0.0;
+    for (int b = threadIdx.x; b < s.blocks_atom; b += kAtomBlock) ke_sum += __ldcg(&s.atom_part[b]);
+    ke_sum = block_sum(ke_sum, s_w);
+    if (VIRIAL) {  // of the bonded terms, the far force and the exclusion
       const int nt = s.term_vir ? s.n_bonds + s.n_angles + s.n_dihedrals : 0;
-      const int nf = s.coul != RBMD_COUL_NONE ? (s.n + kFarAtoms - 1) / kFarAtoms : 0;
+      int nf = s.coul != RBMD_COUL_NONE ? (s.n + kFarAtoms - 1) / kFarAtoms : 0;
+      if (s.ff == RBMD_FF_CVFF) nf += s.blocks_atom;
       for (int t = threadIdx.x; t < nt; t += kAtomBlock)
         for (int k = 0; k < 6; ++k) tv[k] += s.term_vir[6 * (size_t)t + k];
       for (int t = threadIdx.x; t < nf; t += kAtomBlock)
@@ -505,11 +519,11 @@ k_final(const SysDev* __restrict__ S, const int2* __restrict__ work, int mode) {
     }
     if (threadIdx.x == 0) {
       if (VIRIAL) {
-        for (int k = 0; k < 6; ++k) st->virial[k] = st->virial[k] + s_tot[1 + k] + tv[k];
+        for (int k = 0; k < 6; ++k) st->virial[k] = st->virial[k] + tv[k];
       }
       if (mode == kFinalInit) {
         // ExecutionNVT::InitialCondition + SetUp (ExecutionNVT.cpp:139-187, 1106-1122)
-        compute_tempe(s, st, s_tot[0]);
+        compute_tempe(s, st, ke_sum);
         compute_temp_target(s, st);
         const double tf = st->t_freq;
         st->eta_mass[0] = st->tdof * s.boltz * st->t_target / (tf * tf);
@@ -521,7 +535,7 @@ k_final(const SysDev* __restrict__ S, const int2* __restrict__ work, int mode) {
       } else if (mode == kFinalKick) {
         const bool shk_thermo = s.has_triples && s.temp_ctrl != RBMD_TC_NOSE_HOOVER;
         if (!shk_thermo) {
-          compute_tempe(s, st, s_tot[0]);
+          compute_tempe(s, st, ke_sum);
           if (s.temp_ctrl == RBMD_TC_NOSE_HOOVER) {
             if (s.npt == 2) {
               // FinalIntegrate: pressure of this step's forces, barostat velocity half step
@@ -569,11 +583,11 @@ __global__ void __launch_bounds__(kAtomBlock) k_ke_thermostat(const SysDev* __re
   if (threadIdx.x == 0) {
     double t = 0.0;
     for (int k = 0; k < kAtomBlock / 32; ++k) t += s_w[k];
-    s.atom_part[(size_t)blk * 8] = t;
+    s.atom_part[blk] = t;
   }
   if (arrive_last(&st->counter[5], (unsigned)s.blocks_atom)) {
     double t = 0.0;
-    for (int b = threadIdx.x; b < s.blocks_atom; b += kAtomBlock) t += __ldcg(&s.atom_part[(size_t)b * 8]);
+    for (int b = threadIdx.x; b < s.blocks_atom; b += kAtomBlock) t += __ldcg(&s.atom_part[b]);
     t = block_sum(t, s_w);
     if (threadIdx.x == 0) {
       compute_tempe(s, st, t);
@@ -916,6 +930,13 @@ void launch_far(const Batch& b, cudaStream_t st, int virial) {
   if (virial) k_far<false, true><<<grid, kAtomBlock, 0, st>>>(b.sys, b.atom.d);
   else if (b.prec == RBMD_PREC_MIXED && b.coul == RBMD_COUL_RBE) k_far<true, false><<<grid, kAtomBlock, 0, st>>>(b.sys, b.atom.d);
   else k_far<false, false><<<grid, kAtomBlock, 0, st>>>(b.sys, b.atom.d);
+  note_launch();
+}
+
+void launch_intra(const Batch& b, cudaStream_t st, int virial) {
+  if (b.ff != RBMD_FF_CVFF) return;
+  if (virial) k_intra<true><<<b.atom.n, kAtomBlock, 0, st>>>(b.sys, b.atom.d);
+  else k_intra<false><<<b.atom.n, kAtomBlock, 0, st>>>(b.sys, b.atom.d);
   note_launch();
 }
 

@@ -60,6 +60,8 @@ void launch_pair(const Batch& b, cudaStream_t s, int virial);
 void plan_pair_col(Batch& b, double chunks, double longest, int nc);
 // Far forces (RBE, Ewald) from the structure factor, for launch_final to add.
 void launch_far(const Batch& b, cudaStream_t s, int virial);
+// Intramolecular terms (CVFF) added to the far forces, after launch_far and launch_bonded.
+void launch_intra(const Batch& b, cudaStream_t s, int virial);
 void launch_final(const Batch& b, cudaStream_t s, FinalMode mode, int virial);
 void launch_ke_thermostat(const Batch& b, cudaStream_t s);
 void launch_flush_vscale(const Batch& b, cudaStream_t s);
