@@ -2005,7 +2005,6 @@ k_pair_tile(const SysDev* __restrict__ S, const int2* __restrict__ work, int cap
 // tail is short columns.  The RBL mean force is summed per column and the system's last column
 // adds the partials in column order: the result does not depend on which warp took which column.
 constexpr int kColWarps = 4;     // warps per block, a chunk each
-constexpr int kColSplit = 8;     // warps per block of the split form, one chunk between them
 constexpr int kColStage = 256;   // staged candidates per warp
 constexpr int kColQ = kColStage;  // the most steps between evaluations: a staged tile
 constexpr int kColQW = kColQ / 32;  // 32-step blocks between evaluations
@@ -2216,16 +2215,20 @@ struct ColRow {
   int shells[32];
   float3 f[32];
 };
-constexpr size_t col_smem(int nrows) { return kColSplit * sizeof(ColWarp<true>) + (size_t)nrows * sizeof(ColRow); }
+constexpr size_t col_smem(int split, int nrows) {
+  return split == 1 ? 0 : split * sizeof(ColWarp<true>) + (size_t)nrows * sizeof(ColRow);
+}
 
-template <int MODE, bool SPECIAL, bool NEAR, bool SPLIT>
-__global__ void __launch_bounds__(SPLIT ? kColSplit * 32 : kColWarps * 32, SPLIT ? 2 : RBMD_COL_MIN_BLOCKS)
+// WARPS: warps that share a chunk (1: a block of kColWarps warps with a chunk each).
+template <int MODE, bool SPECIAL, bool NEAR, int WARPS>
+__global__ void __launch_bounds__(WARPS > 1 ? WARPS * 32 : kColWarps * 32, WARPS > 1 ? 16 / WARPS : RBMD_COL_MIN_BLOCKS)
 k_pair_col(const SysDev* __restrict__ S, const int2* __restrict__ work, int nwork, int nparts,
            unsigned* __restrict__ ctr, float4 band) {
   static_assert(MODE == kLJ_RBL || MODE == kCOUL_RBL, "column layout: FP32 RBL forces only");
   static_assert(!NEAR || MODE == kCOUL_RBL, "the near-Coulomb table applies to the Coulomb mode");
   static_assert(kColQ % 32 == 0 && kColStage % 32 == 0, "the walk runs in blocks of 32 steps");
-  constexpr int kWarps = SPLIT ? kColSplit : kColWarps;
+  constexpr bool SPLIT = WARPS > 1;
+  constexpr int kWarps = SPLIT ? WARPS : kColWarps;
   using Mine = ColWarp<SPLIT>;
   const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
   __shared__ __align__(16) unsigned char s_fixed[SPLIT ? 16 : kColWarps * sizeof(Mine)];
@@ -2712,12 +2715,13 @@ static void go_near(const Batch& b, cudaStream_t st) {
       if (b.pair.n > 0) {
         k_pair_col_strays<MODE, SPECIAL, NEAR><<<b.atom.n, kAtomBlock, 0, st>>>(b.sys, b.atom.d);
         note_launch();
-        if (b.col_split)
-          k_pair_col<MODE, SPECIAL, NEAR, true><<<b.col_grid, kColSplit * 32, col_smem(b.col_rows), st>>>(
-              b.sys, b.pair.d, b.pair.n, b.col_parts, b.col_ctr, band);
-        else
-          k_pair_col<MODE, SPECIAL, NEAR, false><<<b.col_grid, kColWarps * 32, 0, st>>>(
-              b.sys, b.pair.d, b.pair.n, b.col_parts, b.col_ctr, band);
+        auto col = [&](auto kernel, int warps) {
+          kernel<<<b.col_grid, warps * 32, col_smem(b.col_split, b.col_rows), st>>>(b.sys, b.pair.d, b.pair.n, b.col_parts,
+                                                                                   b.col_ctr, band);
+        };
+        if (b.col_split == 16) col(k_pair_col<MODE, SPECIAL, NEAR, 16>, 16);
+        else if (b.col_split == 8) col(k_pair_col<MODE, SPECIAL, NEAR, 8>, 8);
+        else col(k_pair_col<MODE, SPECIAL, NEAR, 1>, kColWarps);
         note_launch();
       }
       return;
@@ -2745,14 +2749,14 @@ static void go(const Batch& b, cudaStream_t st) {
   go_near<R, MODE, SPECIAL, VIRIAL, false>(b, st);
 }
 
-template <bool SPLIT>
+template <int WARPS>
 static const void* col_kernel(const Batch& b) {
-  if (b.ff == RBMD_FF_LJ_CUT) return (const void*)k_pair_col<kLJ_RBL, false, false, SPLIT>;
+  if (b.ff == RBMD_FF_LJ_CUT) return (const void*)k_pair_col<kLJ_RBL, false, false, WARPS>;
   if (b.special)
-    return b.near ? (const void*)k_pair_col<kCOUL_RBL, true, true, SPLIT>
-                  : (const void*)k_pair_col<kCOUL_RBL, true, false, SPLIT>;
-  return b.near ? (const void*)k_pair_col<kCOUL_RBL, false, true, SPLIT>
-                : (const void*)k_pair_col<kCOUL_RBL, false, false, SPLIT>;
+    return b.near ? (const void*)k_pair_col<kCOUL_RBL, true, true, WARPS>
+                  : (const void*)k_pair_col<kCOUL_RBL, true, false, WARPS>;
+  return b.near ? (const void*)k_pair_col<kCOUL_RBL, false, true, WARPS>
+                : (const void*)k_pair_col<kCOUL_RBL, false, false, WARPS>;
 }
 
 void plan_pair_col(Batch& b, double chunks, double longest, int nc) {
@@ -2762,18 +2766,19 @@ void plan_pair_col(Batch& b, double chunks, double longest, int nc) {
   // Up to about one chunk per resident warp (148 SMs x 16) the split form's eight warps per chunk are
   // faster: 177 -> 56 us (1200 atoms of saline), 216 -> 118 us (9000), 456 -> 439 us (64,000, 2140
   // chunks); above, its second staging costs more than it spreads (3420 -> 5460 us for 985,000 atoms).
-  // Four warps per chunk were no better anywhere (78, 117 and 469 us).
-  b.col_split = b.col_rows <= kColMaxRows && chunks < 2200;
+  // Four warps per chunk were no better anywhere (78, 117 and 469 us).  Sixteen, a block to an SM, while
+  // there are SMs for the chunks: 50 -> 41 us for 1200 atoms; beyond, eight (414 against 530 us at 64,000).
+  b.col_split = b.col_rows > kColMaxRows || chunks >= 2200 ? 1 : (chunks <= 148 && b.col_rows <= 32 ? 16 : 8);
   int dev = 0, sms = 0, per_sm = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const void* fn = b.col_split ? col_kernel<true>(b) : col_kernel<false>(b);
-  const size_t smem = b.col_split ? col_smem(b.col_rows) : 0;
-  const int warps = b.col_split ? kColSplit : kColWarps;
-  if (b.col_split) cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const void* fn = b.col_split == 16 ? col_kernel<16>(b) : (b.col_split == 8 ? col_kernel<8>(b) : col_kernel<1>(b));
+  const size_t smem = col_smem(b.col_split, b.col_rows);
+  const int warps = b.col_split > 1 ? b.col_split : kColWarps;  // per block
+  if (smem) cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, warps * 32, smem);
   const long long items = (long long)b.pair.n * b.col_parts;
-  const long long need = b.col_split ? items : (items + kColWarps - 1) / kColWarps;
+  const long long need = b.col_split > 1 ? items : (items + kColWarps - 1) / kColWarps;
   b.col_grid = (int)std::max(1LL, std::min(need, (long long)std::max(1, sms) * std::max(1, per_sm)));
 }
 

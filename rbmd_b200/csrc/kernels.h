@@ -23,9 +23,9 @@ struct Batch {
   // column layout: pair.d lists every column (slot, column index), most atoms per column first;
   // the persistent column kernel takes them in that order from col_ctr[0] (col_ctr[1] counts the warps
   // that are done; the last one resets both), every column in col_parts items, col_grid blocks;
-  // col_split: eight warps share a chunk of 32 atoms, by its col_rows traversal rows
+  // col_split: warps that share a chunk of 32 atoms, by its col_rows traversal rows (1: none do)
   unsigned* col_ctr = nullptr;
-  int col_grid = 0, col_parts = 1, col_split = 0, col_rows = 0;
+  int col_grid = 0, col_parts = 1, col_split = 1, col_rows = 0;
   // uniform switches of the batch (a batch never mixes them)
   int ff = 0, neigh = 0, coul = 0, prec = 0, temp_ctrl = 0, special = 0;
   int has_shake = 0, has_bonded = 0;
