@@ -639,15 +639,27 @@ int Context::add_system(const rbmd_system_desc& d, const rbmd_params& p, int32_t
   // ---- device allocations
   int64_t total = 0;
   bool oom = false;
+  // one allocation of about the estimated footprint, cut up; what does not fit in it is allocated by itself
+  size_t slab_left = (size_t)estimate_bytes(d, p) + 48 * 256;
+  char* slab = (char*)dmalloc(slab_left);
+  if (slab) s->allocs.push_back(slab);
+  else slab_left = 0;
   auto dal = [&](size_t bytes) -> void* {
     if (bytes == 0) bytes = 16;
+    const size_t rounded = (bytes + 255) & ~(size_t)255;
+    total += (int64_t)bytes;
+    if (rounded <= slab_left) {
+      void* ptr = slab;
+      slab += rounded;
+      slab_left -= rounded;
+      return ptr;
+    }
     void* ptr = dmalloc(bytes);
     if (!ptr) {
       oom = true;
       return nullptr;
     }
     s->allocs.push_back(ptr);
-    total += (int64_t)bytes;
     return ptr;
   };
   auto up = [&](void* dst, const void* src, size_t bytes) {
