@@ -8,12 +8,13 @@
 //   ComputeEAMfp_Worklet / ComputeEAMRBLWorklet  RunWorklet.cpp:1651-1815             (EAM passes)
 //   LJ / Coulomb / EAM energy worklets           RunWorklet.cpp:2987-3221, ThermoOutput.cpp:293-356
 //
-// Three traversals share the selection rule and the pair arithmetic:
+// Four traversals share the selection rule and the pair arithmetic:
 //   k_pair       one warp per atom, any box (cells may repeat in the stencil of a small box);
 //   k_pair2      one warp per atom with per-atom segment tables (every dimension holds 2 nc + 1
 //                cells), cells beyond rc of the atom culled;
-//   k_pair_tile  one warp per home cell: the cell's atoms share each batch of 32 candidates, the
-//                default for mixed precision once cells hold a few atoms.
+//   k_pair_tile  one warp per home cell: the cell's atoms share each batch of 32 candidates;
+//   k_pair_col   one lane per atom of a column of home cells, the default for mixed-precision RBL
+//                forces once cells hold a few atoms.
 // All visit the (2 nc + 1)^3 neighbour cells in the reference order (x offset outermost, z
 // innermost, ascending atom id inside a cell).  The shell rank of every candidate is its position
 // among the shells of that order, which reproduces the reference's sequential "every pice-th shell
@@ -1978,9 +1979,9 @@ k_pair_tile(const SysDev* __restrict__ S, const int2* __restrict__ work, int cap
 }
 
 // ------------------------------------------------------------------------------------------------
-// Column variant (mixed-precision RBL forces: LJ/CUT and LJ + real-space Coulomb).  One warp per
-// column of home cells -- fixed x and y cell, all z -- whose atoms are contiguous in the cell-ordered
-// arrays (cells are numbered z fastest), taken 32 at a time: one lane per home atom.  The chunk's
+// Column variant (mixed-precision RBL forces: LJ/CUT and LJ + real-space Coulomb).  A column of home
+// cells -- fixed x and y cell, all z -- has its atoms contiguous in the cell-ordered arrays (cells are
+// numbered z fastest); a warp takes a chunk of 32 of them, one lane per home atom.  The chunk's
 // atoms sit in a few consecutive z cells, so for a traversal row (x and y cell offset) their
 // candidate windows -- the row's z cells from the atom's own cell - nc to + nc -- are overlapping
 // sub-ranges of one contiguous union, which the warp stages once in shared memory, shifted into
@@ -1996,14 +1997,16 @@ k_pair_tile(const SysDev* __restrict__ S, const int2* __restrict__ work, int cap
 // exactly those of the full traversal.  The selected candidates of up to kColQ steps are evaluated
 // by their own lane from the masks, in traversal order, so an atom's force is summed in a fixed
 // order by one lane.  An atom outside its binned cell (SHAKE moves atoms after binning, and atoms
-// may lie outside the box) walks its own neighbourhood with the whole warp (tile_stray, as in the
-// tile kernel), in a pass of its own before the column kernel (k_pair_col_strays): its force is
-// written there, and the column kernel only reads it back for the RBL mean, so that the stray
-// walk's code does not share the instruction cache with the walk and the evaluation.
-// The kernel is persistent: one grid of resident blocks, each warp taking the batch's columns one at
-// a time from a work counter, longest columns first, so no warp waits for another and the launch's
-// tail is short columns.  The RBL mean force is summed per column and the system's last column
-// adds the partials in column order: the result does not depend on which warp took which column.
+// may lie outside the box) is walked in a pass of its own before the column kernel
+// (k_pair_col_strays): its force is written there, and the column kernel only reads it back for the
+// RBL mean, so that the stray walk's code does not share the instruction cache with the walk and the
+// evaluation.
+// The kernel is persistent: one grid of resident blocks, each warp taking the batch's items (every
+// nparts-th chunk of a column) one at a time from a work counter, longest columns first, so no warp
+// waits for another.  In the split form (few chunks) a block's warps share a chunk by its traversal
+// rows.  A row's force is summed by itself and the rows are added in order, the RBL mean is summed per
+// chunk and the system's last item adds the partials in column order: the result does not depend on
+// the form, nor on which warp took which item.
 constexpr int kColWarps = 4;     // warps per block, a chunk each
 constexpr int kColStage = 256;   // staged candidates per warp
 constexpr int kColQ = kColStage;  // the most steps between evaluations: a staged tile
