@@ -1019,8 +1019,15 @@ __device__ __forceinline__ void lean_atom(const SysDev& s, int sidx, int lane, L
   __syncwarp();
 }
 
-template <typename R, int MODE, bool SPECIAL, bool VIRIAL, bool NEAR = false>
-__global__ void __launch_bounds__(kPairWarps * 32, 3)
+// BLOCKS: resident blocks per SM it is compiled for.  Three (80 registers) keep more warps in flight; two
+// (126-128 registers) leave the FP64 kernels with special bonds without their 32-60 bytes of spill stores.
+// Three blocks -> two, us per launch: saline 1000 atoms 49.3 -> 41.4, 4000 98.6 -> 83.3, Ewald water 4500
+// 138.6 -> 117.0, but Ewald water 15,000 295.6 -> 321.4, saline 16,000 244.0 -> 257.4 and 64,000 838 -> 922.
+// The line is set between 4500 and 15,000 atoms; where exactly the two cross was not measured.
+constexpr long long kLeanFewAtoms = 8192;
+
+template <typename R, int MODE, bool SPECIAL, bool VIRIAL, bool NEAR, int BLOCKS>
+__global__ void __launch_bounds__(kPairWarps * 32, BLOCKS)
 k_pair2(const SysDev* __restrict__ S, const int2* __restrict__ work) {
   constexpr bool F32 = sizeof(R) == 4 && (MODE == kLJ_RBL || MODE == kCOUL_RBL);
   __shared__ LeanShared<R> s_w[kPairWarps];
@@ -2733,9 +2740,13 @@ static void go_near(const Batch& b, cudaStream_t st) {
   if (b.dense)  // the column layout keeps the tile kernel's cell table for every other pass
     k_pair_tile<R, MODE, SPECIAL, VIRIAL, NEAR><<<b.dense == 2 ? b.pair_cells.n : b.pair.n, kCellWarps * 32, 0, st>>>(
         b.sys, b.dense == 2 ? b.pair_cells.d : b.pair.d, 0, nullptr, nullptr, nullptr, nullptr, band);
-  else if (b.lean)
-    k_pair2<R, MODE, SPECIAL, VIRIAL, NEAR><<<b.pair.n, kPairWarps * 32, 0, st>>>(b.sys, b.pair.d);
-  else
+  else if (b.lean) {
+    constexpr bool kSpills = sizeof(R) == 8 && SPECIAL;
+    if (kSpills && b.natoms <= kLeanFewAtoms)
+      k_pair2<R, MODE, SPECIAL, VIRIAL, NEAR, kSpills ? 2 : 3><<<b.pair.n, kPairWarps * 32, 0, st>>>(b.sys, b.pair.d);
+    else
+      k_pair2<R, MODE, SPECIAL, VIRIAL, NEAR, 3><<<b.pair.n, kPairWarps * 32, 0, st>>>(b.sys, b.pair.d);
+  } else
     k_pair<R, MODE, SPECIAL, VIRIAL, NEAR><<<b.pair.n, kPairWarps * 32, 0, st>>>(b.sys, b.pair.d, 0, nullptr,
                                                                                 nullptr, nullptr, nullptr);
   note_launch();
