@@ -1228,17 +1228,25 @@ int Context::step(const int32_t* ids, int n, int nsteps) {
     }
     if (!gr->graph) {
       long long before = launches_issued();
-      cudaGraph_t g;
-      cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal);
-      for (auto* br : bs) enqueue_step(br->b);
-      cudaStreamEndCapture(stream, &g);
-      if (cudaGraphInstantiate(&gr->graph, g, 0) != cudaSuccess) {
-        cudaGraphDestroy(g);
-        return fail(RBMD_ERR_CUDA, "graph instantiate failed");
+      // A launch refused during the capture ends it: nothing is kept, and the next call starts clean.
+      cudaGraph_t g = nullptr;
+      cudaError_t e = cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal);
+      if (e == cudaSuccess) {
+        for (auto* br : bs) enqueue_step(br->b);
+        const cudaError_t refused = cudaGetLastError();
+        e = cudaStreamEndCapture(stream, &g);
+        if (refused != cudaSuccess) e = refused;
       }
-      cudaGraphDestroy(g);
-      gr->graph_steps = (int)(launches_issued() - before);
-      note_launch(-(int)gr->graph_steps);
+      if (e == cudaSuccess) e = cudaGraphInstantiate(&gr->graph, g, 0);
+      if (g) cudaGraphDestroy(g);
+      const int captured = (int)(launches_issued() - before);
+      note_launch(-captured);
+      if (e != cudaSuccess) {
+        gr->graph = nullptr;
+        cudaGetLastError();
+        return fail(RBMD_ERR_CUDA, std::string("step capture: ") + cudaGetErrorString(e));
+      }
+      gr->graph_steps = captured;
     }
     for (int k = 0; k < nsteps; ++k) cudaGraphLaunch(gr->graph, stream);
     note_launch(gr->graph_steps * nsteps);
