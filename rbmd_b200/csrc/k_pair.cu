@@ -2020,6 +2020,7 @@ constexpr int kColQ = kColStage;  // the most steps between evaluations: a stage
 constexpr int kColQW = kColQ / 32;  // 32-step blocks between evaluations
 constexpr int kColKeep = 12;     // 32-step blocks whose masks a warp of the split form keeps
 constexpr int kColMaxRows = 64;  // traversal rows the split form takes
+constexpr int kColMaxRows16 = 32;  // and with sixteen warps per chunk
 constexpr float kColFar = 1e30f;
 // resident blocks per SM: 4 (128 registers per thread) ran the saline stream's column launch in
 // 34.2 ms against 36.1 ms at 5 (96 registers, twice the local-memory traffic of spills)
@@ -2228,6 +2229,8 @@ struct ColRow {
 constexpr size_t col_smem(int split, int nrows) {
   return split == 1 ? 0 : split * sizeof(ColWarp<true>) + (size_t)nrows * sizeof(ColRow);
 }
+static_assert(col_smem(8, kColMaxRows) + 64 <= 227 * 1024 && col_smem(16, kColMaxRows16) + 64 <= 227 * 1024,
+              "a block's shared memory");
 
 // WARPS: warps that share a chunk (1: a block of kColWarps warps with a chunk each).
 template <int MODE, bool SPECIAL, bool NEAR, int WARPS>
@@ -2782,14 +2785,23 @@ void plan_pair_col(Batch& b, double chunks, double longest, int nc) {
   // chunks); above, its second staging costs more than it spreads (3420 -> 5460 us for 985,000 atoms).
   // Four warps per chunk were no better anywhere (78, 117 and 469 us).  Sixteen, a block to an SM, while
   // there are SMs for the chunks: 50 -> 41 us for 1200 atoms; beyond, eight (414 against 530 us at 64,000).
-  b.col_split = b.col_rows > kColMaxRows || chunks >= 2200 ? 1 : (chunks <= 148 && b.col_rows <= 32 ? 16 : 8);
+  b.col_split = b.col_rows > kColMaxRows || chunks >= 2200 ? 1 : (chunks <= 148 && b.col_rows <= kColMaxRows16 ? 16 : 8);
   int dev = 0, sms = 0, per_sm = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  // The limit on dynamic shared memory belongs to the kernel, of the whole process: always the most a
+  // form can need, so that planning a batch of few rows takes nothing from a batch planned before it.
+  if (b.col_split > 1) {
+    const size_t most = b.col_split == 16 ? col_smem(16, kColMaxRows16) : col_smem(8, kColMaxRows);
+    if (cudaFuncSetAttribute(b.col_split == 16 ? col_kernel<16>(b) : col_kernel<8>(b),
+                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most) != cudaSuccess) {
+      cudaGetLastError();
+      b.col_split = 1;
+    }
+  }
   const void* fn = b.col_split == 16 ? col_kernel<16>(b) : (b.col_split == 8 ? col_kernel<8>(b) : col_kernel<1>(b));
   const size_t smem = col_smem(b.col_split, b.col_rows);
   const int warps = b.col_split > 1 ? b.col_split : kColWarps;  // per block
-  if (smem) cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, warps * 32, smem);
   const long long items = (long long)b.pair.n * b.col_parts;
   const long long need = b.col_split > 1 ? items : (items + kColWarps - 1) / kColWarps;

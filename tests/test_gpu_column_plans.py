@@ -55,3 +55,31 @@ def test_a_step_that_cannot_be_captured_leaves_nothing_behind(ctx_factory, pair)
     if done:
         for sid, f in zip(ids, stepped):
             assert np.array_equal(ctx.forces(sid), f)
+
+
+def test_forces_of_one_call_and_in_turns(ctx_factory, pair):
+    init = [_alone(ctx_factory, sd, 0) for sd in pair]
+    stepped = [_alone(ctx_factory, sd, 2) for sd in pair]
+    ctx = ctx_factory()
+    ids = [ctx.add_system(sd) for sd in pair]
+    ctx.init(ids)
+    for sid, f in zip(ids, init):
+        assert np.array_equal(ctx.forces(sid), f)
+    for turn in (0, 1, 0):  # positions unchanged: the same forces again
+        ctx.compute_forces(ids[turn])
+        assert np.array_equal(ctx.forces(ids[turn]), init[turn])
+    ctx.step(ids, 2)
+    for sid, f in zip(ids, stepped):
+        assert np.array_equal(ctx.forces(sid), f)
+    ctx.thermo(ids[0])
+
+
+def test_a_second_context_does_not_disturb_the_first(ctx_factory, pair):
+    init = _alone(ctx_factory, pair[0], 0)
+    first, second = ctx_factory(), ctx_factory()
+    a = first.add_system(pair[0])
+    first.init(a)
+    b = second.add_system(pair[1])
+    second.init(b)
+    first.compute_forces(a)
+    assert np.array_equal(first.forces(a), init)
