@@ -7,7 +7,8 @@ namespace rbmd {
 
 // Puts atom i, at position pc, into its cell: the cell's count, the atom's place in the cell's bucket
 // (in order of arrival; the build kernel orders the ids), and how far the atom lies outside the cell.
-// Buckets hold cell_cap ids; the atoms beyond go to one overflow list per system.
+// Buckets hold cell_cap ids; the atoms beyond are chained per cell, kCellChains chains taken in turn.  A
+// chain's length follows from the cell's count, so heads and links are never cleared.
 __device__ __forceinline__ void bin_atom(const SysDev& s, int i, const double (&pc)[3]) {
   SysState* st = s.st;
   const int par = st->cell_epoch & 1;
@@ -28,7 +29,7 @@ __device__ __forceinline__ void bin_atom(const SysDev& s, int i, const double (&
   s.cell_of_atom[i] = cell;
   const int slot = atomicAdd(&s.cell_count[(size_t)par * s.cell_stride + cell], 1);
   if (slot < s.cell_cap) s.cell_bucket[(size_t)cell * s.cell_cap + slot] = i;
-  else s.cell_ovf[atomicAdd(&st->ovf_n[par], 1)] = i;
+  else s.cell_next[i] = atomicExch(&s.cell_head[(size_t)cell * kCellChains + ((slot - s.cell_cap) & (kCellChains - 1))], i);
 }
 
 }  // namespace rbmd

@@ -21,6 +21,7 @@ constexpr int kCellBlock = 256;        // cells per work item of the cell kernel
 constexpr int kBuildCells = 32;        // cells per block of the cell-list build
 constexpr int kBuildFew = 8;           // and in systems of up to kFewCells cells
 constexpr int kFewCells = 1024;
+constexpr int kCellChains = 4;         // chains of a cell's atoms beyond its bucket
 constexpr int kCellBigGrid = 16384;    // cells of a system above which counts are added up in two levels
 constexpr int kRbeSlack = 64;          // Metropolis proposal slots tried beyond the samples still to draw
 constexpr int kEamRow = 8;             // doubles per row of the device's rhor and z2r tables
@@ -90,10 +91,9 @@ struct SysState {
   unsigned out_bits;
   int mig_n;
   // Cell-list building (k_cells.cu): the buffer of counts the next list takes (bit 0), and for each
-  // buffer the distance above as it is gathered and the atoms beyond the buckets' capacity.
+  // buffer the distance above as it is gathered.
   int cell_epoch;
   unsigned out_acc[2];
-  int ovf_n[2];
   int mig_cell[kMaxMigrated];
 };
 
@@ -157,7 +157,9 @@ struct SysDev {
   int* cell_count;     // [2][cell_stride] two buffers, taken in turn
   int* cell_start;     // [ncell + 1]
   int* cell_bucket;    // [ncell][cell_cap] atom ids in order of arrival
-  int* cell_ovf;       // [n] atoms that found their cell's bucket full
+  int* cell_head;      // [ncell][kCellChains] last atom of each chain of those that found the bucket full
+  int* cell_next;      // [n] the chains' links
+  int* cell_rest;      // [n] scratch, by place in cell order: the chained atoms of a cell, one after the other
   int* cell_gsum;      // [ncell / 32 + 1] atoms per 32 cells (systems of many cells)
   int* sorted;         // atom ids in cell order
   int* rank;           // [n] position of each atom in cell order (inverse of sorted)

@@ -254,7 +254,7 @@ int Context::refresh(System* s) {
 static int rho_chunk(int n) { return n <= 148 * 64 ? 64 : (n <= 148 * 128 ? 128 : kRhoChunk); }
 
 // Ids a cell's bucket holds: twice the mean occupancy and at least 4 more (a liquid's cells rarely pass
-// 1.5 times it; the atoms beyond go through the overflow list, at a cost per atom of the list's length).
+// 1.5 times it; in a box that is filled in part only, most cells that hold atoms do).
 static int cell_bucket(int n, int ncell) { return (int)(2 * (int64_t)n / ncell + 4 + 3) & ~3; }
 
 int64_t Context::estimate_bytes(const rbmd_system_desc& d, const rbmd_params& p) {
@@ -263,7 +263,7 @@ int64_t Context::estimate_bytes(const rbmd_system_desc& d, const rbmd_params& p)
   const int64_t n = d.n_atoms;
   int64_t b = n * (32 * 3 + 16 + 12 + 4 * 2 + 32 + 16 + 16 + 8);  // x v f meta image cells sorted sx sxf smeta fp
   if (p.fix_shake == RBMD_SHAKE_TRUE && d.n_angles > 0) b += n * 32 * 3;
-  b += n * 4 + (int64_t)dv.n_cells * (13 + 4 * cell_bucket(d.n_atoms, dv.n_cells)) *
+  b += n * 8 + (int64_t)dv.n_cells * (13 + 4 * kCellChains + 4 * cell_bucket(d.n_atoms, dv.n_cells)) *
                    (p.ensemble == RBMD_ENS_NPT ? 2 : 1);  // NPT: room for kBoxGrow^3
   const int P = p.coulomb == RBMD_COUL_RBE ? p.coulomb_sample_num : 0;
   int64_t nk = P;
@@ -679,7 +679,9 @@ int Context::add_system(const rbmd_system_desc& d, const rbmd_params& p, int32_t
   D.cell_count = (int*)dal(sizeof(int) * 2 * D.cell_stride);
   D.cell_start = (int*)dal(sizeof(int) * (D.ncell_cap + 1));
   D.cell_bucket = (int*)dal(sizeof(int) * (size_t)D.ncell_cap * D.cell_cap);
-  D.cell_ovf = (int*)dal(sizeof(int) * n);
+  D.cell_head = (int*)dal(sizeof(int) * (size_t)D.ncell_cap * kCellChains);
+  D.cell_next = (int*)dal(sizeof(int) * n);
+  D.cell_rest = (int*)dal(sizeof(int) * n);
   D.cell_gsum = (int*)dal(sizeof(int) * (D.ncell_cap / 32 + 1));
   D.sorted = (int*)dal(sizeof(int) * n);
   D.rank = (int*)dal(sizeof(int) * n);
