@@ -1131,13 +1131,12 @@ void Context::join_side(cudaStream_t side) {
 void Context::enqueue_assembly(const Batch& b, FinalMode mode, int virial) {
   cudaStream_t side = stream;
   if (b.coul != RBMD_COUL_NONE || b.has_bonded) {
+    const bool in_final = far_in_final(b, virial);
     side = fork_side();
-    if (b.coul != RBMD_COUL_NONE) {
-      timed("rho", 0, [&] { launch_rho(b, side, b.coul == RBMD_COUL_EWALD); });
-      timed("far", (double)b.natoms, [&] { launch_far(b, side, virial); });
-    }
+    if (b.coul != RBMD_COUL_NONE) timed("rho", 0, [&] { launch_rho(b, side, b.coul == RBMD_COUL_EWALD); });
+    if (b.coul != RBMD_COUL_NONE && !in_final) timed("far", (double)b.natoms, [&] { launch_far(b, side, virial); });
     if (b.has_bonded) timed("bonded", 0, [&] { launch_bonded(b, side, virial); });
-    timed("intra", (double)b.natoms, [&] { launch_intra(b, side, virial); });
+    if (b.ff == RBMD_FF_CVFF && !in_final) timed("intra", (double)b.natoms, [&] { launch_intra(b, side, virial); });
   }
   timed(pair_name(b), (double)b.natoms, [&] { launch_pair(b, stream, virial); });
   join_side(side);

@@ -264,17 +264,98 @@ __global__ void k_bonded(const SysDev* __restrict__ S, const int2* __restrict__ 
 }
 
 // ------------------------------------------------------------------ final force + kick
-// Far force of every atom (RBE or Ewald) into ffar.  A block takes kFarAtoms atoms and four threads
-// share an atom's k vectors, a quarter each: the sine / cosine loop is the kernel's time, and one thread
-// per atom made it a chain of P evaluations on an SM per 256 atoms (inside the force assembly, which
-// took 49 us for 8000 atoms and P = 200 in FP64, 25 us for 9000 and P = 100 in mixed precision).  A
-// kernel of its own, so that the split costs the assembly's memory-bound part no occupancy.  The
-// quarters are added in order: the sum does not depend on the launch.
+// The far force (RBE or Ewald) of an atom is a sum over k vectors in four parts, each added up by itself
+// and the parts in order, so that the result does not depend on who sums them: four threads in k_far,
+// or the atom's own thread one part after the other in the force assembly (launch_final).
+constexpr int kFarParts = kAtomBlock / kFarAtoms;
+constexpr int kFarK = 256;  // k vectors staged at a time
+static_assert(kFarAtoms % 32 == 0, "a part is whole warps");
+
+template <bool MIXED>
+struct FarStage {
+  using Acc = double;
+  double4 k[kFarK];
+  double2 r[kFarK];
+};
+template <>
+struct FarStage<true> {
+  using Acc = float;
+  float4 m[kFarK], k[kFarK];  // mixed precision: indices and coefficient; FP32 k vector
+  float2 r[kFarK];
+};
+
+// The system's k vectors k0 .. k0 + n - 1 and their structure factors, by the whole block.
+template <bool MIXED>
+__device__ __forceinline__ void far_stage(const SysDev& s, int k0, int n, FarStage<MIXED>& t) {
+  for (int k = threadIdx.x; k < n; k += blockDim.x) {
+    const int l = k0 + k;
+    const double4 kv = s.kv[l];
+    const double re = s.rhok[2 * l], im = s.rhok[2 * l + 1];
+    if constexpr (MIXED) {
+      t.m[k] = make_float4((float)s.km[3 * l], (float)s.km[3 * l + 1], (float)s.km[3 * l + 2], (float)kv.w);
+      t.r[k] = make_float2((float)re, (float)im);
+      t.k[k] = make_float4((float)kv.x, (float)kv.y, (float)kv.z, 0.0f);
+    } else {
+      t.k[k] = kv;
+      t.r[k] = make_double2(re, im);
+    }
+  }
+}
+
+// Adds part p of n staged k vectors to an atom's sum.
+template <bool MIXED, bool VIRIAL>
+__device__ __forceinline__ void far_part(const SysDev& s, const FarStage<MIXED>& t, int n, int p, const double4& xi,
+                                         typename FarStage<MIXED>::Acc (&f)[3], double (&vir)[6]) {
+  const int ka = n * p / kFarParts, kb = n * (p + 1) / kFarParts;
+  if constexpr (MIXED) {
+    const float ux = (float)(xi.x / s.L[0]), uy = (float)(xi.y / s.L[1]), uz = (float)(xi.z / s.L[2]);
+    const float q = (float)xi.w;
+    for (int k = ka; k < kb; ++k) {
+      const float4 m = t.m[k];
+      float ph = m.x * ux + m.y * uy + m.z * uz;
+      ph -= __fsub_rn(__fadd_rn(ph, 12582912.0f), 12582912.0f);  // rint on the FMA pipe, |ph| < 2^22
+      float sn, cs;
+      __sincosf(6.28318531f * ph, &sn, &cs);  // hardware sin / cos: |2 pi ph| <= pi
+      const float2 r = t.r[k];
+      const float Fs = m.w * q * (cs * r.y - sn * r.x);
+      const float4 kf = t.k[k];
+      f[0] += Fs * kf.x;
+      f[1] += Fs * kf.y;
+      f[2] += Fs * kf.z;
+    }
+  } else {
+    for (int k = ka; k < kb; ++k) {
+      const double4 kv = t.k[k];
+      const double2 r = t.r[k];
+      const double dot = kv.x * xi.x + kv.y * xi.y + kv.z * xi.z;
+      double sn, cs;
+      sincos(dot, &sn, &cs);
+      const double Fs = kv.w * xi.w * (cs * r.y - sn * r.x);
+      f[0] += Fs * kv.x;
+      f[1] += Fs * kv.y;
+      f[2] += Fs * kv.z;
+      if (VIRIAL) {  // ComputeKspaceVirial, ExecForceFunction.h:397-410
+        vir[0] += (xi.x * kv.x + xi.x * kv.x) * Fs;
+        vir[1] += (xi.y * kv.y + xi.y * kv.y) * Fs;
+        vir[2] += (xi.z * kv.z + xi.z * kv.z) * Fs;
+        vir[3] += (xi.x * kv.y + xi.y * kv.x) * Fs;
+        vir[4] += (xi.x * kv.z + xi.z * kv.x) * Fs;
+        vir[5] += (xi.y * kv.z + xi.z * kv.y) * Fs;
+      }
+    }
+  }
+}
+
+__device__ __forceinline__ double far_scale(const SysDev& s) {
+  return (s.coul == RBMD_COUL_RBE ? s.S / s.P : 1.0) * s.qqr2e;
+}
+
+// Far force of every atom into ffar.  A block takes kFarAtoms atoms and four threads share an atom's k
+// vectors, a quarter each: the sine / cosine loop is the kernel's time, and one thread per atom made it a
+// chain of P evaluations on an SM per 256 atoms (inside the force assembly, which took 49 us for 8000
+// atoms and P = 200 in FP64, 25 us for 9000 and P = 100 in mixed precision).
 template <bool MIXED, bool VIRIAL>
 __global__ void __launch_bounds__(kAtomBlock, 4) k_far(const SysDev* __restrict__ S, const int2* __restrict__ work) {
-  constexpr int kParts = kAtomBlock / kFarAtoms;
-  constexpr int kK = 256;  // k vectors staged at a time
-  static_assert(kFarAtoms % 32 == 0, "a part is whole warps");
   const int2 wk = work[blockIdx.x];
   const SysDev& s = S[wk.x];
   const int first = wk.y + blockIdx.y * kFarAtoms;
@@ -282,86 +363,29 @@ __global__ void __launch_bounds__(kAtomBlock, 4) k_far(const SysDev* __restrict_
   const int part = threadIdx.x / kFarAtoms, a = threadIdx.x % kFarAtoms;
   const int i = first + a;
   const bool in = i < s.n;
-  __shared__ double4 s_k[kK];
-  __shared__ double2 s_r[kK];
-  __shared__ float4 s_kf[kK];
-  __shared__ float2 s_rf[kK];
-  float4* s_kk = reinterpret_cast<float4*>(s_k);  // mixed precision: FP32 k vectors (s_k unused)
+  __shared__ FarStage<MIXED> s_t;
   __shared__ double s_far[3][kAtomBlock];
   const double4 xi = in ? s.x[i] : make_double4(0, 0, 0, 0);
   const int nk = s.coul == RBMD_COUL_RBE ? s.P : s.nk_ewald;
-  double fx = 0, fy = 0, fz = 0;
+  typename FarStage<MIXED>::Acc f[3] = {0, 0, 0};
   double vir[6] = {0, 0, 0, 0, 0, 0};
-  float gx = 0.f, gy = 0.f, gz = 0.f;
-  const float ux = (float)(xi.x / s.L[0]), uy = (float)(xi.y / s.L[1]), uz = (float)(xi.z / s.L[2]);
-  for (int k0 = 0; k0 < nk; k0 += kK) {
-    const int nch = min(kK, nk - k0);
+  for (int k0 = 0; k0 < nk; k0 += kFarK) {
+    const int nch = min(kFarK, nk - k0);
     __syncthreads();
-    for (int k = threadIdx.x; k < nch; k += blockDim.x) {
-      const double4 kv = s.kv[k0 + k];
-      const double re = s.rhok[2 * (k0 + k)], im = s.rhok[2 * (k0 + k) + 1];
-      if (MIXED) {
-        const int l = k0 + k;
-        s_kf[k] = make_float4((float)s.km[3 * l], (float)s.km[3 * l + 1], (float)s.km[3 * l + 2], (float)kv.w);
-        s_rf[k] = make_float2((float)re, (float)im);
-        s_kk[k] = make_float4((float)kv.x, (float)kv.y, (float)kv.z, 0.0f);
-      } else {
-        s_k[k] = kv;
-        s_r[k] = make_double2(re, im);
-      }
-    }
+    far_stage<MIXED>(s, k0, nch, s_t);
     __syncthreads();
-    const int ka = nch * part / kParts, kb = nch * (part + 1) / kParts;  // this part's k vectors
-    if (in) {
-      if (MIXED) {
-        const float q = (float)xi.w;
-        for (int k = ka; k < kb; ++k) {
-          const float4 m = s_kf[k];
-          float ph = m.x * ux + m.y * uy + m.z * uz;
-          ph -= __fsub_rn(__fadd_rn(ph, 12582912.0f), 12582912.0f);  // rint on the FMA pipe, |ph| < 2^22
-          float sn, cs;
-          __sincosf(6.28318531f * ph, &sn, &cs);  // hardware sin / cos: |2 pi ph| <= pi
-          const float2 r = s_rf[k];
-          const float Fs = m.w * q * (cs * r.y - sn * r.x);
-          const float4 kf = s_kk[k];
-          gx += Fs * kf.x;
-          gy += Fs * kf.y;
-          gz += Fs * kf.z;
-        }
-      } else {
-        for (int k = ka; k < kb; ++k) {
-          const double4 kv = s_k[k];
-          const double2 r = s_r[k];
-          const double dot = kv.x * xi.x + kv.y * xi.y + kv.z * xi.z;
-          double sn, cs;
-          sincos(dot, &sn, &cs);
-          const double Fs = kv.w * xi.w * (cs * r.y - sn * r.x);
-          fx += Fs * kv.x;
-          fy += Fs * kv.y;
-          fz += Fs * kv.z;
-          if (VIRIAL) {  // ComputeKspaceVirial, ExecForceFunction.h:397-410
-            vir[0] += (xi.x * kv.x + xi.x * kv.x) * Fs;
-            vir[1] += (xi.y * kv.y + xi.y * kv.y) * Fs;
-            vir[2] += (xi.z * kv.z + xi.z * kv.z) * Fs;
-            vir[3] += (xi.x * kv.y + xi.y * kv.x) * Fs;
-            vir[4] += (xi.x * kv.z + xi.z * kv.x) * Fs;
-            vir[5] += (xi.y * kv.z + xi.z * kv.y) * Fs;
-          }
-        }
-      }
-    }
+    if (in) far_part<MIXED, VIRIAL>(s, s_t, nch, part, xi, f, vir);
   }
-  s_far[0][threadIdx.x] = MIXED ? (double)gx : fx;
-  s_far[1][threadIdx.x] = MIXED ? (double)gy : fy;
-  s_far[2][threadIdx.x] = MIXED ? (double)gz : fz;
+#pragma unroll
+  for (int k = 0; k < 3; ++k) s_far[k][threadIdx.x] = (double)f[k];
   __syncthreads();
-  const double sc = (s.coul == RBMD_COUL_RBE ? s.S / s.P : 1.0) * s.qqr2e;
+  const double sc = far_scale(s);
   if (in && part == 0) {
     double F[3];
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
       double t = 0.0;
-      for (int p = 0; p < kParts; ++p) t += s_far[k][p * kFarAtoms + a];
+      for (int p = 0; p < kFarParts; ++p) t += s_far[k][p * kFarAtoms + a];
       F[k] = t * sc;
     }
     s.ffar[i] = make_double4(F[0], F[1], F[2], 0.0);
@@ -375,10 +399,52 @@ __global__ void __launch_bounds__(kAtomBlock, 4) k_far(const SysDev* __restrict_
   }
 }
 
-// Intramolecular Coulomb exclusion and bonded terms of every atom, added to its far force.  Chains of
-// dependent gathers (molecule, partner, special list, term slots, term forces) of 10 us that need only
-// positions: beside the pair kernel they cost nothing, in the force assembly they were the wait of it
-// (17 us for 9000 atoms of water against 8 us without them).
+// Intramolecular Coulomb exclusion and bonded terms of an atom, added to F.
+template <bool VIRIAL>
+__device__ __forceinline__ void intra_terms(const SysDev& s, int i, const double4& xi, double (&F)[3], double (&vir)[6]) {
+  // ---- intramolecular Coulomb exclusion (CVFF + RBL + special bonds)
+  if (s.ff == RBMD_FF_CVFF && s.neigh == RBMD_NEIGH_RBL && s.special) {
+    const int4 mi = s.meta[i];
+    const int b = s.mol_off[mi.y], e = s.mol_off[mi.y + 1];
+    if (e - b >= 3) {
+      const int sb = s.sp_off[i], se = s.sp_off[i + 1];
+      for (int k = b; k < e; ++k) {
+        const int j = s.mol_atoms[k];
+        if (j == i) continue;
+        const double4 xj = s.x[j];
+        double rx = xi.x - xj.x, ry = xi.y - xj.y, rz = xi.z - xj.z;
+        min_image(rx, ry, rz, s.L[0], s.L[1], s.L[2]);
+        const double dis = sqrt(rx * rx + ry * ry + rz * rz);
+        const double fc = -332.06371 * xi.w * xj.w / (dis * dis * dis);
+        double w = 1.0;
+        for (int q = sb; q < se; ++q)
+          if (s.sp_ids[q] == j) w = s.sp_w[q];
+        const double cx = (1.0 - w) * fc * rx, cy = (1.0 - w) * fc * ry, cz = (1.0 - w) * fc * rz;
+        F[0] += cx;
+        F[1] += cy;
+        F[2] += cz;
+        if (VIRIAL) {
+          vir[0] += rx * 0.5 * cx; vir[1] += ry * 0.5 * cy; vir[2] += rz * 0.5 * cz;
+          vir[3] += rx * 0.5 * cy; vir[4] += rx * 0.5 * cz; vir[5] += ry * 0.5 * cz;
+        }
+      }
+    }
+  }
+  // ---- bonded terms (per-term forces gathered per atom)
+  if (s.n_bonds + s.n_angles + s.n_dihedrals > 0) {
+    for (int k = s.aterm_off[i]; k < s.aterm_off[i + 1]; ++k) {
+      const double4 tf = s.term_force[s.aterm[k]];
+      F[0] += tf.x;
+      F[1] += tf.y;
+      F[2] += tf.z;
+    }
+  }
+}
+
+// The above for every atom, added to its far force.  Chains of dependent gathers (molecule, partner,
+// special list, term slots, term forces) of 10 us that need only positions: beside the pair kernel they
+// cost nothing, in the force assembly they were the wait of it (17 us for 9000 atoms of water against
+// 8 us without them).
 template <bool VIRIAL>
 __global__ void __launch_bounds__(kAtomBlock) k_intra(const SysDev* __restrict__ S, const int2* __restrict__ work) {
   const int2 wk = work[blockIdx.x];
@@ -386,46 +452,9 @@ __global__ void __launch_bounds__(kAtomBlock) k_intra(const SysDev* __restrict__
   const int i = wk.y + threadIdx.x;
   double vir[6] = {0, 0, 0, 0, 0, 0};
   if (i < s.n) {
-    const double4 xi = s.x[i];
     const double4 ff = s.ffar[i];
     double F[3] = {ff.x, ff.y, ff.z};
-    // ---- intramolecular Coulomb exclusion (CVFF + RBL + special bonds)
-    if (s.ff == RBMD_FF_CVFF && s.neigh == RBMD_NEIGH_RBL && s.special) {
-      const int4 mi = s.meta[i];
-      const int b = s.mol_off[mi.y], e = s.mol_off[mi.y + 1];
-      if (e - b >= 3) {
-        const int sb = s.sp_off[i], se = s.sp_off[i + 1];
-        for (int k = b; k < e; ++k) {
-          const int j = s.mol_atoms[k];
-          if (j == i) continue;
-          const double4 xj = s.x[j];
-          double rx = xi.x - xj.x, ry = xi.y - xj.y, rz = xi.z - xj.z;
-          min_image(rx, ry, rz, s.L[0], s.L[1], s.L[2]);
-          const double dis = sqrt(rx * rx + ry * ry + rz * rz);
-          const double fc = -332.06371 * xi.w * xj.w / (dis * dis * dis);
-          double w = 1.0;
-          for (int q = sb; q < se; ++q)
-            if (s.sp_ids[q] == j) w = s.sp_w[q];
-          const double cx = (1.0 - w) * fc * rx, cy = (1.0 - w) * fc * ry, cz = (1.0 - w) * fc * rz;
-          F[0] += cx;
-          F[1] += cy;
-          F[2] += cz;
-          if (VIRIAL) {
-            vir[0] += rx * 0.5 * cx; vir[1] += ry * 0.5 * cy; vir[2] += rz * 0.5 * cz;
-            vir[3] += rx * 0.5 * cy; vir[4] += rx * 0.5 * cz; vir[5] += ry * 0.5 * cz;
-          }
-        }
-      }
-    }
-    // ---- bonded terms (per-term forces gathered per atom)
-    if (s.n_bonds + s.n_angles + s.n_dihedrals > 0) {
-      for (int k = s.aterm_off[i]; k < s.aterm_off[i + 1]; ++k) {
-        const double4 tf = s.term_force[s.aterm[k]];
-        F[0] += tf.x;
-        F[1] += tf.y;
-        F[2] += tf.z;
-      }
-    }
+    intra_terms<VIRIAL>(s, i, s.x[i], F, vir);
     s.ffar[i] = make_double4(F[0], F[1], F[2], 0.0);
   }
   if (VIRIAL) {
@@ -439,8 +468,9 @@ __global__ void __launch_bounds__(kAtomBlock) k_intra(const SysDev* __restrict__
 }
 
 // Force assembly, half kick, kinetic energy and, in the system's last block, the thermostat.  Bound by
-// memory (200 B per atom).
-template <bool VIRIAL>
+// memory (200 B per atom).  FAR: the far force and the intramolecular terms are formed here (mixed
+// precision with RBE, in batches that fill the chip, see launch_final) and not read from ffar.
+template <bool VIRIAL, bool FAR>
 __global__ void __launch_bounds__(kAtomBlock, 4)
 k_final(const SysDev* __restrict__ S, const int2* __restrict__ work, int mode) {
   const int2 wk = work[blockIdx.x];
@@ -463,7 +493,37 @@ k_final(const SysDev* __restrict__ S, const int2* __restrict__ work, int mode) {
     F[1] -= st->fmean[1];
     F[2] -= st->fmean[2];
   }
-  if (act && s.coul != RBMD_COUL_NONE) {  // far force, intramolecular terms (k_far, k_intra)
+  if constexpr (FAR) {
+    __shared__ FarStage<true> s_t;
+    const double4 xi = act ? s.x[i] : make_double4(0, 0, 0, 0);
+    float f[kFarParts][3];
+    double none[6];
+#pragma unroll
+    for (int p = 0; p < kFarParts; ++p) f[p][0] = f[p][1] = f[p][2] = 0.f;
+    for (int k0 = 0; k0 < s.P; k0 += kFarK) {
+      const int nch = min(kFarK, s.P - k0);
+      __syncthreads();
+      far_stage<true>(s, k0, nch, s_t);
+      __syncthreads();
+      if (act)
+#pragma unroll
+        for (int p = 0; p < kFarParts; ++p) far_part<true, false>(s, s_t, nch, p, xi, f[p], none);
+    }
+    if (act) {
+      const double sc = far_scale(s);
+      double ff[3];
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        double t = 0.0;
+#pragma unroll
+        for (int p = 0; p < kFarParts; ++p) t += (double)f[p][k];
+        ff[k] = t * sc;
+      }
+      if (s.ff == RBMD_FF_CVFF) intra_terms<false>(s, i, xi, ff, none);
+#pragma unroll
+      for (int k = 0; k < 3; ++k) F[k] = ff[k] + F[k];
+    }
+  } else if (act && s.coul != RBMD_COUL_NONE) {  // far force, intramolecular terms (k_far, k_intra)
     const double4 ff = s.ffar[i];
     F[0] = ff.x + F[0];
     F[1] = ff.y + F[1];
@@ -940,9 +1000,19 @@ void launch_intra(const Batch& b, cudaStream_t st, int virial) {
   note_launch();
 }
 
+// Beside the pair kernel k_far and k_intra cost little only while it leaves room on the chip; in batches
+// that fill it for long their own traffic (128 B per atom) and staging count in full.  Steps with the two
+// kernels and with everything in the assembly: 1.02 M atoms 3993 and 4032 us, 1.54 M 5950 and 5950, 2.05 M
+// 7865 and 7860, 4.10 M 15,338 and 15,272, 7.86 M 31.11 and 30.51 ms (before the pair kernel's parts).
+constexpr long long kFarInFinalAtoms = 2000000;
+bool far_in_final(const Batch& b, int virial) {
+  return !virial && b.prec == RBMD_PREC_MIXED && b.coul == RBMD_COUL_RBE && b.natoms >= kFarInFinalAtoms;
+}
+
 void launch_final(const Batch& b, cudaStream_t st, FinalMode mode, int virial) {
-  if (virial) k_final<true><<<b.atom.n, kAtomBlock, 0, st>>>(b.sys, b.atom.d, (int)mode);
-  else k_final<false><<<b.atom.n, kAtomBlock, 0, st>>>(b.sys, b.atom.d, (int)mode);
+  if (virial) k_final<true, false><<<b.atom.n, kAtomBlock, 0, st>>>(b.sys, b.atom.d, (int)mode);
+  else if (far_in_final(b, virial)) k_final<false, true><<<b.atom.n, kAtomBlock, 0, st>>>(b.sys, b.atom.d, (int)mode);
+  else k_final<false, false><<<b.atom.n, kAtomBlock, 0, st>>>(b.sys, b.atom.d, (int)mode);
   note_launch();
 }
 

@@ -62,6 +62,8 @@ void plan_pair_col(Batch& b, double chunks, double longest, int nc);
 void launch_far(const Batch& b, cudaStream_t s, int virial);
 // Intramolecular terms (CVFF) added to the far forces, after launch_far and launch_bonded.
 void launch_intra(const Batch& b, cudaStream_t s, int virial);
+// Whether launch_final forms the far force and the intramolecular terms itself (no launch_far, launch_intra).
+bool far_in_final(const Batch& b, int virial);
 void launch_final(const Batch& b, cudaStream_t s, FinalMode mode, int virial);
 void launch_ke_thermostat(const Batch& b, cudaStream_t s);
 void launch_flush_vscale(const Batch& b, cudaStream_t s);

@@ -52,3 +52,27 @@ def test_forces_match_oracle(ctx_factory, oracle_mod, n, P, precision, tol):
     o = oracle_mod.Oracle(sd)
     o.compute_forces()
     assert rel_rms(ctx.forces(sid), o.forces()) < tol
+
+
+@pytest.mark.parametrize("kind,P", [("water", 100), ("water", 300), ("ions", 200)])
+def test_assembly_of_a_large_batch_forms_the_same_forces(ctx_factory, kind, P):
+    """In batches of two million atoms and more the force assembly forms the far force and the
+    intramolecular terms itself.  The same sums in the same order: a small system alone and in such a
+    batch must agree bit for bit, also with more k vectors than are staged at a time."""
+    if kind == "water":
+        small, fill, count = synth.saline(1300, seed=1, P=P), synth.saline(64000, seed=2, P=P), 32
+    else:
+        small = synth.nacl_melt(n_side=12, P=P, precision=A.PREC_MIXED, seed=1)
+        fill, count = synth.nacl_melt(n_side=64, P=P, precision=A.PREC_MIXED, seed=2), 8
+    alone, large = ctx_factory(), ctx_factory()
+    a = alone.add_system(small)
+    b = [large.add_system(small)] + [large.add_system(fill) for _ in range(count)]
+    assert small.n + count * fill.n > 2000000
+    alone.init(a)
+    large.init(b)
+    assert np.array_equal(alone.forces(a), large.forces(b[0]))
+    alone.step(a, 2)
+    large.step(b, 2)
+    assert np.array_equal(alone.forces(a), large.forces(b[0]))
+    for x, y in zip(alone.state(a), large.state(b[0])):
+        assert np.array_equal(x, y)
