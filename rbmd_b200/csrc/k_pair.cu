@@ -2039,10 +2039,9 @@ __device__ __noinline__ unsigned col_classify_fp64(const SysDev* __restrict__ sp
   return (core ? 1u : 0u) | (shell ? 2u : 0u);
 }
 
-// Whether the atom at sorted index si, binned into home column (hx, hy) at z cell zl, lies outside
-// that cell: the unclamped cell of its FP64 position (ExecPointLocator::InWhichCell) is another.
-__device__ inline bool col_is_stray(const SysDev& s, int si, int hx, int hy, int zl) {
-  const double4 xd = ldg4(&s.sx[si]);
+// Whether an atom at xd, binned into home column (hx, hy) at z cell zl, lies outside that cell: the
+// unclamped cell of its FP64 position (ExecPointLocator::InWhichCell) is another.
+__device__ inline bool col_is_stray(const SysDev& s, const double4& xd, int hx, int hy, int zl) {
   return (int)((xd.x - s.lo[0]) / s.d[0]) != hx || (int)((xd.y - s.lo[1]) / s.d[1]) != hy ||
          (int)((xd.z - s.lo[2]) / s.d[2]) != zl;
 }
@@ -2057,7 +2056,7 @@ __device__ inline int col_first_skip(const SysDev& s, int i, int pice) {
   return nm == 0 ? 0 : pice - nm;
 }
 
-// The stray atoms, before the column kernel: a block looks 256 atoms over (in cell order), lists its
+// The stray atoms, before the column kernel: a block looks 256 atoms over, lists its
 // strays and walks them one after the other, its eight warps sharing a stray's traversal rows: first
 // counting every row's shells, then, with the counts of the rows before known, picking and evaluating.
 // Their forces are written where the column kernel reads them back for the RBL mean.  Strays are few
@@ -2081,11 +2080,12 @@ __global__ void __launch_bounds__(kAtomBlock, 3) k_pair_col_strays(const SysDev*
   const unsigned FULL = 0xffffffffu;
   if (threadIdx.x == 0) s_n = 0;
   __syncthreads();
+  // looked over in the atoms' own order: its loads do not wait for one another
   const int k = wk.y + threadIdx.x;
   if (k < s.n) {
-    const int c = __ldg(&s.cell_of_atom[__ldg(&s.smeta[k]).x]);
+    const int c = __ldg(&s.cell_of_atom[k]);
     const int dy = s.dims[1], dz = s.dims[2];
-    if (col_is_stray(s, k, c / (dz * dy), (c / dz) % dy, c % dz)) s_list[atomicAdd(&s_n, 1)] = k;
+    if (col_is_stray(s, ldg4(&s.x[k]), c / (dz * dy), (c / dz) % dy, c % dz)) s_list[atomicAdd(&s_n, 1)] = s.rank[k];
   }
   __syncthreads();
   const int nc = s.nc, side = 2 * nc + 1, nrows = side * side, pice = s.pice;
@@ -2313,7 +2313,7 @@ k_pair_col(const SysDev* __restrict__ S, const int2* __restrict__ work, int nwor
           i = mi.x;
           p4 = __ldg(&s.sxf[si]);
           zl = __ldg(&s.cell_of_atom[i]) - cbase;  // internal cell id iz + dz (iy + dy ix), this column
-          stray = col_is_stray(s, si, hx, hy, zl);
+          stray = col_is_stray(s, ldg4(&s.sx[si]), hx, hy, zl);
           c = col_first_skip(s, i, pice);
           int nsp = 0, spb = 0, sp0 = -1, sp1 = -1;
           float w0 = 1.0f, w1 = 1.0f;
@@ -2779,7 +2779,6 @@ static const void* col_kernel(const Batch& b) {
 void plan_pair_col(Batch& b, double chunks, double longest, int nc) {
   const int side = 2 * nc + 1;
   b.col_rows = side * side;
-  b.col_parts = std::max(1, std::min(1024, (int)std::ceil(1.2 * longest / 32.0)));
   // Up to about one chunk per resident warp (148 SMs x 16) the split form's eight warps per chunk are
   // faster: 177 -> 56 us (1200 atoms of saline), 216 -> 118 us (9000), 456 -> 439 us (64,000, 2140
   // chunks); above, its second staging costs more than it spreads (3420 -> 5460 us for 985,000 atoms).
@@ -2803,6 +2802,14 @@ void plan_pair_col(Batch& b, double chunks, double longest, int nc) {
   const size_t smem = col_smem(b.col_split, b.col_rows);
   const int warps = b.col_split > 1 ? b.col_split : kColWarps;  // per block
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, warps * 32, smem);
+  // A column is offered in as many parts as the longest holds chunks; in the one-warp form in fewer once
+  // every resident warp has ten items, since an item costs a counter, two loads and a fence also where it
+  // lies past a short column's end.  Column launches with 1, 2, 3, 4, 6 parts and with all nine: 25.90,
+  // 25.88, 25.85, 25.94, 26.13, 26.48 ms for 7.86 M atoms (the rule: one), 3.65, 3.49, 3.47, 3.39, 3.42,
+  // 3.46 ms for 970,000 (four), 1.47, 0.89, 0.74, 0.68, 0.68, 0.56 ms for 129,000 (all).
+  const long long resident = (long long)std::max(1, sms) * std::max(1, per_sm) * warps;
+  b.col_parts = std::max(1, std::min(1024, (int)std::ceil(1.2 * longest / 32.0)));
+  if (b.col_split == 1) b.col_parts = (int)std::min<long long>(b.col_parts, (10 * resident + b.pair.n - 1) / std::max(1, b.pair.n));
   const long long items = (long long)b.pair.n * b.col_parts;
   const long long need = b.col_split > 1 ? items : (items + kColWarps - 1) / kColWarps;
   b.col_grid = (int)std::max(1LL, std::min(need, (long long)std::max(1, sms) * std::max(1, per_sm)));
