@@ -238,9 +238,17 @@ __global__ void __launch_bounds__(kRhoWarps * 32) k_rho(const SysDev* __restrict
     }
   };
   double* part = s.rho_part + (size_t)blk * 2 * nk;
+  // FP32: the next 32 indices are loaded during the present ones' atoms
+  int3 m = make_int3(0, 0, 0);
+  auto index = [&](int l) {
+    if (kF32 && l < nk) m = make_int3(s.km[3 * l], s.km[3 * l + 1], s.km[3 * l + 2]);
+  };
+  index(lane);
   for (int l0 = 0, turn = 0; l0 < nk; l0 += 32, ++turn) {
     const int l = l0 + lane;
     double re = 0.0, im = 0.0;
+    const float mxr = (float)m.x, myr = (float)m.y, mzr = (float)m.z;
+    index(l + 32);
     if (l < nk) {
       if (kF32) {
         // phase in turns m . (r / L), reduced to [-1/2, 1/2] before the FP32 sine and cosine (the
@@ -248,7 +256,6 @@ __global__ void __launch_bounds__(kRhoWarps * 32) k_rho(const SysDev* __restrict
         // warp's atoms (at most 32), added in FP64 (the SFU also converts FP32 to FP64); the nearest
         // integer of the phase by the 1.5 * 2^23 addition (round to nearest even, |ph| < 2^22), on
         // the FMA pipe
-        const float mxr = (float)s.km[3 * l], myr = (float)s.km[3 * l + 1], mzr = (float)s.km[3 * l + 2];
         float pr = 0.0f, pm = 0.0f;
         for (int j = j0; j < j1; ++j) {
           const float4 u = s_u[j];
