@@ -1309,23 +1309,43 @@ int Context::read_back(void* dst, const void* src, size_t bytes) {
   return RBMD_OK;
 }
 
+// Packed on the device; where the memory for that cannot be had (a device that is full to the last) the
+// records themselves cross, into host memory.
 int Context::read3(const double4* src, double* dst, int n) {
   if (!dst) return RBMD_OK;
-  double* packed = (double*)dmalloc(sizeof(double) * 3 * (size_t)n);
-  if (!packed) return fail(RBMD_ERR_OOM, "read-back staging");
-  launch_pack3(src, packed, n, stream);
-  const int rc = read_back(dst, packed, sizeof(double) * 3 * (size_t)n);
-  dfree(packed);
-  return rc;
+  if (double* packed = (double*)dmalloc(sizeof(double) * 3 * (size_t)n)) {
+    launch_pack3(src, packed, n, stream);
+    const int rc = read_back(dst, packed, sizeof(double) * 3 * (size_t)n);
+    dfree(packed);
+    return rc;
+  }
+  std::vector<double4> h(n);
+  cudaMemcpyAsync(h.data(), src, sizeof(double4) * n, cudaMemcpyDeviceToHost, stream);
+  const int rc = sync();
+  if (rc) return rc;
+  for (int i = 0; i < n; ++i) {
+    dst[3 * (size_t)i] = h[i].x;
+    dst[3 * (size_t)i + 1] = h[i].y;
+    dst[3 * (size_t)i + 2] = h[i].z;
+  }
+  return RBMD_OK;
 }
 
 int Context::write3(double4* dst, const double* src, int n) {
-  double* packed = (double*)dmalloc(sizeof(double) * 3 * (size_t)n);
-  if (!packed) return fail(RBMD_ERR_OOM, "upload staging");
-  cudaMemcpyAsync(packed, src, sizeof(double) * 3 * (size_t)n, cudaMemcpyHostToDevice, stream);
-  launch_unpack3(dst, packed, n, stream);
-  dfree(packed);
-  return RBMD_OK;
+  if (double* packed = (double*)dmalloc(sizeof(double) * 3 * (size_t)n)) {
+    cudaMemcpyAsync(packed, src, sizeof(double) * 3 * (size_t)n, cudaMemcpyHostToDevice, stream);
+    launch_unpack3(dst, packed, n, stream);
+    dfree(packed);
+    return RBMD_OK;
+  }
+  std::vector<double4> h(n);
+  cudaMemcpyAsync(h.data(), dst, sizeof(double4) * n, cudaMemcpyDeviceToHost, stream);
+  int rc = sync();
+  if (rc) return rc;
+  for (int i = 0; i < n; ++i)
+    h[i] = make_double4(src[3 * (size_t)i], src[3 * (size_t)i + 1], src[3 * (size_t)i + 2], h[i].w);
+  cudaMemcpyAsync(dst, h.data(), sizeof(double4) * n, cudaMemcpyHostToDevice, stream);
+  return sync();
 }
 
 int Context::get_forces(int id, double* f) {
