@@ -43,6 +43,13 @@ Units make_units(int units) {
   return u;
 }
 
+constexpr int64_t kMaxCells = ((int64_t)1 << 31) - 65536;  // cell indices are ints, with room to round up
+
+// Cells of a box; a box of many empty cells can have more than an int holds (rbmd_derived.n_cells).
+static int64_t cells_of(const rbmd_derived& dv) {
+  return (int64_t)std::min(9e15, (double)dv.dims[0] * dv.dims[1] * dv.dims[2]);
+}
+
 // Derived quantities: ContPointLocator::SetRange/SetCutOff/SetRs (locator/ContPointLocator.h:44-73),
 // RBL capacity arithmetic (ExecutionMD.cpp:582-592, 772-783, 1033-1040), RBE normalisation S
 // (ExecForceFunction.h:771-797).
@@ -55,13 +62,12 @@ static void derive(const rbmd_system_desc& d, const rbmd_params& p, rbmd_derived
   const double rc = p.cut_off;
   const double rs = (p.neighbor == RBMD_NEIGH_RBL) ? p.r_core : p.cut_off;
   dv.num_cycles = (int)std::ceil(rc / rs);
-  dv.n_cells = 1;
   for (int k = 0; k < 3; ++k) {
     dv.dims[k] = (int)(L[k] / (rc / dv.num_cycles));
     if (dv.dims[k] < 1) dv.dims[k] = 1;
     dv.cell_width[k] = L[k] / dv.dims[k];
-    dv.n_cells *= dv.dims[k];
   }
+  dv.n_cells = (int)cells_of(dv);
   if (p.neighbor == RBMD_NEIGH_RBL) {
     double coeff = 1.0;
     if (p.force_field != RBMD_FF_EAM) {
@@ -255,7 +261,7 @@ static int rho_chunk(int n) { return n <= 148 * 64 ? 64 : (n <= 148 * 128 ? 128 
 
 // Ids a cell's bucket holds: twice the mean occupancy and at least 4 more (a liquid's cells rarely pass
 // 1.5 times it; in a box that is filled in part only, most cells that hold atoms do).
-static int cell_bucket(int n, int ncell) { return (int)(2 * (int64_t)n / ncell + 4 + 3) & ~3; }
+static int cell_bucket(int64_t n, int64_t ncell) { return (int)(2 * n / std::max<int64_t>(1, ncell) + 4 + 3) & ~3; }
 
 int64_t Context::estimate_bytes(const rbmd_system_desc& d, const rbmd_params& p) {
   rbmd_derived dv;
@@ -263,7 +269,7 @@ int64_t Context::estimate_bytes(const rbmd_system_desc& d, const rbmd_params& p)
   const int64_t n = d.n_atoms;
   int64_t b = n * (32 * 3 + 16 + 12 + 4 * 2 + 32 + 16 + 16 + 8);  // x v f meta image cells sorted sx sxf smeta fp
   if (p.fix_shake == RBMD_SHAKE_TRUE && d.n_angles > 0) b += n * 32 * 3;
-  b += n * 8 + (int64_t)dv.n_cells * (13 + 4 * kCellChains + 4 * cell_bucket(d.n_atoms, dv.n_cells)) *
+  b += n * 8 + cells_of(dv) * (13 + 4 * kCellChains + 4 * cell_bucket(n, cells_of(dv))) *
                    (p.ensemble == RBMD_ENS_NPT ? 2 : 1);  // NPT: room for kBoxGrow^3
   const int P = p.coulomb == RBMD_COUL_RBE ? p.coulomb_sample_num : 0;
   int64_t nk = P;
@@ -366,6 +372,7 @@ int Context::add_system(const rbmd_system_desc& d, const rbmd_params& p, int32_t
   for (int k = 0; k < 3; ++k)
     if (s->dv.dims[k] < s->dv.num_cycles)
       return fail(RBMD_ERR_UNSUPPORTED, "box shorter than the cut-off: fewer cells than num_cycles");
+  if (cells_of(s->dv) >= kMaxCells) return fail(RBMD_ERR_UNSUPPORTED, "box of about 2^31 cells or more");
   const int n = d.n_atoms;
   const Units u = make_units(p.units);
   SysDev& D = s->dev;
@@ -503,12 +510,14 @@ int Context::add_system(const rbmd_system_desc& d, const rbmd_params& p, int32_t
     s->tuned = true;  // one layout only
     D.lean = 0;
     D.dense = 0;
-    D.ncell_cap = 1;
+    double cap = 1;
     for (int k = 0; k < 3; ++k) {
       D.L0[k] = D.L[k];
       D.kmax[k] = p.kmax[k];
-      D.ncell_cap *= std::max(1, (int)((kBoxGrow * D.L0[k]) / (D.rc / D.nc)));
+      cap *= std::max(1, (int)((kBoxGrow * D.L0[k]) / (D.rc / D.nc)));
     }
+    if (cap >= (double)kMaxCells) return fail(RBMD_ERR_UNSUPPORTED, "box of about 2^31 cells or more at its largest");
+    D.ncell_cap = (int)cap;
     D.p_start = p.pressure[0];
     D.p_stop = p.pressure[1];
     D.p_damp = p.pressure[2];
