@@ -22,7 +22,9 @@ constexpr int kBuildCells = 32;        // cells per block of the cell-list build
 constexpr int kBuildFew = 8;           // and in systems of up to kFewCells cells
 constexpr int kFewCells = 1024;
 constexpr int kCellChains = 4;         // chains of a cell's atoms beyond its bucket
-constexpr int kCellBigGrid = 16384;    // cells of a system above which counts are added up in two levels
+constexpr int kCellBigGrid = 16384;     // cells of a system above which counts are added up by groups
+constexpr int kCellHugeGrid = 524288;   // and in two levels, the second of
+constexpr int kCellSuper = 65536;       // this many cells
 constexpr int kRbeSlack = 64;          // Metropolis proposal slots tried beyond the samples still to draw
 constexpr int kEamRow = 8;             // doubles per row of the device's rhor and z2r tables
 constexpr int kQueue = 64;             // per-warp pair queue of the pair kernel
@@ -160,7 +162,8 @@ struct SysDev {
   int* cell_head;      // [ncell][kCellChains] last atom of each chain of those that found the bucket full
   int* cell_next;      // [n] the chains' links
   int* cell_rest;      // [n] scratch, by place in cell order: the chained atoms of a cell, one after the other
-  int* cell_gsum;      // [ncell / 32 + 1] atoms per 32 cells (systems of many cells)
+  int* cell_gsum;      // [ncell / 32 + 4] atoms per 32 cells (systems of many cells)
+  int* cell_super;     // [ncell / kCellSuper + 1] and per kCellSuper cells, zero between lists
   int* sorted;         // atom ids in cell order
   int* rank;           // [n] position of each atom in cell order (inverse of sorted)
   double4* sx;         // sorted positions + charge (FP64)

@@ -691,7 +691,8 @@ int Context::add_system(const rbmd_system_desc& d, const rbmd_params& p, int32_t
   D.cell_head = (int*)dal(sizeof(int) * (size_t)D.ncell_cap * kCellChains);
   D.cell_next = (int*)dal(sizeof(int) * n);
   D.cell_rest = (int*)dal(sizeof(int) * n);
-  D.cell_gsum = (int*)dal(sizeof(int) * (D.ncell_cap / 32 + 1));
+  D.cell_gsum = (int*)dal(sizeof(int) * (D.ncell_cap / kBuildCells + 4));
+  D.cell_super = (int*)dal(sizeof(int) * (D.ncell_cap / kCellSuper + 1));
   D.sorted = (int*)dal(sizeof(int) * n);
   D.rank = (int*)dal(sizeof(int) * n);
   D.sx = (double4*)dal(sizeof(double4) * n);
@@ -846,6 +847,7 @@ int Context::add_system(const rbmd_system_desc& d, const rbmd_params& p, int32_t
   up(D.v, hv.data(), sizeof(double4) * n);
   cudaMemsetAsync(D.f, 0, sizeof(double4) * n, stream);
   cudaMemsetAsync(D.cell_count, 0, sizeof(int) * 2 * D.cell_stride, stream);
+  cudaMemsetAsync(D.cell_super, 0, sizeof(int) * (D.ncell_cap / kCellSuper + 1), stream);
   up(D.meta, hmeta.data(), sizeof(int4) * n);
   up(D.image, himg.data(), sizeof(int) * 3 * n);
   up(D.eps, d.epsilon, sizeof(double) * d.n_types);

@@ -25,11 +25,13 @@ __global__ void k_cells_count(const SysDev* __restrict__ S, const int2* __restri
 // box of a few hundred cells has a warp per cell and blocks for a third of the chip: with 32 cells per
 // block the kernel took 9 us for 512 cells of 18 atoms and 58 us for 27 cells of 167.
 constexpr int kBuildThreads = 256;
-static_assert(kCellBlock % kBuildCells == 0 && kBuildCells % kBuildFew == 0 && kBuildCells == 32 && kBuildFew % 4 == 0,
+static_assert(kCellBlock % kBuildCells == 0 && kBuildCells % kBuildFew == 0 && kBuildCells == 32 && kBuildFew % 4 == 0 &&
+                  kCellSuper % (4 * kBuildCells) == 0,
               "a work item is a whole number of build blocks, a block's counts start on 16 bytes");
 static_assert((kCellChains & (kCellChains - 1)) == 0 && kCellChains <= 8, "a chain per lane of a cell");
 
-// Atoms per group of kBuildCells cells, for systems of more than kCellBigGrid cells.
+// Atoms per group of kBuildCells cells, for systems of more than kCellBigGrid cells, and per kCellSuper
+// cells in those of more than kCellHugeGrid (sums that the build clears).
 __global__ void k_cells_group_sums(const SysDev* __restrict__ S, const int2* __restrict__ work) {
   const int2 w = work[blockIdx.x];
   const SysDev& s = S[w.x];
@@ -37,11 +39,16 @@ __global__ void k_cells_group_sums(const SysDev* __restrict__ S, const int2* __r
   const int par = s.st->cell_epoch & 1;
   const int cnt = c < s.ncell ? s.cell_count[(size_t)par * s.cell_stride + c] : 0;
   const int sum = __reduce_add_sync(0xffffffffu, cnt);
-  if ((threadIdx.x & 31) == 0 && c < s.ncell) s.cell_gsum[c / kBuildCells] = sum;
+  if ((threadIdx.x & 31) == 0 && c < s.ncell) {
+    s.cell_gsum[c / kBuildCells] = sum;
+    if (s.ncell > kCellHugeGrid && sum > 0) atomicAdd(&s.cell_super[c / kCellSuper], sum);
+  }
 }
 
 // One block per kBuildCells (or kBuildFew) cells.  Bound by latency: the loads of the preceding counts (at most
-// kCellBigGrid / (4 x 256) 16-byte loads per thread; above that the group sums of the kernel before),
+// kCellBigGrid / (4 x 256) 16-byte loads per thread; above that the sums of the kernel before, at most
+// kCellHugeGrid / (32 x 4 x 256) such loads, or two and the sums of kCellSuper cells: with one level for
+// any size a list of 17 M cells took 21.6 ms and of 64 M cells 331 ms, for now 3.2 and 13.7 ms),
 // then one dependent gather per atom.  A cell's ids are taken by 8 lanes where buckets are small (cells
 // of a few atoms) and by a warp otherwise; each lane ranks its ids against the whole cell, so cells
 // of hundreds of atoms need no serial sort.  Atoms beyond the bucket are collected from their cell's
@@ -65,7 +72,13 @@ __global__ void __launch_bounds__(kBuildThreads) k_cells_build(const SysDev* __r
   if (c0 < s.ncell) {  // block-uniform
     int sum = 0;
     if (big && per == kBuildCells) {
-      for (int g = tid; g < c0 / kBuildCells; g += kBuildThreads) sum += s.cell_gsum[g];
+      const int super = s.ncell > kCellHugeGrid ? c0 / kCellSuper : 0, end = c0 / kBuildCells;
+      const int* g = s.cell_gsum;  // 16 bytes per load from the first group of the super group on
+      for (int k = super * (kCellSuper / kBuildCells) + 4 * tid; k < end; k += 4 * kBuildThreads) {
+        const int4 v = *reinterpret_cast<const int4*>(g + k);
+        sum += v.x + (k + 1 < end ? v.y : 0) + (k + 2 < end ? v.z : 0) + (k + 3 < end ? v.w : 0);
+      }
+      for (int k = tid; k < super; k += kBuildThreads) sum += s.cell_super[k];
     } else {
       const int4* c4 = reinterpret_cast<const int4*>(count);  // c0 is a multiple of 4
       for (int g = tid; g < c0 / 4; g += kBuildThreads) {
@@ -154,7 +167,11 @@ __global__ void __launch_bounds__(kBuildThreads) k_cells_build(const SysDev* __r
   if (c0 == 0)
     for (int c = items * kCellBlock + tid; c < s.ncell_cap; c += kBuildThreads) other[c] = 0;
   // every block has read this list's buffer index: the next list takes the other buffer
-  if (arrive_last(&st->counter[7], (unsigned)(items * (kCellBlock / per))) && tid == 0) st->cell_epoch ^= 1;
+  if (arrive_last(&st->counter[7], (unsigned)(items * (kCellBlock / per)))) {
+    if (tid == 0) st->cell_epoch ^= 1;
+    if (big && s.ncell > kCellHugeGrid)
+      for (int g = tid; g <= (s.ncell - 1) / kCellSuper; g += kBuildThreads) s.cell_super[g] = 0;
+  }
 }
 
 void launch_cells_build(const Batch& b, cudaStream_t st) {

@@ -106,3 +106,29 @@ def test_lists_built_by_every_route_in_turn(ctx_factory, oracle_mod, batch):
         ctx.step(ids, 2)
         ctx.thermo(ids[0])
         check()
+
+
+@pytest.mark.parametrize("edge", [80, 81])  # 512,000 cells: groups; 531,441: groups of groups
+def test_cells_of_a_huge_box_match_oracle(ctx_factory, oracle_mod, edge):
+    rng = np.random.default_rng(edge)
+    box = 2.5 * edge + 0.01
+    sd = _lj(5000, box, rng.uniform(0, box, (5000, 3)))
+    sd.params.r_core = 2.5
+    ctx = ctx_factory()
+    sid = ctx.add_system(sd)
+    for _ in range(3):
+        for a, b in zip(ctx.cells(sid), oracle_mod.Oracle(sd).cells()):
+            assert np.array_equal(a, b)
+        sd.pos = rng.uniform(0, box, (5000, 3))
+        ctx.set_state(sid, x=sd.pos)
+
+
+def test_cost_of_a_huge_box_is_linear(ctx_factory):
+    """64 times the cells for 200,000 atoms: at most 160 times the time (the sums before a block's cells
+    went up with the square of the cells: 1400 times)."""
+    def gas(edge):
+        g = np.stack(np.meshgrid(*[np.arange(59)] * 3), -1).reshape(-1, 3)[:200000]
+        sd = _lj(200000, 2.5 * edge + 0.1, (g + 0.5) * (2.5 * edge / 59))
+        sd.params.r_core = 2.5
+        return sd
+    assert _cells_ms(ctx_factory, gas(400)) < 160 * _cells_ms(ctx_factory, gas(100))
