@@ -45,17 +45,63 @@ __global__ void k_cells_group_sums(const SysDev* __restrict__ S, const int2* __r
   }
 }
 
+// Atom i at place k of the cell order.
+__device__ __forceinline__ void place(const SysDev& s, int i, int k) {
+  s.sorted[k] = i;
+  s.rank[i] = k;
+  const double4 p = s.x[i];
+  s.sx[k] = p;
+  s.sxf[k] = make_float4((float)p.x, (float)p.y, (float)p.z, (float)p.w);
+  const int4 m = s.meta[i];
+  s.smeta[k] = make_int4(i, m.x, m.y, m.z);
+}
+
+// How many of a bucket's n ids are below id (a bucket starts on 16 bytes).
+__device__ __forceinline__ int rank_in(const int* ids, int n, int id) {
+  int r = 0, j = 0;
+  for (; j + 4 <= n; j += 4) {
+    const int4 v = *reinterpret_cast<const int4*>(ids + j);
+    r += (v.x < id ? 1 : 0) + (v.y < id ? 1 : 0) + (v.z < id ? 1 : 0) + (v.w < id ? 1 : 0);
+  }
+  for (; j < n; ++j) r += ids[j] < id ? 1 : 0;
+  return r;
+}
+
+// A cell of more atoms than its bucket holds, by the cell's lanes (8, or a warp).  The rest hang on the
+// cell's chains and are laid out one after the other first.  Not inlined: the build would spill.
+__device__ __noinline__ void place_overfull(const SysDev& s, int c, int cnt, int start, int lanes, int lane) {
+  const int cap = s.cell_cap, over = cnt - cap, gl = lane & (lanes - 1);
+  const int* ids = s.cell_bucket + (size_t)c * cap;
+  int* rest = s.cell_rest + start + cap;
+  if (gl < kCellChains && gl < over) {
+    int id = s.cell_head[(size_t)c * kCellChains + gl];
+    for (int k = gl;;) {
+      rest[k] = id;
+      k += kCellChains;
+      if (k >= over) break;
+      id = s.cell_next[id];
+    }
+  }
+  __syncwarp(lanes == 32 ? 0xffffffffu : 0xffu << (lane & 24));  // the cell's lanes
+  for (int k = gl; k < cnt; k += lanes) {
+    const int id = k < cap ? ids[k] : rest[k - cap];
+    int r = rank_in(ids, cap, id);
+    for (int j = 0; j < over; ++j) r += rest[j] < id ? 1 : 0;
+    place(s, id, start + r);
+  }
+}
+
 // One block per kBuildCells (or kBuildFew) cells.  Bound by latency: the loads of the preceding counts (at most
 // kCellBigGrid / (4 x 256) 16-byte loads per thread; above that the sums of the kernel before, at most
 // kCellHugeGrid / (32 x 4 x 256) such loads, or two and the sums of kCellSuper cells: with one level for
-// any size a list of 17 M cells took 21.6 ms and of 64 M cells 331 ms, for now 3.2 and 13.7 ms),
+// any size a list of 17 M cells took 21.6 ms and of 64 M cells 331 ms, for now 2.9 and 12.6 ms),
 // then one dependent gather per atom.  A cell's ids are taken by 8 lanes where buckets are small (cells
 // of a few atoms) and by a warp otherwise; each lane ranks its ids against the whole cell, so cells
 // of hundreds of atoms need no serial sort.  Atoms beyond the bucket are collected from their cell's
 // chains first, so an atom is compared with those of its own cell only: in a slab that fills a tenth of
 // its box (64,000 atoms, buckets of 8, 13 atoms per cell) a list takes 27 us, against 44 ms when each atom
-// of an over-full cell went through the overflow of the whole system.  `items` is the number of work items where the table covers a
-// single system's present cells only, 0 where it covers the ncell_cap of each system.
+// of an over-full cell went through the overflow of the whole system.  `items` is the number of work items
+// where the table covers a single system's present cells only, 0 where it covers the ncell_cap of each.
 __global__ void __launch_bounds__(kBuildThreads) k_cells_build(const SysDev* __restrict__ S,
                                                              const int2* __restrict__ work, int big, int items) {
   const int2 w = work[blockIdx.x];
@@ -105,54 +151,13 @@ __global__ void __launch_bounds__(kBuildThreads) k_cells_build(const SysDev* __r
     const int cap = s.cell_cap;
     const int lanes = cap <= 16 ? 8 : 32;  // lanes per cell
     const int gl = tid & (lanes - 1);
-    auto place = [&](int i, int k) {
-      s.sorted[k] = i;
-      s.rank[i] = k;
-      const double4 p = s.x[i];
-      s.sx[k] = p;
-      s.sxf[k] = make_float4((float)p.x, (float)p.y, (float)p.z, (float)p.w);
-      const int4 m = s.meta[i];
-      s.smeta[k] = make_int4(i, m.x, m.y, m.z);
-    };
     for (int cc = tid / lanes; cc < per; cc += kBuildThreads / lanes) {
-      const int c = c0 + cc, cnt = s_cnt[cc], in = min(cnt, cap);
-      const int* ids = s.cell_bucket + (size_t)c * cap;
-      auto rank_of = [&](int id) {
-        int r = 0, j = 0;
-        for (; j + 4 <= in; j += 4) {  // a bucket starts on 16 bytes
-          const int4 v = *reinterpret_cast<const int4*>(ids + j);
-          r += (v.x < id ? 1 : 0) + (v.y < id ? 1 : 0) + (v.z < id ? 1 : 0) + (v.w < id ? 1 : 0);
-        }
-        for (; j < in; ++j) r += ids[j] < id ? 1 : 0;
-        return r;
-      };
+      const int cnt = s_cnt[cc];
+      const int* ids = s.cell_bucket + (size_t)(c0 + cc) * cap;
       if (cnt <= cap) {
-        for (int k = gl; k < cnt; k += lanes) {
-          const int id = ids[k];
-          place(id, s_start[cc] + rank_of(id));
-        }
-      } else {  // more atoms than the bucket holds: the rest hang on the cell's chains
-        const int over = cnt - cap;
-        int* rest = s.cell_rest + s_start[cc] + cap;
-        if (gl < kCellChains && gl < over) {
-          int id = s.cell_head[(size_t)c * kCellChains + gl];
-          for (int k = gl;;) {
-            rest[k] = id;
-            k += kCellChains;
-            if (k >= over) break;
-            id = s.cell_next[id];
-          }
-        }
-        __syncwarp(lanes == 32 ? 0xffffffffu : 0xffu << (lane & 24));  // the cell's lanes
-        auto rank_all = [&](int id) {
-          int r = rank_of(id);
-          for (int k = 0; k < over; ++k) r += rest[k] < id ? 1 : 0;
-          return r;
-        };
-        for (int k = gl; k < cnt; k += lanes) {
-          const int id = k < cap ? ids[k] : rest[k - cap];
-          place(id, s_start[cc] + rank_all(id));
-        }
+        for (int k = gl; k < cnt; k += lanes) place(s, ids[k], s_start[cc] + rank_in(ids, cnt, ids[k]));
+      } else {
+        place_overfull(s, c0 + cc, cnt, s_start[cc], lanes, lane);
       }
     }
     if (c0 == 0 && tid == 0) {  // a new cell list: nothing has moved since
