@@ -256,7 +256,8 @@ int Context::refresh(System* s) {
 
 // Atoms per block of the structure factor: small while the blocks do not fill the 148 SMs (the sums over
 // a chunk's warps cost more the shorter it is: with 64 and 128 atoms for every system the saline stream's
-// kernel took 127 us for 97 us).  By the system's size alone: its sums are the same in any batch.
+// kernel took 127 us for 97 us).  By the system's size alone, not the batch's or the device's: the sums are
+// the same everywhere.
 static int rho_chunk(int n) { return n <= 148 * 64 ? 64 : (n <= 148 * 128 ? 128 : kRhoChunk); }
 
 // Ids a cell's bucket holds: twice the mean occupancy and at least 4 more (a liquid's cells rarely pass
@@ -966,6 +967,8 @@ Context::BatchRec* Context::build_batch(const std::vector<System*>& group, int& 
   Batch& b = br->b;
   b.sys = d_sys_;
   b.nsys = (int)group.size();
+  int sms = 0;
+  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, cfg.device) == cudaSuccess && sms > 0) b.sms = sms;
   const SysDev& g = group[0]->dev;
   b.ff = g.ff;
   b.neigh = g.neigh;

@@ -1020,11 +1020,15 @@ __device__ __forceinline__ void lean_atom(const SysDev& s, int sidx, int lane, L
 }
 
 // BLOCKS: resident blocks per SM it is compiled for.  Three (80 registers) keep more warps in flight; two
-// (126-128 registers) leave the FP64 kernels with special bonds without their 32-60 bytes of spill stores.
-// Three blocks -> two, us per launch: saline 1000 atoms 49.3 -> 41.4, 4000 98.6 -> 83.3, Ewald water 4500
-// 138.6 -> 117.0, but Ewald water 15,000 295.6 -> 321.4, saline 16,000 244.0 -> 257.4 and 64,000 838 -> 922.
-// The line is set between 4500 and 15,000 atoms; where exactly the two cross was not measured.
-constexpr long long kLeanFewAtoms = 8192;
+// (126-128 registers) leave the FP64 kernels with special bonds without their 32-60 bytes of spill stores,
+// but leave the side stream's kernels no registers.  Two are used where they fill the chip no more often than
+// three would, in the first wave (up to 2 blocks per SM: 2368 atoms) and the second (above 3, up to 4: 3553
+// to 4736 atoms).  Kernel (step), us, three -> two: saline 1000 atoms 49.7 -> 41.7 (84.5 -> 77.6), 4 x 1000
+// 96.1 -> 82.0 (133.0 -> 118.3), 4500 93.6 -> 79.1 (127.8 -> 119.2), Ewald water 4500 138.1 -> 116.3 (187.4
+// -> 182.0), alkanes 4374 27.3 -> 25.9 (67.8 -> 70.8); but saline 3000 60.9 -> 76.0 (94.6 -> 111.2), 6000
+// 112.7 -> 117.2, 8000 142.2 -> 144.2 (178.6 -> 183.2), 16,000 244 -> 257, Ewald water 6000 175.8 -> 182.3,
+// 15,000 296 -> 322, alkanes 7986 37.9 -> 41.4.
+static bool lean_two_blocks(int blocks, int sms) { return blocks <= 2 * sms || (blocks > 3 * sms && blocks <= 4 * sms); }
 
 template <typename R, int MODE, bool SPECIAL, bool VIRIAL, bool NEAR, int BLOCKS>
 __global__ void __launch_bounds__(kPairWarps * 32, BLOCKS)
@@ -2745,7 +2749,7 @@ static void go_near(const Batch& b, cudaStream_t st) {
         b.sys, b.dense == 2 ? b.pair_cells.d : b.pair.d, 0, nullptr, nullptr, nullptr, nullptr, band);
   else if (b.lean) {
     constexpr bool kSpills = sizeof(R) == 8 && SPECIAL;
-    if (kSpills && b.natoms <= kLeanFewAtoms)
+    if (kSpills && lean_two_blocks(b.pair.n, b.sms))
       k_pair2<R, MODE, SPECIAL, VIRIAL, NEAR, kSpills ? 2 : 3><<<b.pair.n, kPairWarps * 32, 0, st>>>(b.sys, b.pair.d);
     else
       k_pair2<R, MODE, SPECIAL, VIRIAL, NEAR, 3><<<b.pair.n, kPairWarps * 32, 0, st>>>(b.sys, b.pair.d);
@@ -2779,15 +2783,17 @@ static const void* col_kernel(const Batch& b) {
 void plan_pair_col(Batch& b, double chunks, double longest, int nc) {
   const int side = 2 * nc + 1;
   b.col_rows = side * side;
-  // Up to about one chunk per resident warp (148 SMs x 16) the split form's eight warps per chunk are
-  // faster: 177 -> 56 us (1200 atoms of saline), 216 -> 118 us (9000), 456 -> 439 us (64,000, 2140
-  // chunks); above, its second staging costs more than it spreads (3420 -> 5460 us for 985,000 atoms).
-  // Four warps per chunk were no better anywhere (78, 117 and 469 us).  Sixteen, a block to an SM, while
-  // there are SMs for the chunks: 50 -> 41 us for 1200 atoms; beyond, eight (414 against 530 us at 64,000).
-  b.col_split = b.col_rows > kColMaxRows || chunks >= 2200 ? 1 : (chunks <= 148 && b.col_rows <= kColMaxRows16 ? 16 : 8);
-  int dev = 0, sms = 0, per_sm = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  // Up to about a chunk per resident warp (16 per SM) the split form's eight warps per chunk are faster:
+  // 9000 atoms of saline (313 chunks) 231 -> 134 us, 32,000 (1084) 337 -> 249, 64,000 (2144) 450 -> 432;
+  // above, its second staging costs more than it spreads: 80,000 (2662) 477 -> 517, 128,000 (4220) 711 ->
+  // 815.  Batches of small systems cross sooner: 4 x 9000 (1253) 281 -> 277, 40 x 1200 (1819) 287 -> 337, 8 x
+  // 9000 (2506) 451 -> 477.  Sixteen warps, a block to an SM, while there are SMs for the chunks: eight ->
+  // sixteen 1200 atoms (45) 56 -> 48 us, 4000 (143) 71 -> 55, 3 x 1200 (136) 58 -> 48; but 5000 (181) 112 ->
+  // 115, 4 x 1200 (182) 68 -> 81, 9000 134 -> 144.  Four warps per chunk were no better anywhere (78 us for
+  // 1200 atoms, 117 for 9000, 469 for 64,000).
+  const int sms = b.sms;
+  int per_sm = 0;
+  b.col_split = b.col_rows > kColMaxRows || chunks >= 15.0 * sms ? 1 : (chunks <= sms && b.col_rows <= kColMaxRows16 ? 16 : 8);
   // The limit on dynamic shared memory belongs to the kernel, of the whole process: always the most a
   // form can need, so that planning a batch of few rows takes nothing from a batch planned before it.
   if (b.col_split > 1) {
@@ -2807,12 +2813,12 @@ void plan_pair_col(Batch& b, double chunks, double longest, int nc) {
   // lies past a short column's end.  Column launches with 1, 2, 3, 4, 6 parts and with all nine: 25.90,
   // 25.88, 25.85, 25.94, 26.13, 26.48 ms for 7.86 M atoms (the rule: one), 3.65, 3.49, 3.47, 3.39, 3.42,
   // 3.46 ms for 970,000 (four), 1.47, 0.89, 0.74, 0.68, 0.68, 0.56 ms for 129,000 (all).
-  const long long resident = (long long)std::max(1, sms) * std::max(1, per_sm) * warps;
+  const long long resident = (long long)sms * std::max(1, per_sm) * warps;
   b.col_parts = std::max(1, std::min(1024, (int)std::ceil(1.2 * longest / 32.0)));
   if (b.col_split == 1) b.col_parts = (int)std::min<long long>(b.col_parts, (10 * resident + b.pair.n - 1) / std::max(1, b.pair.n));
   const long long items = (long long)b.pair.n * b.col_parts;
   const long long need = b.col_split > 1 ? items : (items + kColWarps - 1) / kColWarps;
-  b.col_grid = (int)std::max(1LL, std::min(need, (long long)std::max(1, sms) * std::max(1, per_sm)));
+  b.col_grid = (int)std::max(1LL, std::min(need, (long long)sms * std::max(1, per_sm)));
 }
 
 template <typename R, bool VIRIAL>

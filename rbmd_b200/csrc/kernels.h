@@ -39,6 +39,7 @@ struct Batch {
   int max_P = 0;             // largest P (or Ewald nk) in the batch
   float band[4] = {0, 0, 0, 0};  // FP32 classification bands: union over the batch (same rc, rs)
   long long natoms = 0;      // atoms over all systems of the batch
+  int sms = 148;             // SMs of the context's device
 };
 
 enum FinalMode { kFinalForceOnly = 0, kFinalKick = 1, kFinalInit = 2 };
