@@ -525,7 +525,7 @@ enum rbmd_pair_layout {
   RBMD_LAYOUT_TILE = 0,     /* warp per home cell, candidate batches shared by the cell's atoms */
   RBMD_LAYOUT_LEAN = 1,     /* warp per atom over per-row segment tables (dims >= 2 nc + 1) */
   RBMD_LAYOUT_GENERAL = 2,  /* warp per atom, any box */
-  RBMD_LAYOUT_COLUMN = 3    /* warp per column of home cells, lane per atom walking its own candidate
+  RBMD_LAYOUT_COLUMN = 3    /* lane per atom of a column of home cells, walking its own candidate
                                window of a shared staged row (mixed-precision RBL forces of LJ/CUT,
                                LJ/CUT/COUL/LONG and CVFF; the tile layout's boxes) */
 };

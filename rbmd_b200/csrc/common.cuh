@@ -108,8 +108,9 @@ struct SysDev {
   int eam_per_type;  // EAM tables per type (setfl): frho / rhor by type, z2r by type pair
   int eam_pad;
   int lean;   // segment-table traversal usable (every dimension holds more than nc cells)
-  int dense;  // pair kernel layout: 0 warp per atom, 1 tile (warp per home cell), 2 column (warp per
-              // column of home cells, lane per atom; FP32 RBL forces only, the tile kernel otherwise)
+  int dense;  // pair kernel layout: 0 warp per atom, 1 tile (warp per home cell), 2 column (lane per atom
+              // of a column of home cells, one or several warps per chunk of 32 of them; FP32 RBL forces
+              // only, the tile kernel otherwise)
   int blocks_pair, blocks_atom, blocks_rho, blocks_tri, rbe_mmax, has_triples, n_triples;
   // NPT barostats (npt 1: Berendsen at the end of the step, 2: MTK around the integrator): the
   // box changes on the device every step.  Cell arrays and the cell work table hold ncell_cap cells

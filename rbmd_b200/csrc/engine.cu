@@ -472,8 +472,8 @@ int Context::add_system(const rbmd_system_desc& d, const rbmd_params& p, int32_t
   // tile kernel (warp per home cell, candidates shared by the cell's atoms) pays off in mixed
   // precision once cells hold a few atoms on average; the lean kernel (warp per atom) is faster
   // below that and in FP64, where the tile kernel's per-lane FP64 state no longer fits in
-  // registers.  In mixed precision the column kernel (warp per column of home cells, lane per
-  // atom) takes the tile kernel's systems for the RBL forces.  RBMD_PAIR_LAYOUT overrides the
+  // registers.  In mixed precision the column kernel (lane per atom of a column of home cells
+  // chunk by chunk) takes the tile kernel's systems for the RBL forces.  RBMD_PAIR_LAYOUT overrides the
   // choice for tuning and tests: "atom" (general), "lean", "cell" (tile), "column".
   const bool stencil_ok = D.dims[0] >= 2 * D.nc + 1 && D.dims[1] >= 2 * D.nc + 1 && D.dims[2] >= 2 * D.nc + 1;
   // The lean, tile and column kernels also walk stencils that repeat cells, as long as every

@@ -53,7 +53,7 @@ inline bool tile_layout_ok(const SysDev& D) {
 inline bool lean_layout_ok(const SysDev& D) {
   return D.dims[0] >= D.nc + 1 && D.dims[1] >= D.nc + 1 && D.dims[2] >= D.nc + 1;
 }
-// The column kernel's (warp per column of home cells, lane per atom): the tile kernel's boxes, FP32
+// The column kernel's (lane per atom of a column of home cells): the tile kernel's boxes, FP32
 // RBL forces of LJ/CUT, LJ/CUT/COUL/LONG and CVFF; every other pass of such a system runs the tile
 // kernel over its cell table.
 inline bool column_layout_ok(const SysDev& D) {

@@ -2064,9 +2064,9 @@ __device__ inline int col_first_skip(const SysDev& s, int i, int pice) {
 // strays and walks them one after the other, its eight warps sharing a stray's traversal rows: first
 // counting every row's shells, then, with the counts of the rows before known, picking and evaluating.
 // Their forces are written where the column kernel reads them back for the RBL mean.  Strays are few
-// (one atom in a thousand), so the pass lasts as long as one walk: 45 us when a warp walked a stray by
-// itself, and 167 us (9000 atoms) to 324 us (64,000) when a warp per column of cells walked its strays cell
-// after cell.
+// (one atom in a thousand), so the pass lasts as long as a walk or two: 25 us for 9000 atoms of saline and
+// 40 us for 64,000, against 58 and 57 us when a warp walked a stray by itself, and 167 and 315 us when a warp
+// per column of cells walked its strays cell after cell.
 constexpr int kStrayRows = 512;  // rows counted at a time
 constexpr int kStrayQ = 64;      // a warp's queue of selected pairs
 

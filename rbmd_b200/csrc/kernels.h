@@ -20,16 +20,17 @@ struct Batch {
   int nsys = 0;
   Work atom, pair, cell, rho, tri, term, kred, draw;
   Work pair_cells;           // column layout: the tile kernel's cell table (energies, other modes)
-  // column layout: pair.d lists every column (slot, column index), most atoms per column first;
-  // the persistent column kernel takes them in that order from col_ctr[0] (col_ctr[1] counts the warps
-  // that are done; the last one resets both), every column in col_parts items, col_grid blocks;
-  // col_split: warps that share a chunk of 32 atoms, by its col_rows traversal rows (1: none do)
+  // column layout: pair.d lists every column (slot, column index), most atoms per column first.  The
+  // persistent column kernel (col_grid blocks) takes items in that order from col_ctr[0] (col_ctr[1] counts
+  // the warps that are done; the last one resets both): item k is part k % col_parts of column k /
+  // col_parts, every col_parts-th of its chunks of 32 atoms.  col_split: warps that share a chunk, by its
+  // col_rows traversal rows (1: none do)
   unsigned* col_ctr = nullptr;
   int col_grid = 0, col_parts = 1, col_split = 1, col_rows = 0;
   // uniform switches of the batch (a batch never mixes them)
   int ff = 0, neigh = 0, coul = 0, prec = 0, temp_ctrl = 0, special = 0;
   int has_shake = 0, has_bonded = 0;
-  int dense = 0;             // pair kernel: 0 = warp per atom, 1 = warp per home cell, 2 = warp per column
+  int dense = 0;             // pair kernel: 0 = warp per atom, 1 = warp per home cell, 2 = column (lane per atom)
   int lean = 0;              // warp per atom with segment tables (dims >= 2 nc + 1 everywhere)
   int npt = 0;               // NPT barostat: 0 none, 1 Berendsen (end of step), 2 MTK (around the integrator)
   int near = 0;              // RBL Coulomb with the reference's near-Coulomb table (RBMD_NEAR_TABLE)

@@ -43,7 +43,7 @@ def pair(ctx_factory, oracle_mod, sd, layout="auto", **ctxkw):
     """GPU context + system and the oracle twin.  `layout` selects the pair kernel: "auto" (the
     library's choice), "atom" (general warp-per-atom traversal), "lean" (warp per atom with segment
     tables), "cell" (tile: warp per home cell, candidates shared by the cell's atoms), "column"
-    (warp per column of home cells, lane per atom; mixed-precision RBL forces, else as "cell")."""
+    (lane per atom of a column of home cells; mixed-precision RBL forces, else as "cell")."""
     import os
     ctx = ctx_factory(**ctxkw)
     old = os.environ.get("RBMD_PAIR_LAYOUT")
