@@ -689,11 +689,7 @@ int Context::add_system(const rbmd_system_desc& d, const rbmd_params& p, int32_t
   D.cell_count = (int*)dal(sizeof(int) * 2 * D.cell_stride);
   D.cell_start = (int*)dal(sizeof(int) * (D.ncell_cap + 1));
   D.cell_bucket = (int*)dal(sizeof(int) * (size_t)D.ncell_cap * D.cell_cap);
-  D.cell_head = (int*)dal(sizeof(int) * (size_t)D.ncell_cap * kCellChains);
-  D.cell_next = (int*)dal(sizeof(int) * n);
-  D.cell_rest = (int*)dal(sizeof(int) * n);
   D.cell_gsum = (int*)dal(sizeof(int) * (D.ncell_cap / kBuildCells + 4));
-  D.cell_super = (int*)dal(sizeof(int) * (D.ncell_cap / kCellSuper + 1));
   D.sorted = (int*)dal(sizeof(int) * n);
   D.rank = (int*)dal(sizeof(int) * n);
   D.sx = (double4*)dal(sizeof(double4) * n);
@@ -840,6 +836,11 @@ int Context::add_system(const rbmd_system_desc& d, const rbmd_params& p, int32_t
   D.vir_part = (double*)dal(sizeof(double) * std::max(9 * part_blocks, 3 * part_chunks));
   D.tri_part = (double*)dal(sizeof(double) * 6 * std::max(1, D.blocks_tri));
   D.st = (SysState*)dal(sizeof(SysState));
+  // what only over-full cells and huge boxes use, behind the arrays of every step
+  D.cell_head = (int*)dal(sizeof(int) * (size_t)D.ncell_cap * kCellChains);
+  D.cell_next = (int*)dal(sizeof(int) * n);
+  D.cell_rest = (int*)dal(sizeof(int) * n);
+  D.cell_super = (int*)dal(sizeof(int) * (D.ncell_cap / kCellSuper + 1));
   if (oom) {
     for (void* ptr : s->allocs) dfree(ptr);
     return fail(RBMD_ERR_OOM, "device allocation failed for a system of " + std::to_string(n) + " atoms");

@@ -2084,12 +2084,13 @@ __global__ void __launch_bounds__(kAtomBlock, 3) k_pair_col_strays(const SysDev*
   const unsigned FULL = 0xffffffffu;
   if (threadIdx.x == 0) s_n = 0;
   __syncthreads();
-  // looked over in the atoms' own order: its loads do not wait for one another
+  // in cell order: in the atoms' own order, whose loads would not wait for one another, the strays of a molecule
+  // fall to one block (9000 atoms of SPC/E water 154.7 -> 156.3 us per step, 970,000 of saline 94 -> 87 us)
   const int k = wk.y + threadIdx.x;
   if (k < s.n) {
-    const int c = __ldg(&s.cell_of_atom[k]);
+    const int c = __ldg(&s.cell_of_atom[__ldg(&s.smeta[k]).x]);
     const int dy = s.dims[1], dz = s.dims[2];
-    if (col_is_stray(s, ldg4(&s.x[k]), c / (dz * dy), (c / dz) % dy, c % dz)) s_list[atomicAdd(&s_n, 1)] = s.rank[k];
+    if (col_is_stray(s, ldg4(&s.sx[k]), c / (dz * dy), (c / dz) % dy, c % dz)) s_list[atomicAdd(&s_n, 1)] = k;
   }
   __syncthreads();
   const int nc = s.nc, side = 2 * nc + 1, nrows = side * side, pice = s.pice;
