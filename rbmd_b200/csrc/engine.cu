@@ -650,7 +650,9 @@ int Context::add_system(const rbmd_system_desc& d, const rbmd_params& p, int32_t
   int64_t total = 0;
   bool oom = false;
   // one allocation of about the estimated footprint, cut up; what does not fit in it is allocated by itself
-  size_t slab_left = (size_t)estimate_bytes(d, p) + 48 * 256;
+  rbmd_params need = p;
+  need.coulomb = D.coul;  // none without a Coulomb force field, whatever the parameters say
+  size_t slab_left = (size_t)estimate_bytes(d, need) + 48 * 256;
   char* slab = (char*)dmalloc(slab_left);
   if (slab) s->allocs.push_back(slab);
   else slab_left = 0;
