@@ -1,5 +1,5 @@
-"""Cell lists where the build kernel's branches part: cells with more atoms than a bucket holds (the
-overflow list), boxes of more cells than are added up in one level, boxes of a few cells, and lists
+"""Cell lists where the build kernel's branches part: cells with more atoms than a bucket holds (their
+chains), boxes of more cells than are added up in one level, boxes of a few cells, and lists
 built one after the other from the two count buffers.  Integer work: equal to the oracle's."""
 import numpy as np
 import pytest
